@@ -53,13 +53,12 @@
 
 #include <math.h>
 
-#include "lbm_internal.h"
-#include "lbm_node.cuh"
+#include "ib_device.cuh"
 
 namespace {
 
-constexpr int BS = 16;                 // block size of the cyclic reduction
-constexpr int NMARK_MAX = 2048;        // largest marker count
+using namespace lbm_ib;
+
 #ifndef LBM_FACTOR_THREADS
 #define LBM_FACTOR_THREADS 512
 #endif
@@ -73,9 +72,6 @@ constexpr int FACTOR_THREADS = LBM_FACTOR_THREADS;
 constexpr int BOPS_WARPS = FACTOR_THREADS / 32;   // warps running block operations
 constexpr int SOLVE_THREADS = LBM_SOLVE_THREADS;
 constexpr int STAGE_BLOCKS = 32;       // factor blocks of one level staged in shared memory by ib_solve
-constexpr int FL = 2 * BS;             // columns of a coupling panel [L_o | L_q^T]
-constexpr int GW = 3 * BS;             // row width of a stored factor block [D^-1 | F_L | F_U]
-constexpr int GP = BS + 1;             // padded row stride of square blocks in shared memory
 constexpr int SOLVE_SMEM_BUDGET = LBM_SOLVE_SMEM;   // dynamic shared memory of ib_solve (bytes)
 
 // factor blocks ib_solve can stage next to the right-hand sides of nb blocks
@@ -96,9 +92,6 @@ __host__ __device__ constexpr int stage_blocks(int nb)
     return need < stage_cap(nb) ? need : stage_cap(nb);
 }
 constexpr int WS = BS * GP + BS * FL + BS * GP;   // workspace per warp (doubles)
-constexpr int NPART = 3 * LBM_MAXW + 3;           // per-CTA partials of ib_tile_update
-constexpr int TILE = 16;                          // correction-patch tile (nodes per side)
-constexpr int TILE_CAP = 256;                     // markers listed per tile
 
 // one-axis kernel value (boundary_condition.f90:1563-1600), disr = |r|
 __device__ __forceinline__ double delta1(double disr, int smooth)
@@ -123,33 +116,6 @@ __device__ __forceinline__ double delta1(double disr, int smooth)
     return 0.0;
 }
 
-
-// FP64 moments of the streamed populations at an interior node
-template <typename T>
-__device__ __forceinline__ void node_moments(const IBArgs &a, int i, int j, double &rho, double &u, double &v)
-{
-    const T *fin = (const T *)a.fin;
-    double g[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k)
-        g[k] = (double)Store<T>::ld(fin + (long long)k * a.plane + (long long)(j - lbm_ey(k)) * a.pitch +
-                                    (i - lbm_ex(k)));
-    const double drho = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])) + g[8];
-    const double jx = (g[1] - g[3]) + (g[5] - g[6]) + (g[8] - g[7]);
-    const double jy = (g[2] - g[4]) + (g[5] + g[6]) - (g[7] + g[8]);
-    rho = 1.0 + drho;
-    u = jx / rho;
-    v = jy / rho;
-}
-
-__device__ __forceinline__ const double *motion_row(const IBArgs &a, int step_index, double *time_out)
-{
-    const double time = (double)(step_index - 1) * (a.scale * a.uu);   // solution.f90:289
-    int idx = (int)llround(time / a.mdt) + 1;                             // mode.f90:280-281
-    idx = idx < 1 ? 1 : (idx > a.msteps ? a.msteps : idx);
-    if (time_out) *time_out = time;
-    return a.mstep + (long long)(idx - 1) * a.mcols;
-}
 
 // Step of this CTA's member of a factorization launch: step0 + blockIdx.y,
 // or per case in batched launches (the case's own start and count; -1 for
@@ -177,6 +143,8 @@ __device__ __forceinline__ IBArgs member_args(IBArgs a, int step)
     a.nsup += slot;
     a.fmode += 2 * slot;
     a.fstatus += slot;
+    a.rhs += slot * a.st_rhs;
+    a.y += slot * a.st_rhs;
     a.status = a.fstatus;   // errors of the chain are reported by the step that uses it
     a.bD += mem * a.wk_blocks;
     a.bL += mem * a.wk_blocks;
@@ -256,6 +224,10 @@ __global__ void __launch_bounds__(128) ib_geometry(const IBArgs base0, const IBA
     if (k >= a.nseg) return;
     const double *row = motion_row(a, step_index, nullptr);
     a.mk[k] = make_marker(a, row, k);
+    // the step's right-hand sides and solution are not there yet (the step
+    // loop's CTAs wait for the values themselves)
+    a.rhs[k] = a.rhs[a.nseg + k] = not_yet();
+    a.y[k] = a.y[a.nseg + k] = not_yet();
 }
 
 // one warp per marker: b = D u* over the support box, rhs = U_b - b
@@ -275,46 +247,11 @@ __global__ void __launch_bounds__(256) ib_interp(const IBArgs a0, const IBArgs *
     }
     const int k = blockIdx.x * 8 + warp;
     if (k >= a.nseg) return;
-    // the marker's box and kernel values are read where they lie (a local
-    // copy of the struct, indexed by node, would live on the stack)
-    const Marker *mp = a.mk + k;
-    const int i1 = mp->i1, i2 = mp->i2, j1 = mp->j1, j2 = mp->j2;
-    const bool ok = box_in_bounds(i1, i2, j1, j2, a.nx, a.ny);
-    if (!ok && lane == 0) atomicOr(a.status, LBM_ST_INDEX_INTERP);
-    const int nbx = ok ? i2 - i1 + 1 : 0, nby = ok ? j2 - j1 + 1 : 0;
-    const int nn = nbx > 0 && nby > 0 ? nbx * nby : 0;
-    double su = 0.0, sv = 0.0;
-    if (nn > 0) {
-        // at most LBM_BOX^2 = 36 nodes: lane t takes nodes t and t + 32, and
-        // both nodes' populations are loaded before either is summed (a lane
-        // without a second node loads its first again and weighs it 0); the
-        // sums are the loop's, node t then node t + 32, each a fused
-        // multiply-add onto the running sum
-        const bool h0 = lane < nn, h1 = lane + 32 < nn;
-        const int t0 = h0 ? lane : 0, t1 = h1 ? lane + 32 : t0;
-        const int ii0 = t0 % nbx, jj0 = t0 / nbx, ii1 = t1 % nbx, jj1 = t1 / nbx;
-        double rho0, u0, v0, rho1, u1, v1;
-        node_moments<T>(a, i1 + ii0, j1 + jj0, rho0, u0, v0);
-        node_moments<T>(a, i1 + ii1, j1 + jj1, rho1, u1, v1);
-        const double w0 = mp->phx[ii0] * mp->phy[jj0];   // X1(k,i) = kernel1*kernel2 (:1602)
-        const double w1 = mp->phx[ii1] * mp->phy[jj1];
-        if (h0) {
-            su = fma(w0, u0, su);
-            sv = fma(w0, v0, sv);
-        }
-        if (h1) {
-            su = fma(w1, u1, su);
-            sv = fma(w1, v1, sv);
-        }
-    }
-#pragma unroll
-    for (int off = 16; off; off >>= 1) {
-        su += __shfl_down_sync(0xffffffffu, su, off);
-        sv += __shfl_down_sync(0xffffffffu, sv, off);
-    }
+    double ru, rv;
+    interp_sum<T, LdNc>(a, (const T *)a.fin, interp_lane(a, k, lane), ru, rv);
     if (lane == 0) {
-        a.rhs[k] = mp->ub - su;                 // comj (:1624-1629)
-        a.rhs[a.nseg + k] = mp->vb - sv;
+        a.rhs[k] = ru;
+        a.rhs[a.nseg + k] = rv;
     }
 }
 
@@ -336,15 +273,6 @@ __device__ __forceinline__ bool box_overlap(int4 p, int4 q)
     return max(p.x, q.x) <= min(p.y, q.y) && max(p.z, q.z) <= min(p.w, q.w);
 }
 
-__device__ __forceinline__ int4 mbox(const Marker &m) { return make_int4(m.i1, m.i2, m.j1, m.j2); }
-
-// a marker as make_marker leaves it: support box within bounds (an empty
-// box included) and a wing index of the case
-__device__ __forceinline__ bool marker_ok(const IBArgs &a, const Marker &m)
-{
-    return box_in_bounds(m.i1, m.i2, m.j1, m.j2, a.nx, a.ny) && m.wing >= 0 && m.wing < a.nwing;
-}
-
 // the marker at position srt of the solve order, or null (and the kernel's
 // status bit set) when the order holds an index outside the markers or the
 // marker is not as make_marker leaves it
@@ -357,36 +285,6 @@ __device__ __forceinline__ const Marker *sorted_marker(const IBArgs &a, int srt,
     }
     return a.mk + k;
 }
-
-// marker at position s of the solve order, or -1 (and the kernel's status
-// bit set) when the order holds an index outside the markers
-__device__ __forceinline__ int order_at(const IBArgs &a, int s, unsigned bit)
-{
-    const int k = a.perm[s];
-    if (k < 0 || k >= a.nseg) {
-        atomicOr(a.status, bit);
-        return -1;
-    }
-    return k;
-}
-
-// tiles of the patch grid (the tile lists of one slot)
-__device__ __forceinline__ int patch_tiles(const IBArgs &a) { return (int)(a.st_tiles / (TILE_CAP + 1)); }
-
-// time and motion columns of this step's force.dat row (solution.f90:350-375)
-__device__ void write_header(const IBArgs &a, const double *row, double time, int ring_slot)
-{
-    double *fr = a.force_ring + (long long)ring_slot * a.row_len;
-    fr[0] = time;
-    const int mc = 1 + 3 * a.nwing + 3;
-    for (int w = 0; w < a.nwing; ++w) {
-        const double *r = row + 1 + 9 * w;   // angle omega omgac sa sau saac sb sbv sbac
-        double *o = fr + mc + 9 * w;         // solution.f90:363-374 order
-        o[0] = r[3]; o[1] = r[4]; o[2] = r[5]; o[3] = r[6]; o[4] = r[7]; o[5] = r[8];
-        o[6] = r[0]; o[7] = r[1]; o[8] = r[2];
-    }
-}
-
 
 // Several bodies: sort the markers along the longer axis of the marker cloud
 // (stable, ties by index) into perm/key, with reach = 6 lattice units along
@@ -655,36 +553,6 @@ __device__ void dense_factor(const IBArgs &a, int *bad)
     }
 }
 
-// dense fallback, solve: L z = r, then L^T y = z, for the two right-hand
-// sides yv[0..n) and yv[n..2n) (shared memory), whole CTA
-__device__ void dense_tri(const IBArgs &a, double *yv)
-{
-    const int n = a.nseg, tid = threadIdx.x, nt = blockDim.x;
-    const double *L = a.B;
-    for (int k = 0; k < n; ++k) {
-        const double dk = L[(long long)k * n + k];
-        const double z0 = yv[k] / dk, z1 = yv[n + k] / dk;
-        __syncthreads();
-        if (tid == 0) { yv[k] = z0; yv[n + k] = z1; }
-        for (int i = k + 1 + tid; i < n; i += nt) {
-            const double lik = L[(long long)i * n + k];
-            yv[i] -= lik * z0;
-            yv[n + i] -= lik * z1;
-        }
-        __syncthreads();
-    }
-    for (int j = n - 1; j >= 0; --j) {
-        if (tid < 2) yv[tid * n + j] /= L[(long long)j * n + j];
-        __syncthreads();
-        for (int q = tid; q < 2 * j; q += nt) {
-            const int c = q / j, i = q % j;
-            yv[c * n + i] -= L[(long long)j * n + i] * yv[c * n + j];
-        }
-        __syncthreads();
-    }
-}
-
-
 // Factorization of one step's D D^T, one CTA of FACTOR_THREADS threads;
 // dynamic shared memory: one block-operation workspace of WS doubles per warp.
 // Block cyclic reduction: at stride st the active blocks are the multiples
@@ -885,10 +753,7 @@ __global__ void __launch_bounds__(FACTOR_THREADS, 65536 / (FACTOR_THREADS * 128)
 // instead of one per dependent load. The levels above the first usually fit
 // together (31 blocks for 1024 markers): they then come in one round trip and
 // serve both sweeps, so that the whole solve stages three times (level 1,
-// the levels above it, level 1 again) instead of twice per level. Rows of a block are GW = 96 words apart,
-// all on one bank: the backward sweep, which reads one row per lane pair,
-// walks the columns in a rotated order (lane row i starts at column i) so
-// that the 16 rows read in one step fall on distinct banks. Also writes the force row's header and reports the
+// the levels above it, level 1 again) instead of twice per level. Also writes the force row's header and reports the
 // errors of the factorization chain. Dynamic shared memory: the staged
 // blocks, then the right-hand sides in the solve order (two per marker,
 // padded to whole blocks), then the mbarrier.
@@ -936,7 +801,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1024 / SOLVE_THREADS) ib_solve(
             X[n + s] = k >= 0 ? a.rhs[n + k] : 0.0;
         }
         __syncthreads();
-        dense_tri(a, X);
+        dense_tri(a, X, nt);
         for (int s = tid; s < n; s += nt) {
             const int k = order_at(a, s, LBM_ST_INDEX_SOLVE);
             if (k < 0) continue;
@@ -1020,51 +885,27 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1024 / SOLVE_THREADS) ib_solve(
         return stage_level(st) ? 0 : -1;
     };
     __syncthreads();
-    const int i = lane >> 1, c = lane & 1;   // row of the block, right-hand side
     int levels = 0;
     for (int st = 1; st < nb; st <<= 1, ++levels) {
         const int sbase = level_base(st, true);
         const bool staged = sbase >= 0;
         if (timed_out) break;
         const int neven = (nb + 2 * st - 1) / (2 * st);
-        // one even block e per warp: F_L(q) and F_U(p) from block bases that
-        // are either staged (shared memory, row stride GW) or global (GW);
-        // the two forms are separate so that staged reads stay shared loads
-        auto fwd = [&](const double *Fq, const double *Fp, int ld, int e, bool has_q, bool has_p) {
-            double acc = 0.0;
-            if (has_q) {
-                const double *F = Fq + BS + i;       // F_L(q)[t][i]
-                const double *r = X + 2 * (e + st) * BS + c;
-#pragma unroll
-                for (int t = 0; t < BS; ++t) acc += F[t * ld] * r[2 * t];
-            }
-            if (has_p) {
-                const double *F = Fp + 2 * BS + i;   // F_U(p)[t][i]
-                const double *r = X + 2 * (e - st) * BS + c;
-#pragma unroll
-                for (int t = 0; t < BS; ++t) acc += F[t * ld] * r[2 * t];
-            }
-            X[2 * (e * BS + i) + c] -= acc;
-        };
+        // one even block e per warp, F_L(q) and F_U(p) from staged blocks or
+        // from global memory
         for (int m = warp; m < neven; m += nw) {
             const int e = 2 * st * m, o1 = e - st, o2 = e + st;
             const bool has_q = o2 < nb, has_p = m > 0;
             if (staged)   // odd block st(2k+1) is staged at index sbase + k
-                fwd(stage_buf + (sbase + m) * BS * GW, stage_buf + (sbase + m - 1) * BS * GW, GW, e, has_q, has_p);
+                bcr_forward(stage_buf + (sbase + m) * BS * GW, stage_buf + (sbase + m - 1) * BS * GW, X, e, st, has_q, has_p,
+                            lane);
             else
-                fwd(Gf + (long long)o2 * BS * GW, Gf + (long long)o1 * BS * GW, GW, e, has_q, has_p);
+                bcr_forward(Gf + (long long)o2 * BS * GW, Gf + (long long)o1 * BS * GW, X, e, st, has_q, has_p, lane);
         }
         __syncthreads();
     }
     if (!timed_out) {
-        if (warp == 0) {
-            const double *G = Gf + i * GW;
-            double x = 0.0;
-#pragma unroll
-            for (int t = 0; t < BS; ++t) x += G[t] * X[2 * t + c];
-            __syncwarp();
-            X[lane] = x;
-        }
+        if (warp == 0) bcr_root(Gf, GW, X, lane);
         __syncthreads();
         for (int lv = levels - 1; lv >= 0; --lv) {
             const int st = 1 << lv;
@@ -1072,31 +913,12 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1024 / SOLVE_THREADS) ib_solve(
             const bool staged = sbase >= 0;
             if (timed_out) break;
             const int nodd = (nb - st + 2 * st - 1) / (2 * st);
-            auto bwd = [&](const double *G, int o) {
-                const int p = o - st, q2 = o + st;
-                double s1 = 0.0, s2 = 0.0, s3 = 0.0;
-#pragma unroll
-                for (int t0 = 0; t0 < BS; ++t0) {
-                    const int t = (t0 + i) & (BS - 1);   // rotated column order
-                    s1 += G[t] * X[2 * (o * BS + t) + c];
-                    s2 += G[BS + t] * X[2 * (p * BS + t) + c];
-                }
-                if (q2 < nb) {
-#pragma unroll
-                    for (int t0 = 0; t0 < BS; ++t0) {
-                        const int t = (t0 + i) & (BS - 1);
-                        s3 += G[2 * BS + t] * X[2 * (q2 * BS + t) + c];
-                    }
-                }
-                __syncwarp();
-                X[2 * (o * BS + i) + c] = s1 - s2 - s3;
-            };
             for (int m = warp; m < nodd; m += nw) {
                 const int o = st * (2 * m + 1);
                 if (staged)
-                    bwd(stage_buf + ((sbase + m) * BS + i) * GW, o);
+                    bcr_backward(stage_buf + (sbase + m) * BS * GW, X, o, st, o + st < nb, lane);
                 else
-                    bwd(Gf + ((long long)o * BS + i) * GW, o);
+                    bcr_backward(Gf + (long long)o * BS * GW, X, o, st, o + st < nb, lane);
             }
             __syncthreads();
         }
@@ -1250,10 +1072,8 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) ib_tile_sort(const IBArgs bas
 // compact tile list in ascending tile order (deterministic), one CTA; no
 // correction tile gives zero forces (solution.f90:327-330 normalisation).
 // Needed by no kernel of the step, so it runs after the step's update.
-template <bool BATCH>
-__global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *batch, int ring_slot)
+__device__ __forceinline__ void force_row(const IBArgs &a, int rr)
 {
-    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
     __shared__ double red[8][NPART];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nt = patch_tiles(a);
@@ -1283,7 +1103,6 @@ __global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int rr = BATCH ? a.ring_row : ring_slot;
         if (rr < 0 || rr >= a.ring_rows) {
             atomicOr(a.status, LBM_ST_INDEX_FORCES);
             return;
@@ -1305,6 +1124,26 @@ __global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *
         fr[2 + 3 * a.nwing] = tot[1];
         fr[3 + 3 * a.nwing] = tot[2];
     }
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *batch, int ring_slot)
+{
+    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
+    force_row(a, BATCH ? a.ring_row : ring_slot);
+}
+
+// the force rows of consecutive steps (CTA b: step step0 + b), headers included
+__global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, int step0, int ring0)
+{
+    const int step = step0 + (int)blockIdx.x, rr = ring0 + (int)blockIdx.x;
+    const IBArgs a = step_args(a0, step);
+    if (threadIdx.x == 0 && rr >= 0 && rr < a.ring_rows) {
+        double time;
+        const double *row = motion_row(a, step, &time);
+        write_header(a, row, time, rr);
+    }
+    force_row(a, rr);
 }
 
 // Residual of the step's solve, ||B y - rhs|| / ||rhs|| with B = D D^T
@@ -1403,14 +1242,7 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
 {
     const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
     const KFArgs<C> &kf = BATCH ? kbatch[blockIdx.z] : kf0;
-    __shared__ int wsum[8];
-    __shared__ int nlist;
-    __shared__ double red[8][NPART];
-    // markers whose support box meets the current tile, staged in marker order
-    __shared__ int4 sbox[256];
-    __shared__ double sph[256][12];
-    __shared__ double sy[256][2];
-    __shared__ int swing[256];
+    __shared__ TileSmem S;
     const int nt = patch_tiles(a);
     const int ntile = *a.nsup;
     if (ntile == 0) return;   // no correction tile
@@ -1451,36 +1283,15 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
         int wing = 1 << 20;
         if (listed <= TILE_CAP) {
             // markers listed for this tile by the factorization chain
-            if (threadIdx.x == 0) nlist = listed;
             if ((int)threadIdx.x < listed) {
                 const int k = tlist[1 + threadIdx.x];
-                if (k >= 0 && k < a.nseg && marker_ok(a, a.mk[k])) {
-                    const Marker &m = a.mk[k];
-                    sbox[threadIdx.x] = mbox(m);
-#pragma unroll
-                    for (int q = 0; q < 6; ++q) { sph[threadIdx.x][q] = m.phx[q]; sph[threadIdx.x][6 + q] = m.phy[q]; }
-                    sy[threadIdx.x][0] = a.y[k];
-                    sy[threadIdx.x][1] = a.y[a.nseg + k];
-                    swing[threadIdx.x] = m.wing;
-                } else {   // not staged: an empty box meets no node
-                    atomicOr(a.status, LBM_ST_INDEX_TILE);
-                    sbox[threadIdx.x] = make_int4(1, 0, 1, 0);
-                    sy[threadIdx.x][0] = sy[threadIdx.x][1] = 0.0;
-                    swing[threadIdx.x] = 0;
+                if (tile_stage(a, S, threadIdx.x, k)) {
+                    S.y[threadIdx.x][0] = a.y[k];
+                    S.y[threadIdx.x][1] = a.y[a.nseg + k];
                 }
             }
             __syncthreads();
-            if (active) {
-                for (int t = 0; t < nlist; ++t) {
-                    const int4 b = sbox[t];
-                    if (gi >= b.x && gi <= b.y && gj >= b.z && gj <= b.w) {
-                        const double wgt = sph[t][gi - b.x] * sph[t][6 + gj - b.z];
-                        du += wgt * sy[t][0];
-                        dv += wgt * sy[t][1];
-                        wing = min(wing, swing[t]);
-                    }
-                }
-            }
+            if (active) tile_gather(S, 0, listed, gi, gj, du, dv, wing);
         } else {
             // more markers than a list holds: scan all of them, in order
             for (int c0 = 0; c0 < a.nseg; c0 += 256) {
@@ -1496,36 +1307,23 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
                     }
                 }
                 const unsigned bal = __ballot_sync(0xffffffffu, hit);
-                if (lane == 0) wsum[warp] = __popc(bal);
+                if (lane == 0) S.wsum[warp] = __popc(bal);
                 __syncthreads();
                 if (threadIdx.x == 0) {
                     int acc = 0;
-                    for (int w = 0; w < 8; ++w) { const int t = wsum[w]; wsum[w] = acc; acc += t; }
-                    nlist = acc;
+                    for (int w = 0; w < 8; ++w) { const int t = S.wsum[w]; S.wsum[w] = acc; acc += t; }
+                    S.nlist = acc;
                 }
                 __syncthreads();
                 if (hit) {
-                    const int slot = wsum[warp] + __popc(bal & ((1u << lane) - 1u));
-                    const Marker &m = a.mk[k];
-                    sbox[slot] = q;
-#pragma unroll
-                    for (int r = 0; r < 6; ++r) { sph[slot][r] = m.phx[r]; sph[slot][6 + r] = m.phy[r]; }
-                    sy[slot][0] = a.y[k];
-                    sy[slot][1] = a.y[a.nseg + k];
-                    swing[slot] = m.wing;
-                }
-                __syncthreads();
-                if (active) {
-                    for (int t = 0; t < nlist; ++t) {
-                        const int4 b = sbox[t];
-                        if (gi >= b.x && gi <= b.y && gj >= b.z && gj <= b.w) {
-                            const double wgt = sph[t][gi - b.x] * sph[t][6 + gj - b.z];
-                            du += wgt * sy[t][0];
-                            dv += wgt * sy[t][1];
-                            wing = min(wing, swing[t]);
-                        }
+                    const int slot = S.wsum[warp] + __popc(bal & ((1u << lane) - 1u));
+                    if (tile_stage(a, S, slot, k)) {
+                        S.y[slot][0] = a.y[k];
+                        S.y[slot][1] = a.y[a.nseg + k];
                     }
                 }
+                __syncthreads();
+                if (active) tile_gather(S, 0, S.nlist, gi, gj, du, dv, wing);
                 __syncthreads();
             }
         }
@@ -1536,40 +1334,13 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
             C gout[9], frho, fu, fv;
             lbm_node::collide_interior<C>(kf, g, true, (C)du, (C)dv, gout, frho, fu, fv);
             lbm_node::store_node<T, C, FIELDS>(kf, (T *)kf.fout, gi, gj, gout, frho, fu, fv);
-            if (in_support) {
-                // FP64 density of the same streamed populations
-                const double drho = (((double)g[0] + (double)g[1]) + ((double)g[2] + (double)g[3])) +
-                                    (((double)g[4] + (double)g[5]) + ((double)g[6] + (double)g[7])) + (double)g[8];
-                const double rho = 1.0 + drho;
-                const double *row = motion_row(a, BATCH ? a.cur_step : step_index, nullptr);
-                const double temp1 = 2.0 * rho * du, temp2 = 2.0 * rho * dv;
-                const double sa = row[4 + 9 * wing], sb = row[7 + 9 * wing];
-                fx = -temp1;
-                fy = -temp2;
-                const double x0 = (a.ox + a.scale * (double)gi - (a.xc + sa)) / a.scale;
-                const double y0 = (a.oy + a.scale * (double)gj - (a.yc + sb)) / a.scale;
-                mz = -x0 * temp2 + y0 * temp1;
-            }
+            if (in_support)
+                node_force(a, motion_row(a, BATCH ? a.cur_step : step_index, nullptr), g, gi, gj, wing, du, dv, fx, fy, mz);
         }
         // deterministic tile reduction per wing, into the tile's partials
-        for (int w = 0; w < a.nwing; ++w) {
-            double v0 = (in_support && wing == w) ? fx : 0.0;
-            double v1 = (in_support && wing == w) ? fy : 0.0;
-            double v2 = (in_support && wing == w) ? mz : 0.0;
-#pragma unroll
-            for (int off = 16; off; off >>= 1) {
-                v0 += __shfl_down_sync(0xffffffffu, v0, off);
-                v1 += __shfl_down_sync(0xffffffffu, v1, off);
-                v2 += __shfl_down_sync(0xffffffffu, v2, off);
-            }
-            if (lane == 0) { red[warp][3 * w] = v0; red[warp][3 * w + 1] = v1; red[warp][3 * w + 2] = v2; }
-        }
+        tile_force_warp(a, S, in_support, wing, fx, fy, mz, warp, lane);
         __syncthreads();
-        if (threadIdx.x < 3 * a.nwing) {
-            double sum = 0.0;
-            for (int w8 = 0; w8 < 8; ++w8) sum += red[w8][threadIdx.x];
-            a.partial[(long long)tile * NPART + threadIdx.x] = sum;
-        }
+        tile_force_store(a, S, tile, threadIdx.x);
         __syncthreads();   // shared arrays are reused by the next tile
     }
 }
@@ -1636,21 +1407,21 @@ IBArgs make_args(lbm_handle *h, const void *fin, int slot)
     a.st_tiles = (long long)h->patch_gx() * h->patch_gy() * (TILE_CAP + 1);
     a.tiles = h->d_tiles + slot * a.st_tiles;
     a.gf = h->d_gf + slot * h->gf_slot;
-    // the step's own right-hand sides, solution, tile partials and residual
-    // slots: one set per step parity, so that the check of a step may run
-    // while the next step's flow chain fills the other set
-    const int par = h->n & 1;
-    const long long ns2 = 2ll * (h->nseg > 0 ? h->nseg : 1);
-    a.rhs = h->d_rhs + par * ns2; a.y = h->d_y + par * ns2;
+    // the step's own right-hand sides, solution, tile partials and residual,
+    // one set per slot: the check of a step may run while later steps' flow
+    // chains fill theirs
+    a.st_rhs = 2ll * (long long)ns;
+    a.st_part = (long long)h->part_stride;
+    a.rhs = h->d_rhs + slot * a.st_rhs; a.y = h->d_y + slot * a.st_rhs;
     a.bD = h->d_bD; a.bL = h->d_bL;
     a.reach = h->d_reach; a.wmax = h->d_wmax;
     a.nsup = h->d_nsup + slot;
     a.ctile = h->d_ctile + slot * (a.st_tiles / (TILE_CAP + 1));
     a.patch_wmax = h->patch_wmax; a.patch_hmax = h->patch_hmax;
-    a.partial = h->d_partial + par * (long long)h->part_stride; a.counter = h->d_counter;
+    a.partial = h->d_partial + slot * a.st_part; a.counter = h->d_counter;
     a.force_ring = h->d_ring; a.row_len = h->row_len;
     a.ring_row = 0; a.ring_rows = h->ring_cap;
-    a.status = h->d_status; a.solve_res = h->d_solve_res + 2 * par;
+    a.status = h->d_status; a.solve_res = h->d_solve_res + 2 * slot;
     a.cur_step = h->n;
     a.fstep0 = 0; a.fcount = 0;
     a.check_res = 1;
@@ -1747,6 +1518,20 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st)
     const int sort_ctas = std::min((h->patch_gx() * h->patch_gy() + SORT_WARPS - 1) / SORT_WARPS, SORT_CTAS);
     ib_tile_sort<false><<<dim3(sort_ctas, count), 32 * SORT_WARPS, 0, st>>>(a, nullptr, step0);
     h->launches += h->static_order ? 6 : 7;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_check_steps(lbm_handle *h, int step0, int count, int ring_slot, bool last, cudaStream_t st)
+{
+    const IBArgs a = make_args(h, nullptr, 0);
+    ib_forces_steps<<<count, 256, 0, st>>>(a, step0, ring_slot);
+    h->launches += count;   // a force row each
+    for (int t = 0; t < count; ++t) {
+        if (!check_due(step0 + t) && !(last && t == count - 1)) continue;
+        const IBArgs b = make_args(h, nullptr, (step0 + t) % h->nslots);
+        ib_residual<false><<<(h->nseg + 7) / 8, 256, 0, st>>>(b, nullptr);
+        h->launches += 1;
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -612,7 +612,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 IBArgs *ia = (IBArgs *)(hs + ((size_t)t * na + c) * b->ib_sz);
                 ib_args_write(h, h->fbuf[h->cur], q, ia);
                 // a segment holds neither the call's nor a case's last step
-                ia->check_res = (h->n + 1) % K == 0;
+                ia->check_res = check_due(h->n);
                 p.residual = p.residual || ia->check_res;
                 ia->ring_row = pending + t;
                 kf_args_write(h, h->fbuf[h->cur], h->fbuf[h->cur ^ 1], nullptr, KF_OUTER,
@@ -781,8 +781,11 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 act_idx.push_back(c);
             }
         if (act.empty()) break;
-        // a graph segment where the next kGraphSteps steps allow one
-        if (b->graphs && tcur >= 0 && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
+        // a graph segment where the next kGraphSteps steps allow one. Segments
+        // start at every half of a factorization batch (of the first case),
+        // so that runs of any length need two structures, not one for each
+        // phase of the batch
+        if (b->graphs && act[0]->n % std::max(1, K / 2) == 0 && tcur >= 0 && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
             pending + kGraphSteps <= ring_cap) {
             bool ok = true;
             for (size_t c = 0; c < act.size() && ok; ++c) ok = act[c]->n + kGraphSteps < last_step[act_idx[c]];
@@ -820,9 +823,9 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             h->pinfo_slot = q;
             IBArgs *ia = (IBArgs *)((char *)b->h_sargs[buf] + c * b->ib_sz);
             ib_args_write(h, fin, q, ia);
-            // the solve-residual check: last step of the case's factorization
-            // batch, of the call, or of the case's motion
-            ia->check_res = (h->n + 1) % K == 0 || step == nsteps - 1 || h->n >= last_step[act_idx[c]];
+            // the solve-residual check: every kCheckEvery-th step of the case, the
+            // last step of the call, or of the case's motion
+            ia->check_res = check_due(h->n) || step == nsteps - 1 || h->n >= last_step[act_idx[c]];
             any_check = any_check || ia->check_res;
             ia->ring_row = pending;
             kf_args_write(h, fin, fout, fd, KF_OUTER, (char *)b->h_kargs[buf] + c * b->kf_sz);

@@ -20,6 +20,7 @@ const double kWref[9] = {4.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0, 1.0 / 9.0,
 const int kEx[9] = {0, 1, 0, -1, 0, 1, -1, -1, 1};
 const int kEy[9] = {0, 0, 1, 0, -1, 1, 1, -1, -1};
 const int kRing = 2048;   // force rows kept on the device between host copies
+const int kLoopSpare = 16;   // SMs left free beside a step_loop launch
 
 
 int set_err(lbm_handle *h, int code, const char *msg)
@@ -286,9 +287,8 @@ int ensure_ib(lbm_handle *h)
     const int ns = std::max(1, h->nseg);
     const size_t S = (size_t)h->nslots, K = (size_t)h->fbatch;
     CK(dmalloc(h, &h->d_mk, S * sizeof(Marker) * ns), "alloc markers");
-    // right-hand sides and solution: one pair per step parity
-    CK(dmalloc(h, &h->d_rhs, sizeof(double) * 2 * 2 * ns), "alloc rhs");
-    CK(dmalloc(h, &h->d_y, sizeof(double) * 2 * 2 * ns), "alloc y");
+    CK(dmalloc(h, &h->d_rhs, S * sizeof(double) * 2 * ns), "alloc rhs");
+    CK(dmalloc(h, &h->d_y, S * sizeof(double) * 2 * ns), "alloc y");
     CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
     ib_factor_scratch(ns, &h->work_blocks, &h->gf_slot);
     CK(dmalloc(h, &h->d_bD, K * sizeof(double) * h->work_blocks), "alloc block D");
@@ -299,11 +299,11 @@ int ensure_ib(lbm_handle *h)
     CK(cudaMemsetAsync(h->d_fmode, 0, S * 2 * sizeof(int), h->stream), "clear factor mode");
     CK(cudaMemsetAsync(h->d_fstatus, 0, S * sizeof(unsigned), h->stream), "clear factor status");
     const int nblk = h->patch_gx() * h->patch_gy();
-    // partials of the spread (per patch tile) and of the residual check (per 8 markers)
-    // (one set per step parity)
+    // partials of the spread (per patch tile) and of the residual check (per 8
+    // markers), per slot
     const size_t npart = std::max((size_t)ib_partials_per_block() * nblk, 2 * (size_t)((ns + 7) / 8));
     h->part_stride = npart;
-    CK(dmalloc(h, &h->d_partial, sizeof(double) * 2 * npart), "alloc partials");
+    CK(dmalloc(h, &h->d_partial, S * sizeof(double) * npart), "alloc partials");
     h->tiles_slot = (size_t)ib_tile_ints() * nblk;
     CK(dmalloc(h, &h->d_tiles, S * sizeof(int) * h->tiles_slot), "alloc tile lists");
     CK(cudaMemsetAsync(h->d_tiles, 0, S * sizeof(int) * h->tiles_slot, h->stream), "clear tile lists");
@@ -396,6 +396,7 @@ int check_status(lbm_handle *h)
     CK(cudaStreamSynchronize(h->stream), "step sync");
     if (!st) return LBM_OK;
     CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream), "clear status");
+    if (st & LBM_ST_TIMEOUT) CK(loop_reset(h), "reset step loop");
     std::string msg;
     const int code = status_error(st, msg);
     return set_err(h, code, msg.c_str());
@@ -494,10 +495,85 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         return LBM_OK;
     };
     int done = 0, pending = 0;
+    // a small lattice's steps run as step_loop launches; per-kernel timing
+    // needs the kernels one by one
+    const bool loop = split && h->timing != LBM_TIMING_KERNELS && loop_fits(h);
+    bool joined = loop;   // nothing queued on the side and check streams since the last flush
+    // force rows, mass check, status and timing of the steps since the last flush
+    auto flush = [&]() -> int {
+        if (split && !joined) {   // force rows and residual checks run on the check stream after the update
+            CK(cudaEventRecord(h->ev_ib, h->side), "event");
+            CK(cudaStreamWaitEvent(h->stream, h->ev_ib, 0), "wait");
+            CK(cudaEventRecord(h->ev_cjoin, h->cstream), "event");
+            CK(cudaStreamWaitEvent(h->stream, h->ev_cjoin, 0), "wait");
+            joined = loop;
+        }
+        // the span ends with the chunk's last step; the row copy and the
+        // mass check after it are per-call work, not per-step work
+        if (h->timing == LBM_TIMING_SPAN) CK(cudaEventRecord(h->ev[4 * (pending - 1) + 3], h->stream), "event");
+        if (rows_out)
+            CK(cudaMemcpyAsync(rows_out + (size_t)(done - pending) * h->row_len, h->d_ring,
+                               sizeof(double) * h->row_len * pending, cudaMemcpyDeviceToHost, h->stream),
+               "copy force rows");
+        double dsum = 0.0;
+        const bool mass = mass_due();
+        int st = mass ? mass_launch(h, h->stream, &dsum) : LBM_OK;
+        if (st) return st;
+        st = check_status(h);
+        if (st) return st;
+        if (mass && (st = mass_result(h, dsum))) return st;
+        if (h->timing && (st = collect_timing(h, pending, split))) return st;
+        pending = 0;
+        return LBM_OK;
+    };
     rc = LBM_OK;
     for (int s = 0; s < nsteps; ++s) {
         const double time = (double)(h->n - 1) * dt_time;   // main.f90:352
         if (time > h->mend + 1.0e-12) { rc = LBM_DONE; break; }
+        if (loop) {
+            // as many steps as the slot half, the force ring, the call and the
+            // motion hold, in one launch
+            const int b = h->n / K, half = b & 1;
+            int m = 1;
+            while (m < nsteps - s && (h->n + m) / K == b && pending + m < h->ring_cap &&
+                   (double)(h->n + m - 1) * dt_time <= h->mend + 1.0e-12)
+                ++m;
+            if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
+            // the next batch's factorization, beside this launch (it waits for
+            // the previous one, not for this one)
+            if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
+            void *fields[LBM_NSLOT_MAX] = {};
+            for (int t = 0; t < m; ++t)
+                if (fields_every || s + t >= nsteps - 2) {
+                    const int fs = h->fields_slot ^ 1;
+                    fields[t] = h->d_fields[fs];
+                    h->fields_slot = fs;
+                    h->fields_step[fs] = h->n + t;
+                }
+            if (h->timing == LBM_TIMING_SPAN && pending == 0) CK(cudaEventRecord(h->ev[0], h->stream), "event");
+            CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
+            if (launch_loop(h, m, fields, h->stream)) return cuda_err(h, cudaGetLastError(), "launch step loop");
+            CK(cudaEventRecord(h->ev_inner, h->stream), "event");
+            // force rows and residual checks beside the next launch; those of
+            // a call that is one launch have nothing to run beside
+            cudaStream_t cs = joined && s + m == nsteps ? h->stream : h->cstream;
+            if (cs != h->stream) {
+                CK(cudaStreamWaitEvent(cs, h->ev_inner, 0), "wait");
+                joined = false;
+            }
+            if (launch_check_steps(h, h->n, m, pending, s + m == nsteps, cs))
+                return cuda_err(h, cudaGetLastError(), "launch check");
+            CK(cudaEventRecord(h->ev_free[half], cs), "event");
+            if (m & 1) h->cur ^= 1;
+            h->n += m;
+            h->steps_done += m;
+            done += m;
+            pending += m;
+            s += m - 1;
+            if (pending == h->ring_cap || s == nsteps - 1)
+                if ((rc = flush())) return rc;
+            continue;
+        }
         const int slot = pending, b = h->n / K, half = b & 1, q = h->n % h->nslots;
         h->pinfo_slot = q;
         const void *fin = h->fbuf[h->cur];
@@ -514,18 +590,15 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         // first step's start and the last step's end of each chunk of steps
         cudaEvent_t *e = h->timing == LBM_TIMING_KERNELS ? &h->ev[4 * slot] : nullptr;
         if (h->timing == LBM_TIMING_SPAN && slot == 0) CK(cudaEventRecord(h->ev[0], h->stream), "event");
-        // the solve-residual check: on the last step of each factorization
-        // batch and on the last step of the call
-        const bool check_res = (h->n + 1) % K == 0 || s == nsteps - 1;
+        // the solve-residual check: on every kCheckEvery-th step and on the
+        // last step of the call
+        const bool check_res = check_due(h->n) || s == nsteps - 1;
         if (split) {
             // side stream: the immersed-boundary chain and the correction
             // tiles; main stream: every other node, concurrently
             if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
             CK(cudaStreamWaitEvent(h->side, h->ev_inner, 0), "wait");
             CK(cudaStreamWaitEvent(h->side, h->ev_batch[half], 0), "wait");
-            // this step's buffers of its parity were last read by the check
-            // two steps back
-            CK(cudaStreamWaitEvent(h->side, h->ev_check[h->n & 1], 0), "wait");
             if (e) CK(cudaEventRecord(h->ev_side[2 * slot], h->side), "event");
             cudaEvent_t ei = h->after_interp ? h->ev_interp : nullptr;
             if (launch_flow(h, fin, fout, fields, h->n, slot, q, h->side, ei)) return cuda_err(h, cudaGetLastError(), "launch ib");
@@ -535,7 +608,6 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             // slot half is free for the next factorization after them
             CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
             if (launch_check(h, q, slot, check_res, h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
-            CK(cudaEventRecord(h->ev_check[h->n & 1], h->cstream), "event");
             CK(cudaEventRecord(h->ev_free[half], h->cstream), "event");
             // the next batch's factorization, overlapping this batch's steps
             if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
@@ -568,50 +640,13 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         done++;
         pending++;
         if (pending == h->ring_cap || s == nsteps - 1) {
-            if (split) {   // force rows and residual checks run on the check stream after the update
-                CK(cudaEventRecord(h->ev_ib, h->side), "event");
-                CK(cudaStreamWaitEvent(h->stream, h->ev_ib, 0), "wait");
-                CK(cudaEventRecord(h->ev_cjoin, h->cstream), "event");
-                CK(cudaStreamWaitEvent(h->stream, h->ev_cjoin, 0), "wait");
-            }
-            // the span ends with the chunk's last step; the row copy and the
-            // mass check after it are per-call work, not per-step work
-            if (h->timing == LBM_TIMING_SPAN) CK(cudaEventRecord(h->ev[4 * (pending - 1) + 3], h->stream), "event");
-            if (rows_out)
-                CK(cudaMemcpyAsync(rows_out + (size_t)(done - pending) * h->row_len, h->d_ring,
-                                   sizeof(double) * h->row_len * pending, cudaMemcpyDeviceToHost, h->stream),
-                   "copy force rows");
-            double dsum = 0.0;
-            const bool mass = mass_due();
-            int st = mass ? mass_launch(h, h->stream, &dsum) : LBM_OK;
+            const int st = flush();
             if (st) return st;
-            st = check_status(h);
-            if (st) return st;
-            if (mass && (st = mass_result(h, dsum))) return st;
-            if (h->timing && (st = collect_timing(h, pending, split))) return st;
-            pending = 0;
         }
     }
     if (pending) {
-        if (split) {
-            CK(cudaEventRecord(h->ev_ib, h->side), "event");
-            CK(cudaStreamWaitEvent(h->stream, h->ev_ib, 0), "wait");
-            CK(cudaEventRecord(h->ev_cjoin, h->cstream), "event");
-            CK(cudaStreamWaitEvent(h->stream, h->ev_cjoin, 0), "wait");
-        }
-        if (h->timing == LBM_TIMING_SPAN) CK(cudaEventRecord(h->ev[4 * (pending - 1) + 3], h->stream), "event");
-        if (rows_out)
-            CK(cudaMemcpyAsync(rows_out + (size_t)(done - pending) * h->row_len, h->d_ring,
-                               sizeof(double) * h->row_len * pending, cudaMemcpyDeviceToHost, h->stream),
-               "copy force rows");
-        double dsum = 0.0;
-        const bool mass = mass_due();
-        int st = mass ? mass_launch(h, h->stream, &dsum) : LBM_OK;
+        const int st = flush();
         if (st) return st;
-        st = check_status(h);
-        if (st) return st;
-        if (mass && (st = mass_result(h, dsum))) return st;
-        if (h->timing && (st = collect_timing(h, pending, split))) return st;
     }
     if (done_out) *done_out = done;
     return rc;
@@ -816,8 +851,7 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     if ((e = cudaStreamCreateWithFlags(&h->fstream, cudaStreamNonBlocking)) != cudaSuccess) return fail(e, "factor stream");
     if ((e = cudaStreamCreateWithPriority(&h->cstream, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(e, "check stream");
-    for (cudaEvent_t *ev : {&h->ev_check[0], &h->ev_check[1], &h->ev_cjoin})
-        if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
+    if ((e = cudaEventCreateWithFlags(&h->ev_cjoin, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
     for (int q = 0; q < 2; ++q) {
         if ((e = cudaEventCreateWithFlags(&h->ev_batch[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
         if ((e = cudaEventCreateWithFlags(&h->ev_free[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
@@ -828,6 +862,14 @@ int lbm_create(const lbm_params *p, lbm_t **out)
         if (v >= 1 && 2 * v <= LBM_NSLOT_MAX) h->fbatch = v;
     }
     h->nslots = 2 * h->fbatch;
+    {
+        // a CTA of the step loop fills an SM; kLoopSpare SMs stay free for the
+        // factorization of the next steps, which runs beside it
+        int sms = 0, coop = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev);
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, h->dev);
+        h->loop_ctas = coop && h->overlap && h->kf_tma ? std::max(0, sms - kLoopSpare) : 0;
+    }
     // population buffers carry LBM_FPAD elements of padding before and after
     // the 9 planes, so the bulk row copies of the lattice kernel (which read a
     // 16-byte halo left and right of every row segment) stay in bounds
@@ -848,8 +890,9 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     if ((e = dmalloc(h, &h->d_mass, sizeof(double) * mass_slots())) != cudaSuccess) return fail(e, "alloc mass");
     if ((e = dmalloc(h, &h->d_mcount, sizeof(unsigned))) != cudaSuccess) return fail(e, "alloc mass counter");
 
-    // solve residual and half-bandwidth, per step parity
-    if ((e = dmalloc(h, &h->d_solve_res, 2 * 2 * sizeof(double))) != cudaSuccess) return fail(e, "alloc res");
+    // solve residual and half-bandwidth, per slot
+    if ((e = dmalloc(h, &h->d_solve_res, LBM_NSLOT_MAX * 2 * sizeof(double))) != cudaSuccess) return fail(e, "alloc res");
+    if ((e = dmalloc(h, &h->d_sync, sizeof(unsigned) * loop_sync_words())) != cudaSuccess) return fail(e, "alloc sync");
     if ((e = dmalloc(h, &h->d_ring, sizeof(double) * h->row_len * (size_t)h->ring_cap)) != cudaSuccess)
         return fail(e, "alloc ring");
     if (h->npts > 0) {
@@ -878,7 +921,7 @@ int lbm_destroy(lbm_t *h)
     free_ib(h);
     free_devp(h->d_pinfo); free_devp(h->d_counter);
     free_devp(h->d_ring); free_devp(h->d_status); free_devp(h->d_solve_res); free_devp(h->d_red);
-    free_devp(h->d_mass); free_devp(h->d_mcount);
+    free_devp(h->d_mass); free_devp(h->d_mcount); free_devp(h->d_sync);
 
     free_devp(h->d_stage);
     if (h->side) cudaStreamSynchronize(h->side);
@@ -897,8 +940,7 @@ int lbm_destroy(lbm_t *h)
         if (h->ev_batch[q]) cudaEventDestroy(h->ev_batch[q]);
         if (h->ev_free[q]) cudaEventDestroy(h->ev_free[q]);
     }
-    for (cudaEvent_t ev : {h->ev_check[0], h->ev_check[1], h->ev_cjoin})
-        if (ev) cudaEventDestroy(ev);
+    if (h->ev_cjoin) cudaEventDestroy(h->ev_cjoin);
     if (h->cstream) cudaStreamDestroy(h->cstream);
     if (h->fstream) cudaStreamDestroy(h->fstream);
     if (h->side) cudaStreamDestroy(h->side);
@@ -1132,7 +1174,7 @@ int lbm_get_markers(lbm_t *h, double *xb2, double *yb2, double *solve_residual, 
     const Marker *last = h->d_mk + (size_t)((h->n - 1) % h->nslots) * h->nseg;   // slot of the last step
     CK(cudaMemcpyAsync(mk.data(), last, sizeof(Marker) * h->nseg, cudaMemcpyDeviceToHost, h->stream), "copy markers");
     double res[2] = {0, 0};
-    const double *last_res = h->d_solve_res + 2 * ((h->n - 1) & 1);   // parity of the last step
+    const double *last_res = h->d_solve_res + 2 * ((h->n - 1) % h->nslots);
     CK(cudaMemcpyAsync(res, last_res, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream), "copy res");
     CK(cudaStreamSynchronize(h->stream), "sync markers");
     for (int k = 0; k < h->nseg; ++k) {

@@ -111,6 +111,16 @@ template <> struct Store<__nv_bfloat16> {
     static __device__ __forceinline__ __nv_bfloat16 pack(float x) { return __float2bfloat16_rn(x); }
 };
 
+// How a kernel loads populations: through the read-only path (nothing writes
+// them while the kernel runs), or from L2 (other CTAs of the same launch wrote
+// them earlier in it)
+struct LdNc {
+    template <typename T> static __device__ __forceinline__ T ld(const T *p) { return __ldg(p); }
+};
+struct LdCg {
+    template <typename T> static __device__ __forceinline__ T ld(const T *p) { return __ldcg(p); }
+};
+
 // two adjacent 2-byte elements as one 32-bit word (low half: the lower
 // column) <-> a float2 (x: the lower column); the paired conversions round
 // each element to nearest, as the scalar ones above do
@@ -145,6 +155,13 @@ template <> struct Pair2<__nv_bfloat16> {
         return w;
     }
 };
+
+// a product rounded on its own, and one fused into an addition, whatever
+// surrounds them (see collide_moments, lbm_node.cuh)
+__device__ __forceinline__ float rmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double rmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float rfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double rfma(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // m = M g for the MRT matrix of solution.f90:17-25 (rows: rho, e, eps, jx, qx,
 // jy, qy, pxx, pxy), written out for its 0/+-1/+-2/+-4 entries.

@@ -80,6 +80,7 @@ struct IBArgs {
     int fstep0, fcount; // steps of the factorization chain (batched launches: per case)
     int check_res;      // batched launches: run the solve-residual check for this case's step
     long long st_mk, st_perm, st_B, wk_blocks, wk_gf;
+    long long st_rhs, st_part;   // right-hand sides (and solution) and tile partials of a slot
     PatchInfo *pinfo;
     int *tiles;         // per patch tile: marker count, then the listed markers (slot)
     int tiles_x;        // tiles per patch row
@@ -136,7 +137,7 @@ struct lbm_handle {
     // fbatch consecutive steps (batch b: steps b*fbatch .. b*fbatch+fbatch-1),
     // each step into slot step % nslots (nslots = 2 fbatch): the next batch
     // is factorized while the steps of the current one run.
-    int fbatch = 4, nslots = 8;
+    int fbatch = 8, nslots = 16;
     int batch_in_half[2] = {-1, -1};                // batch index held by each half of the slots
     Marker *d_mk = nullptr;                         // nslots x nseg
     double *d_B = nullptr;                          // nslots x nseg*nseg
@@ -179,12 +180,16 @@ struct lbm_handle {
     cudaEvent_t ev_batch[2] = {nullptr, nullptr}, ev_free[2] = {nullptr, nullptr};
     // the step's force row and solve-residual check (with the split): their
     // own stream, after the step's correction tiles, so that the next step's
-    // flow chain need not wait for them. What they read is kept per step
-    // parity (right-hand sides, solution, tile partials, residual slots), and
-    // ev_check[p] marks the check of the last step of parity p done.
+    // flow chain need not wait for them. What they read is kept per slot
+    // (right-hand sides, solution, tile partials, residual).
     cudaStream_t cstream = nullptr;
-    cudaEvent_t ev_check[2] = {nullptr, nullptr}, ev_cjoin = nullptr;
-    size_t part_stride = 0;   // doubles of one parity's tile partials
+    cudaEvent_t ev_cjoin = nullptr;
+    size_t part_stride = 0;   // doubles of one slot's tile partials
+    // steps of small lattices as step_loop launches: their CTA limit (0: not
+    // on this device or in this configuration) and counters
+    int loop_ctas = 0;
+    unsigned *d_sync = nullptr;
+    unsigned sync_base = 0;   // their step counter after the launches so far
     double *d_partial = nullptr;
     unsigned *d_counter = nullptr;
     double *d_ring = nullptr;
@@ -232,6 +237,18 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st);
 int launch_flow(lbm_handle *h, const void *fin, void *fout, void *fields, int step_index, int ring_slot, int slot,
                 cudaStream_t st, cudaEvent_t after_interp = nullptr);
 int launch_check(lbm_handle *h, int slot, int ring_slot, bool residual, cudaStream_t st);
+// force rows (headers included) and residual checks of the `count` steps from
+// step0 on, after their step_loop launch; a step is checked as check_due says,
+// and the last one if `last`
+int launch_check_steps(lbm_handle *h, int step0, int count, int ring_slot, bool last, cudaStream_t st);
+// the solve residual is checked on every kCheckEvery-th step
+constexpr int kCheckEvery = 4;
+inline bool check_due(int step) { return (step + 1) % kCheckEvery == 0; }
+// several steps in one launch (step_loop.cu)
+bool loop_fits(const lbm_handle *h);
+int loop_sync_words();
+cudaError_t loop_reset(lbm_handle *h);   // after a launch that gave up
+int launch_loop(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t st);
 // batches of cases stepped together (lbm_batch.cu)
 int handle_prepare_ib(lbm_handle *h);                    // immersed-boundary buffers (once per geometry)
 int handle_error(lbm_handle *h, int code, const char *msg);

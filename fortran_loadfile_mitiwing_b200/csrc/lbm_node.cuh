@@ -60,12 +60,12 @@ inline KFArgs<C> make_kf_args(lbm_handle *h, const void *fin, void *fout, void *
 
 namespace lbm_node {
 
-template <typename T, typename C>
+template <typename T, typename C, typename LD = LdNc>
 __device__ __forceinline__ void pull(const T *__restrict__ fin, long long plane, int pitch, int i, int j, C g[9])
 {
 #pragma unroll
     for (int k = 0; k < 9; ++k)
-        g[k] = (C)Store<T>::ld(fin + (long long)k * plane + (long long)(j - lbm_ey(k)) * pitch + (i - lbm_ex(k)));
+        g[k] = (C)Store<T>::cvt(LD::ld(fin + (long long)k * plane + (long long)(j - lbm_ey(k)) * pitch + (i - lbm_ex(k))));
 }
 
 template <typename C>
@@ -83,7 +83,7 @@ __device__ __forceinline__ void moments(const C g[9], C &drho, C &u, C &v)
 // (boundary_condition.f90:418-438 and :500-520). Returns the updated
 // (drho, u, v) at the edge node and the streamed populations + moments of its
 // first interior neighbour.
-template <typename T, typename C>
+template <typename T, typename C, typename LD = LdNc>
 __device__ __forceinline__ void side_bc(const KFArgs<C> &a, const T *__restrict__ fin, int side, int j, C &dr1,
                                         C &u1, C &v1, C g0n[9], C &drn, C &un, C &vn)
 {
@@ -91,9 +91,9 @@ __device__ __forceinline__ void side_bc(const KFArgs<C> &a, const T *__restrict_
     const C drs = col[3 * j], us = col[3 * j + 1], vs = col[3 * j + 2];
     const int in1 = side == 0 ? 1 : a.nx - 2, in2 = side == 0 ? 2 : a.nx - 3;
     C g2[9], dr2, u2, v2;
-    pull<T, C>(fin, a.plane, a.pitch, in1, j, g0n);
+    pull<T, C, LD>(fin, a.plane, a.pitch, in1, j, g0n);
     moments(g0n, drn, un, vn);
-    pull<T, C>(fin, a.plane, a.pitch, in2, j, g2);
+    pull<T, C, LD>(fin, a.plane, a.pitch, in2, j, g2);
     moments(g2, dr2, u2, v2);
     const C cs = a.cs, rhos = C(1) + drs;
     if (side == 0) {
@@ -123,16 +123,52 @@ __device__ __forceinline__ void side_bc(const KFArgs<C> &a, const T *__restrict_
 // CONS0: the relaxation rates of the conserved moments (s[0], s[3], s[5])
 // are zero, as the reference sets them (ini_mesh.f90:59-67); their terms of
 // the update are then left out at compile time.
-template <typename C, bool CONS0 = false>
-__device__ __forceinline__ void collide_interior(const KFArgs<C> &a, const C g[9], bool corr, C du, C dv, C gout[9],
-                                                 C &frho, C &fu, C &fv)
+// Two parts: what the streamed populations alone give, and the update.
+template <typename C> struct NodeMoments {
+    C u, v;    // uncorrected velocity
+    C m[9];    // M g; rows 0, 3, 5 are rho - 1 and the momentum
+};
+
+template <typename C>
+__device__ __forceinline__ NodeMoments<C> node_moments_of(const C g[9])
 {
     // physical_variables (solution.f90:471-542) on the deviations
+    NodeMoments<C> q;
     const C drho = ((g[0] + g[1]) + (g[2] + g[3])) + ((g[4] + g[5]) + (g[6] + g[7])) + g[8];
     const C jx0 = (g[1] - g[3]) + (g[5] - g[6]) + (g[8] - g[7]);
     const C jy0 = (g[2] - g[4]) + (g[5] + g[6]) - (g[7] + g[8]);
     const C rho = C(1) + drho;
-    C u = jx0 / rho, v = jy0 / rho;   // needed only for the fields and the correction
+    q.u = jx0 / rho;   // needed only for the fields and the correction
+    q.v = jy0 / rho;
+    // m = M g (solution.f90:580-600)
+    const C as = g[1] + g[2] + g[3] + g[4];
+    const C ds = g[5] + g[6] + g[7] + g[8];
+    const C dx = g[5] - g[6] - g[7] + g[8];
+    const C dy = g[5] + g[6] - g[7] - g[8];
+    q.m[0] = drho;
+    q.m[1] = rfma(C(2), ds, rfma(C(-4), g[0], -as));
+    q.m[2] = rfma(C(4), g[0], C(-2) * as) + ds;
+    q.m[3] = jx0;
+    q.m[4] = rfma(C(-2), g[1] - g[3], dx);
+    q.m[5] = jy0;
+    q.m[6] = rfma(C(-2), g[2] - g[4], dy);
+    q.m[7] = g[1] - g[2] + g[3] - g[4];
+    q.m[8] = g[5] - g[6] + g[7] - g[8];
+    return q;
+}
+
+// The update, its products rounded on their own (rmul) or fused as written
+// (rfma): the correction tiles and the step loop compile it in different
+// surroundings and have to agree bit for bit, while a sum of products leaves
+// the compiler the choice which one to fuse into the addition.
+template <typename C, bool CONS0 = false>
+__device__ __forceinline__ void collide_moments(const KFArgs<C> &a, const C g[9], const NodeMoments<C> &q, bool corr, C du,
+                                                C dv, C gout[9], C &frho, C &fu, C &fv)
+{
+    const C drho = q.m[0], jx0 = q.m[3], jy0 = q.m[5];
+    const C rho = C(1) + drho;
+    const C (&m)[9] = q.m;
+    C u = q.u, v = q.v;
     // j = rho u of the equilibrium: the summed momentum itself when there is
     // no correction (rho (jx/rho) = jx up to one rounding)
     C jx = jx0, jy = jy0;
@@ -140,60 +176,64 @@ __device__ __forceinline__ void collide_interior(const KFArgs<C> &a, const C g[9
     if (corr) {
         u = u + du;                       // boundary_condition.f90:1650-1651
         v = v + dv;
-        jx = rho * u;
-        jy = rho * v;
-        gx = C(2) * rho * du;             // :1652-1656
-        gy = C(2) * rho * dv;
+        jx = rmul(rho, u);
+        jy = rmul(rho, v);
+        gx = rmul(C(2) * rho, du);        // :1652-1656
+        gy = rmul(C(2) * rho, dv);
     }
-    // m = M g (solution.f90:580-600); rows 0, 3, 5 are the moments above
-    C m[9];
-    {
-        const C as = g[1] + g[2] + g[3] + g[4];
-        const C ds = g[5] + g[6] + g[7] + g[8];
-        const C dx = g[5] - g[6] - g[7] + g[8];
-        const C dy = g[5] + g[6] - g[7] - g[8];
-        m[0] = drho;
-        m[1] = C(-4) * g[0] - as + C(2) * ds;
-        m[2] = C(4) * g[0] - C(2) * as + ds;
-        m[3] = jx0;
-        m[4] = C(-2) * (g[1] - g[3]) + dx;
-        m[5] = jy0;
-        m[6] = C(-2) * (g[2] - g[4]) + dy;
-        m[7] = g[1] - g[2] + g[3] - g[4];
-        m[8] = g[5] - g[6] + g[7] - g[8];
-    }
-    const C jj = jx * jx + jy * jy;
-    C e[9];
-    e[0] = C(-1);                          // temp(1)=0 minus (M w)_1
-    e[1] = C(-2) * drho + C(3) * jj;       // solution.f90:605 minus (M w)_2
-    e[2] = drho - C(3) * jj;               // :606
-    e[3] = C(0);
-    e[4] = -jx;
-    e[5] = C(0);
-    e[6] = -jy;
-    e[7] = jx * jx - jy * jy;
-    e[8] = jx * jy;
-    // m' = m + s(meq - m) + fp (solution.f90:632-634); the new populations
-    // are taken as g + M^-1 (m' - m), which equals M^-1 m' exactly but
-    // rounds relative to the small non-equilibrium update, not to g
+    const C yy = rmul(jy, jy), jj = rfma(jx, jx, yy);
+    // (meq - m) s (solution.f90:603-612, 632-634; meq in deviation form); the
+    // new populations are taken as g + M^-1 (m' - m), which equals M^-1 m'
+    // exactly but rounds relative to the small non-equilibrium update, not to g
     C d[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) d[k] = (CONS0 && (k == 0 || k == 3 || k == 5)) ? C(0) : (e[k] - m[k]) * a.s[k];
+    d[0] = CONS0 ? C(0) : rmul(C(-1) - m[0], a.s[0]);
+    d[1] = rmul(rfma(C(3), jj, C(-2) * drho) - m[1], a.s[1]);   // :605
+    d[2] = rmul(rfma(C(-3), jj, drho) - m[2], a.s[2]);          // :606
+    d[3] = CONS0 ? C(0) : rmul(C(0) - m[3], a.s[3]);
+    d[4] = rmul(-jx - m[4], a.s[4]);
+    d[5] = CONS0 ? C(0) : rmul(C(0) - m[5], a.s[5]);
+    d[6] = rmul(-jy - m[6], a.s[6]);
+    d[7] = rmul(rfma(jx, jx, -yy) - m[7], a.s[7]);
+    d[8] = rmul(rfma(jx, jy, -m[8]), a.s[8]);
     if (gx != C(0) || gy != C(0)) {        // :614-626
-        const C ug = u * gx + v * gy;
-        d[1] += C(6) * (C(1) - C(0.5) * a.s[1]) * ug;
-        d[2] += C(-6) * (C(1) - C(0.5) * a.s[2]) * ug;
+        const C hs1 = C(1) - C(0.5) * a.s[1], hs2 = C(1) - C(0.5) * a.s[2], hs4 = C(1) - C(0.5) * a.s[4];
+        const C hs6 = C(1) - C(0.5) * a.s[6], hs7 = C(1) - C(0.5) * a.s[7], hs8 = C(1) - C(0.5) * a.s[8];
+        const C vgy = rmul(v, gy), ug = rfma(u, gx, vgy);
+        d[1] = rfma(rmul(C(6), hs1), ug, d[1]);
+        d[2] = rfma(rmul(C(-6), hs2), ug, d[2]);
         d[3] += gx;
-        d[4] += -(C(1) - C(0.5) * a.s[4]) * gx;
+        d[4] = rfma(-hs4, gx, d[4]);
         d[5] += gy;
-        d[6] += -(C(1) - C(0.5) * a.s[6]) * gy;
-        d[7] += C(2) * (C(1) - C(0.5) * a.s[7]) * (u * gx - v * gy);
-        d[8] += (C(1) - C(0.5) * a.s[8]) * (u * gy + v * gx);
+        d[6] = rfma(-hs6, gy, d[6]);
+        d[7] = rfma(C(2) * hs7, rfma(u, gx, -vgy), d[7]);
+        d[8] = rfma(hs8, rfma(u, gy, rmul(v, gx)), d[8]);
     }
-    mrt_inverse(d, gout);
+    // M^-1 d (mrt_inverse), the scale of d[3] and d[5] fused into their sums
+    const C k6 = C(1.0 / 6.0);
+    const C a1 = rmul(d[0], C(1.0 / 9.0)), a2 = rmul(d[1], C(1.0 / 36.0)), a3 = rmul(d[2], C(1.0 / 36.0));
+    const C a5 = rmul(d[4], C(1.0 / 12.0)), a7 = rmul(d[6], C(1.0 / 12.0)), a8 = C(0.25) * d[7], a9 = C(0.25) * d[8];
+    gout[0] = rfma(C(4), a3, rfma(C(-4), a2, a1));
+    const C ax = rfma(C(-2), a3, a1 - a2);
+    gout[1] = rfma(C(-2), a5, rfma(d[3], k6, ax)) + a8;
+    gout[3] = rfma(C(2), a5, rfma(-d[3], k6, ax)) + a8;
+    gout[2] = rfma(C(-2), a7, rfma(d[5], k6, ax)) - a8;
+    gout[4] = rfma(C(2), a7, rfma(-d[5], k6, ax)) - a8;
+    const C ad = rfma(C(2), a2, a1) + a3;
+    const C px = rfma(d[3], k6, a5), py = rfma(d[5], k6, a7);
+    gout[5] = ad + px + py + a9;
+    gout[6] = ad - px + py - a9;
+    gout[7] = ad - px - py + a9;
+    gout[8] = ad + px - py - a9;
 #pragma unroll
     for (int k = 0; k < 9; ++k) gout[k] += g[k];
     frho = rho; fu = u; fv = v;
+}
+
+template <typename C, bool CONS0 = false>
+__device__ __forceinline__ void collide_interior(const KFArgs<C> &a, const C g[9], bool corr, C du, C dv, C gout[9],
+                                                 C &frho, C &fu, C &fv)
+{
+    collide_moments<C, CONS0>(a, g, node_moments_of(g), corr, du, dv, gout, frho, fu, fv);
 }
 
 // Two interior nodes at once (no correction) with the paired FP32
@@ -280,7 +320,7 @@ __device__ __forceinline__ void collide_pair(const KFArgs<float> &a, const float
 }
 
 // edge node: boundary_condition1 (boundary_condition.f90:413-853)
-template <typename T, typename C>
+template <typename T, typename C, typename LD = LdNc>
 __device__ __forceinline__ void edge_update(const KFArgs<C> &a, const T *__restrict__ fin, int i, int j, C gout[9],
                                             C &frho, C &fu, C &fv)
 {
@@ -292,12 +332,12 @@ __device__ __forceinline__ void edge_update(const KFArgs<C> &a, const T *__restr
         if (i == 0 || i == a.nx - 1) {
             const int side = i == 0 ? 0 : 1;
             C d2[9], dr2, u2, v2;
-            side_bc<T, C>(a, fin, side, jn, drn, un, vn, d2, dr2, u2, v2);
+            side_bc<T, C, LD>(a, fin, side, jn, drn, un, vn, d2, dr2, u2, v2);
             const C *c = a.corner + 9 * (2 * side + (j == 0 ? 0 : 1));
 #pragma unroll
             for (int k = 0; k < 9; ++k) g0n[k] = c[k];   // edge f0, never rewritten
         } else {
-            pull<T, C>(fin, a.plane, a.pitch, i, jn, g0n);
+            pull<T, C, LD>(fin, a.plane, a.pitch, i, jn, g0n);
             moments(g0n, drn, un, vn);
         }
         extrapolate_dev<C>(a.s, drn, C(0), C(0), drn, un, vn, g0n, gout);
@@ -306,7 +346,7 @@ __device__ __forceinline__ void edge_update(const KFArgs<C> &a, const T *__restr
         // left/right column (boundary_condition.f90:413-483, 495-567)
         const int side = i == 0 ? 0 : 1;
         C dr1, u1, v1;
-        side_bc<T, C>(a, fin, side, j, dr1, u1, v1, g0n, drn, un, vn);
+        side_bc<T, C, LD>(a, fin, side, j, dr1, u1, v1, g0n, drn, un, vn);
         extrapolate_dev<C>(a.s, dr1, u1, v1, drn, un, vn, g0n, gout);
         frho = C(1) + dr1; fu = u1; fv = v1;
     }

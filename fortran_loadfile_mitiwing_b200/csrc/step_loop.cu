@@ -1,0 +1,661 @@
+// step_loop.cu -- several time steps of a small case in one launch.
+//
+// On a lattice whose populations stay in L2 a step is not bound by memory but
+// by the chain of its dependent stages: interpolation -> solve -> correction
+// tiles -> next step. As separate launches each link costs a kernel's start
+// and end and a cross-stream event besides its own arithmetic. Here one
+// cooperative launch runs up to a factorization batch of steps, and its CTAs
+// (one per SM) hand the stages to one another through L2:
+//
+//   CTA 0       the solver: stages the step's factor blocks in shared memory
+//               while the markers are interpolated, solves as soon as the
+//               right-hand sides are there, and publishes the solution
+//   other CTAs  interpolation (a warp per marker); then, while the solver
+//               works, every lattice node outside the correction tiles, and
+//               the correction tiles' markers and populations brought on
+//               chip; then, with the solution, the correction tiles; and a
+//               barrier among themselves before the next step
+//
+// Right-hand sides and solutions are their own flags: the factorization chain
+// leaves not_yet() in the step's slot and the reader polls the value it needs,
+// which saves a fence, a counter and a second round trip per hand-over (with a
+// counter each, a 96x64 step took 15.2 us). What the next stage needs besides
+// (a marker's weights, the markers of a tile) is loaded a step ahead, off the
+// chain, and what it does not need (the forces of a tile) is left for after.
+//
+// Measured on a B200, us a step, launches per stage -> here: 96x64 27.9 ->
+// 9.1; 400x200 33.5 -> 11.7 (FP64 31.7 -> 12.5); 1001x501 with two wings
+// 42 -> 18; 1280x640 42 -> 16.8; 2048x1024 in BF16 46 -> 30, where the
+// lattice's 18 us, L2 traffic by loads through registers, are most of it.
+// On large lattices the staged kernel is the better one (loop_fits).
+//
+// The force rows and residual checks of the steps follow as ordinary launches
+// (what they read is kept per step slot). Populations, right-hand sides and
+// solutions are read from L2 (LdCg): other CTAs wrote them in this launch.
+// Every wait is bounded; one that gives up sets LBM_ST_TIMEOUT and a flag
+// that ends the other CTAs' waits too.
+#include <algorithm>
+#include <type_traits>
+
+#include "ib_device.cuh"
+
+namespace {
+
+using namespace lbm_ib;
+using namespace lbm_node;
+
+constexpr int LOOP_STEPS = LBM_NSLOT_MAX / 2;   // steps of one launch at most (a slot half)
+// counters, each on a line of its own
+enum { SYNC_STEP = 0, SYNC_ABORT = 32, SYNC_WORDS = 64 };
+constexpr int LOOP_SMEM = 232448 - 1024;        // dynamic shared memory a CTA may use
+
+constexpr int NT = 512;                         // threads of a CTA (at 1024 the 64 registers left to each spill)
+
+template <typename C> struct LoopArgs {
+    IBArgs ib;               // slot 0
+    KFArgs<C> kf;            // fin, fout, tiles, pinfo and the field pointers are not used
+    void *f[2];              // population buffers: step s reads f[s & 1], writes the other
+    C *fields[LOOP_STEPS];   // rho, u, v of a step (nx*ny each), or null
+    int step0, nsteps;
+    unsigned *sync;          // SYNC_WORDS counters; base: what the step counter holds at the launch
+    unsigned base;
+};
+
+__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+{
+    unsigned v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void red_release(unsigned *p, unsigned v)
+{
+    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+constexpr int SPINS = 1 << 22;
+
+// a wait of this CTA gave up: report it and end the other CTAs' waits
+__device__ __forceinline__ void give_up(unsigned *sync, unsigned *status)
+{
+    atomicOr(status, LBM_ST_TIMEOUT);
+    red_release(sync + SYNC_ABORT, 1u);
+}
+
+// bounded wait for the step counter to reach target (one thread); false when
+// it gave up or another CTA did
+__device__ __forceinline__ bool wait_step(unsigned *sync, unsigned target, unsigned *status)
+{
+    for (int spins = 0; spins < SPINS; ++spins) {
+        if ((int)(ld_acquire(sync + SYNC_STEP) - target) >= 0) return true;
+        if ((spins & 63) == 63 && ld_acquire(sync + SYNC_ABORT)) return false;
+    }
+    give_up(sync, status);
+    return false;
+}
+
+// bounded wait for the two values p[0] and p[n] of a marker (right-hand side
+// or solution); false when it gave up or another CTA did
+__device__ __forceinline__ bool wait_pair(const double *p, int n, unsigned *sync, unsigned *status, double &x, double &y)
+{
+    for (int spins = 0; spins < SPINS; ++spins) {
+        long long a, b;
+        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(b) : "l"(p + n) : "memory");
+        if (a != (long long)LBM_NOT_YET && b != (long long)LBM_NOT_YET) {
+            x = __longlong_as_double(a);
+            y = __longlong_as_double(b);
+            return true;
+        }
+        if ((spins & 63) == 63 && ld_acquire(sync + SYNC_ABORT)) return false;
+    }
+    give_up(sync, status);
+    return false;
+}
+__device__ __forceinline__ void put_value(double *p, double x)
+{
+    const long long v = __double_as_longlong(is_value(x));
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// shared memory of a tile's threads
+struct GroupSmem {
+    TileSmem tile;
+    TileWeights weights;
+};
+
+__device__ __forceinline__ void group_sync(int grp)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(grp + 1), "r"(TILE_THREADS) : "memory");
+}
+
+template <typename C>
+__device__ __forceinline__ void put_fields(C *fl, long long nn, long long q, C rho, C u, C v)
+{
+    fl[q] = rho;
+    fl[nn + q] = u;
+    fl[2 * nn + q] = v;
+}
+
+template <typename T, typename C>
+__device__ __forceinline__ void put_node(const KFArgs<C> &a, T *fout, C *fl, int i, int j, const C gout[9], C rho, C u, C v)
+{
+    const long long o = (long long)j * a.pitch + i;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) Store<T>::st(fout + (long long)k * a.plane + o, gout[k]);
+    if (fl) put_fields(fl, (long long)a.nx * a.ny, (long long)j * a.nx + i, rho, u, v);
+}
+
+// node (i, j) lies in a correction tile of the step
+__device__ __forceinline__ bool in_tile(const IBArgs &a, const PatchInfo &r, int i, int j)
+{
+    const unsigned li = (unsigned)(i - r.i0), lj = (unsigned)(j - r.j0);
+    if (li >= (unsigned)r.w || lj >= (unsigned)r.h) return false;
+    const unsigned tx = li >> 4, t = (lj >> 4) * (unsigned)a.tiles_x + tx;
+    if (tx >= (unsigned)a.tiles_x || t >= (unsigned)patch_tiles(a)) {
+        atomicOr(a.status, LBM_ST_INDEX_LATTICE);
+        return false;
+    }
+    return a.tiles[(long long)t * (TILE_CAP + 1)] > 0;
+}
+
+// One warp's item of the interior: with FP32 arithmetic two nodes per lane
+// (rows j, j + 1 of a column, or with 2-byte storage columns i, i + 1 of a
+// row) by the paired update, as in the staged lattice kernel; one node per
+// lane in FP64.
+template <typename T> struct LatticeItem {
+    float2 g[9];
+    int i, j;
+    bool w0, w1;   // first, second node is written
+};
+template <> struct LatticeItem<double> {
+    double g[9];
+    int i, j;
+    bool w0, w1;
+};
+
+template <typename T, typename C>
+__device__ __forceinline__ void item_load(LatticeItem<T> &x, const KFArgs<C> &a, const IBArgs &ib, const PatchInfo &pr,
+                                          const T *fin, int item, int segs, int lane)
+{
+    const int r = item / segs, sg = item - r * segs;
+    const int pitch = a.pitch, plane = (int)a.plane;   // 9 planes < 2^31 elements (loop_fits)
+    if constexpr (sizeof(T) == 2) {
+        const int j = 1 + r, i = 2 * (32 * sg + lane);
+        x.i = i;
+        x.j = j;
+        x.w0 = i >= 1 && i <= a.nx - 2 && !in_tile(ib, pr, i, j);
+        x.w1 = i + 1 <= a.nx - 2 && !in_tile(ib, pr, i + 1, j);
+        if (!x.w0 && !x.w1) return;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const uint32_t *wk = reinterpret_cast<const uint32_t *>(fin + k * plane + (j - lbm_ey(k)) * pitch + i);
+            uint32_t w;
+            if (lbm_ex(k) == 0) w = __ldcg(wk);
+            else if (lbm_ex(k) == 1) w = __byte_perm(__ldcg(wk - 1), __ldcg(wk), 0x5432);   // columns i-1, i
+            else w = __byte_perm(__ldcg(wk), __ldcg(wk + 1), 0x5432);                       // columns i+1, i+2
+            x.g[k] = Pair2<T>::unpack(w);
+        }
+    } else if constexpr (sizeof(T) == 4) {
+        const int j = 1 + 2 * r, i = 32 * sg + lane;
+        const bool in = i >= 1 && i <= a.nx - 2, second = j + 1 <= a.ny - 2;
+        x.i = i;
+        x.j = j;
+        x.w0 = in && !in_tile(ib, pr, i, j);
+        x.w1 = in && second && !in_tile(ib, pr, i, j + 1);
+        if (!x.w0 && !x.w1) return;
+        const int up = second ? pitch : 0;   // an odd last row fills both halves
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const T *p = fin + k * plane + (j - lbm_ey(k)) * pitch + (i - lbm_ex(k));
+            x.g[k] = make_float2(__ldcg(p), __ldcg(p + up));
+        }
+    } else {
+        const int j = 1 + r, i = 32 * sg + lane;
+        x.i = i;
+        x.j = j;
+        x.w0 = i >= 1 && i <= a.nx - 2 && !in_tile(ib, pr, i, j);
+        x.w1 = false;
+        if (x.w0) pull<T, C, LdCg>(fin, a.plane, pitch, i, j, x.g);
+    }
+}
+
+template <typename T, typename C, bool CONS0>
+__device__ __forceinline__ void item_update(const LatticeItem<T> &x, const KFArgs<C> &a, T *fout, C *fl)
+{
+    if (!x.w0 && !x.w1) return;
+    if constexpr (sizeof(T) == 8) {
+        C o[9], rho, u, v;
+        collide_interior<C, CONS0>(a, x.g, false, C(0), C(0), o, rho, u, v);
+        put_node<T, C>(a, fout, fl, x.i, x.j, o, rho, u, v);
+    } else {
+        constexpr bool XPAIR = sizeof(T) == 2;
+        const int pitch = a.pitch, plane = (int)a.plane, d = XPAIR ? 1 : pitch;   // to the second node
+        float2 o[9], rho, u, v;
+        if (fl) collide_pair<CONS0, true>(a, x.g, o, rho, u, v);
+        else collide_pair<CONS0, false>(a, x.g, o, rho, u, v);
+        T *q = fout + x.j * pitch + x.i;
+        if (XPAIR && x.w0 && x.w1) {
+            if constexpr (XPAIR) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) *reinterpret_cast<uint32_t *>(q + k * plane) = Pair2<T>::pack(o[k]);
+            }
+        } else {
+            if (x.w0) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) q[k * plane] = Store<T>::pack(o[k].x);
+            }
+            if (x.w1) {
+#pragma unroll
+                for (int k = 0; k < 9; ++k) q[k * plane + d] = Store<T>::pack(o[k].y);
+            }
+        }
+        if (fl) {
+            const long long nn = (long long)a.nx * a.ny, n0 = (long long)x.j * a.nx + x.i;
+            if (x.w0) put_fields(fl, nn, n0, rho.x, u.x, v.x);
+            if (x.w1) put_fields(fl, nn, n0 + (XPAIR ? 1 : a.nx), rho.y, u.y, v.y);
+        }
+    }
+}
+
+// node e of the lattice's edge, 0 <= e < 2 nx + 2 (ny - 2)
+template <typename T, typename C>
+__device__ __forceinline__ void edge_node(const KFArgs<C> &a, const T *fin, T *fout, C *fl, int e)
+{
+    int i, j;
+    if (e < 2 * a.nx) {
+        i = e >> 1;
+        j = (e & 1) ? a.ny - 1 : 0;
+    } else {
+        j = 1 + ((e - 2 * a.nx) >> 1);
+        i = (e & 1) ? a.nx - 1 : 0;
+    }
+    C o[9], rho, u, v;
+    edge_update<T, C, LdCg>(a, fin, i, j, o, rho, u, v);
+    put_node<T, C>(a, fout, fl, i, j, o, rho, u, v);
+}
+
+// warps of the solver: one per even block of the first level (and a thread
+// per marker); more would only lengthen its barriers
+__device__ __forceinline__ int solver_warps(int nb) { return max(4, (nb + 1) / 2); }
+
+// The solver CTA's steps. Dynamic shared memory: the step's factor blocks
+// (block o at index o), the right-hand sides in the solve order, an mbarrier.
+template <typename C>
+__device__ __forceinline__ void solver_cta(const LoopArgs<C> &L, double *smem)
+{
+    const int n = L.ib.nseg, nb = (n + BS - 1) / BS, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int NW = min(solver_warps(nb), (int)blockDim.x / 32), NT = 32 * NW;
+    if (warp >= NW) return;   // barriers below count the threads that have not exited
+    double *stage = smem, *X = smem + nb * BS * GW;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(X + 2 * nb * BS);
+    // block o at index o; block 0 only its D_0^-1, whose rows (read in one
+    // step, like columns of the others) are kept apart by banks
+    constexpr uint32_t kBlock = sizeof(double) * BS * GW, kRow = sizeof(double) * BS;
+    constexpr int ROOT_LD = BS + 2;
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        mbar_init_fence();
+    }
+    __syncthreads();
+    uint32_t parity = 0;
+    // warp 0, once the CTA is done with the previous step's factor blocks:
+    // the copies of step s
+    auto issue = [&](int s) {
+        const IBArgs a = step_args(L.ib, L.step0 + s);
+        if (warp != 0 || a.fmode[0]) return;
+        if (lane == 0) mbar_expect_tx(bar, kBlock * (uint32_t)(nb - 1) + kRow * BS);
+        __syncwarp();
+        fence_proxy_async();
+        if (lane < BS) bulk_g2s(stage + lane * ROOT_LD, a.gf + lane * GW, kRow, bar);   // D_0^-1
+        for (int m = 1 + lane; m < nb; m += 32) bulk_g2s(stage + m * BS * GW, a.gf + (long long)m * BS * GW, kBlock, bar);
+    };
+    issue(0);
+    for (int s = 0; s < L.nsteps; ++s) {
+        const IBArgs a = step_args(L.ib, L.step0 + s);
+        const bool dense = a.fmode[0] != 0;
+        if (tid == 0) {
+            const unsigned fs = *a.fstatus;
+            if (fs) { atomicOr(a.status, fs); *a.fstatus = 0u; }
+            a.solve_res[1] = (double)a.fmode[1];
+        }
+        bool ok = true;
+        if (!dense) {   // the factor blocks
+            int spins = 0;
+            while (!mbar_try_wait(bar, parity))
+                if (++spins > SPINS) {
+                    ok = false;
+                    break;
+                }
+            if (!ok) give_up(L.sync, a.status);
+            parity ^= 1u;
+        }
+        // the right-hand sides in the solve order, each as soon as it is
+        // there (16-byte pairs; the dense solve keeps the two apart)
+        const int np = dense ? n : nb * BS;
+        for (int q = tid; q < np && ok; q += NT) {
+            const int k = q < n ? order_at(a, q, LBM_ST_INDEX_SOLVE) : -1;
+            double x = 0.0, y = 0.0;
+            if (k >= 0) ok = wait_pair(a.rhs + k, n, L.sync, a.status, x, y);
+            X[dense ? q : 2 * q] = x;
+            X[dense ? n + q : 2 * q + 1] = y;
+        }
+        if (__syncthreads_or(!ok)) return;
+        if (dense) {
+            dense_tri(a, X, NT);
+            __syncthreads();
+        } else {
+            // the levels with more than one even block
+            int st = 1;
+            for (; 2 * st < nb; st <<= 1) {
+                for (int e = 2 * st * warp; e < nb; e += 2 * st * NW)
+                    bcr_forward(stage + (e + st) * BS * GW, stage + (e - st) * BS * GW, X, e, st, e + st < nb, e > 0, lane);
+                __syncthreads();
+            }
+            // two blocks are left, 0 and st (or one): warp 0's alone
+            if (warp == 0) {
+                if (st < nb) bcr_forward(stage + st * BS * GW, stage, X, 0, st, true, false, lane);
+                __syncwarp();
+                bcr_root(stage, ROOT_LD, X, lane);
+                __syncwarp();
+                if (st < nb) bcr_backward(stage + st * BS * GW, X, st, st, false, lane);
+            }
+            __syncthreads();
+            for (st >>= 1; st > 0; st >>= 1) {
+                for (int o = st * (2 * warp + 1); o < nb; o += 2 * st * NW)
+                    bcr_backward(stage + o * BS * GW, X, o, st, o + st < nb, lane);
+                __syncthreads();
+            }
+        }
+        for (int q = tid; q < n; q += NT) {
+            const int k = order_at(a, q, LBM_ST_INDEX_SOLVE);
+            if (k < 0) continue;
+            put_value(a.y + k, X[dense ? q : 2 * q]);
+            put_value(a.y + n + k, X[dense ? n + q : 2 * q + 1]);
+        }
+        __syncthreads();
+        if (s + 1 < L.nsteps) issue(s + 1);
+    }
+}
+
+template <typename T, typename C, bool CONS0>
+__global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopArgs<C> L)
+{
+    constexpr int NW = NT / 32, NG = NT / TILE_THREADS;
+    extern __shared__ __align__(128) double smem[];
+    if (blockIdx.x == 0) {
+        solver_cta<C>(L, smem);
+        return;
+    }
+    __shared__ int good[NG];
+    const int cta = blockIdx.x - 1, G = gridDim.x - 1;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int grp = tid / TILE_THREADS, gt = tid % TILE_THREADS;
+    if (gt == 0) good[grp] = 1;
+    group_sync(grp);
+    const KFArgs<C> &kf = L.kf;
+    TileSmem &S = reinterpret_cast<GroupSmem *>(smem)[grp].tile;
+    TileWeights &W = reinterpret_cast<GroupSmem *>(smem)[grp].weights;
+    const int n = L.ib.nseg, nx = kf.nx, ny = kf.ny;
+    constexpr bool XPAIR = sizeof(T) == 2, YPAIR = sizeof(T) == 4;
+    const int segs = XPAIR ? (nx + 63) / 64 : (nx + 31) / 32;
+    const int items = segs * (YPAIR ? (ny - 1) / 2 : ny - 2);
+    const int nedge = 2 * nx + 2 * (ny - 2), nthr = G * NT;
+    // The CTA's two groups of TILE_THREADS threads work apart from each other.
+    // Correction tiles go to the CTAs from the last one on, in turn to the one
+    // or the other group from step to step: the group that has no tiles in a
+    // step prepares those of the next one as soon as its part of the step is
+    // done. Markers go to the CTAs from the first one on that have no tile
+    // (but to half of the CTAs at least); the first marker's weights are
+    // loaded a step ahead.
+    auto tiles_of = [&](const IBArgs &a) -> int {
+        const int c = *a.nsup;
+        if (c >= 0 && c <= patch_tiles(a)) return c;
+        if (tid == 0) atomicOr(a.status, LBM_ST_INDEX_TILE);
+        return 0;
+    };
+    auto marker_ctas = [&](int ntile) { return max(G - ntile, (G + 1) / 2); };
+    IBArgs a = step_args(L.ib, L.step0);
+    int ntile = tiles_of(a), mctas = marker_ctas(ntile);
+    int k0 = cta < mctas ? warp * mctas + cta : n;
+    InterpLane il;
+    if (k0 < n) il = interp_lane(a, k0, lane);
+    // the tile in hand: node, markers, populations, correction
+    int tile = -1, gi = 0, gj = 0, listed = 0, mark = -1, wing = 0, cnt = 0;
+    bool active = false;
+    C g[9];
+    NodeMoments<C> q;
+    double du = 0.0, dv = 0.0;
+    auto forces = [&](const IBArgs &a) {
+        const bool sup = active && wing < (1 << 20);
+        double fx = 0.0, fy = 0.0, mz = 0.0;
+        if (sup) node_force(a, motion_row(a, a.cur_step, nullptr), g, gi, gj, wing, du, dv, fx, fy, mz);
+        tile_force_warp(a, S, sup, wing, fx, fy, mz, gt >> 5, lane);
+        group_sync(grp);
+        tile_force_store(a, S, tile, gt);
+    };
+    // the markers of correction tile c, and the weights with which they act on
+    // the thread's node
+    auto prepare = [&](int c) {
+        const int nt = patch_tiles(a);
+        const PatchInfo pr = *a.pinfo;
+        tile = a.ctile[c];
+        if (tile < 0 || tile >= nt) {
+            if (gt == 0) atomicOr(a.status, LBM_ST_INDEX_TILE);
+            tile = -1;   // the same for the whole group
+            return;
+        }
+        const int ti0 = (tile % a.tiles_x) * TILE, tj0 = (tile / a.tiles_x) * TILE;
+        const int li = ti0 + (gt & 15), lj = tj0 + (gt >> 4);
+        gi = pr.i0 + li;
+        gj = pr.j0 + lj;
+        active = li < pr.w && lj < pr.h;
+        if (active && (gi < 1 || gi > nx - 2 || gj < 1 || gj > ny - 2)) {
+            atomicOr(a.status, LBM_ST_INDEX_TILE);
+            active = false;
+        }
+        const int *tl = a.tiles + (long long)tile * (TILE_CAP + 1);
+        listed = tl[0];
+        mark = -1;
+        if (listed <= TILE_CAP && gt < listed) {
+            mark = tl[1 + gt];
+            if (!tile_stage(a, S, gt, mark)) mark = -1;
+        }
+        group_sync(grp);
+        wing = 1 << 20;
+        cnt = listed <= TILE_CAP ? tile_cover(S, W, listed, active, gi, gj, gt, wing) : 0;
+    };
+    const int c0 = G - 1 - cta;   // the CTA's first tile
+    if (grp == 0 && c0 < ntile) prepare(c0);
+    for (int s = 0; s < L.nsteps; ++s) {
+        const T *fin = (const T *)L.f[s & 1];
+        T *fout = (T *)L.f[(s & 1) ^ 1];
+        C *fl = L.fields[s];
+        const bool duty = (s & 1) == grp;
+        for (int k = k0; k < n; k += NW * mctas) {
+            if (k > k0) il = interp_lane(a, k, lane);
+            double ru, rv;
+            interp_sum<T, LdCg>(a, fin, il, ru, rv);
+            if (lane == 0) {
+                put_value(a.rhs + k, ru);
+                put_value(a.rhs + n + k, rv);
+            }
+        }
+        // while the solver works: the nodes outside the correction tiles, edge
+        // nodes and interior, each dealt out from the group without tiles on
+        const PatchInfo pr = *a.pinfo;
+        const int et = duty ? TILE_THREADS + gt : gt;   // thread of the CTA, the free group first
+        for (int e = (TILE_THREADS - 1 - et + (duty ? NT : 0)) * G + cta; e < nedge; e += nthr) edge_node<T, C>(kf, fin, fout, fl, e);
+        for (int it = (et >> 5) * G + cta; it < items; it += NW * G) {
+            LatticeItem<T> x;
+            item_load<T, C>(x, kf, a, pr, fin, it, segs, lane);
+            item_update<T, C, CONS0>(x, kf, fout, fl);
+        }
+        // the update of the prepared tile; what its forces need is kept
+        auto update = [&]() {
+            du = dv = 0.0;
+            if (active) {
+                pull<T, C, LdCg>(fin, kf.plane, kf.pitch, gi, gj, g);
+                q = node_moments_of(g);
+            }
+            if (listed <= TILE_CAP) {
+                if (mark >= 0) {
+                    double x = 0.0, y = 0.0;
+                    if (!wait_pair(a.y + mark, n, L.sync, a.status, x, y)) good[grp] = 0;
+                    S.y[gt][0] = x;
+                    S.y[gt][1] = y;
+                }
+                group_sync(grp);
+                if (active) tile_sum(S, W, cnt, listed, gi, gj, gt, du, dv);
+            } else {
+                // more markers than a list holds: scan all of them, in order
+                const int ti0 = (tile % a.tiles_x) * TILE, tj0 = (tile / a.tiles_x) * TILE;
+                const int ta = pr.i0 + ti0, tb = ta + TILE - 1, sa = pr.j0 + tj0, sb = sa + TILE - 1;
+                const int gw = gt >> 5;
+                for (int m0 = 0; m0 < n; m0 += TILE_THREADS) {
+                    const int k = m0 + gt;
+                    bool hit = false;
+                    if (k < n) {
+                        if (marker_ok(a, a.mk[k])) {
+                            const int4 b = mbox(a.mk[k]);
+                            hit = b.x <= tb && b.y >= ta && b.z <= sb && b.w >= sa && b.y >= b.x;
+                        } else {
+                            atomicOr(a.status, LBM_ST_INDEX_TILE);
+                        }
+                    }
+                    const unsigned bal = __ballot_sync(0xffffffffu, hit);
+                    if (lane == 0) S.wsum[gw] = __popc(bal);
+                    group_sync(grp);
+                    int before = 0, all = 0;
+                    for (int w = 0; w < 8; ++w) {
+                        const int t = S.wsum[w];
+                        before += w < gw ? t : 0;
+                        all += t;
+                    }
+                    if (hit) {
+                        const int at = before + __popc(bal & ((1u << lane) - 1u));
+                        if (tile_stage(a, S, at, k)) {
+                            double x = 0.0, y = 0.0;
+                            if (!wait_pair(a.y + k, n, L.sync, a.status, x, y)) good[grp] = 0;
+                            S.y[at][0] = x;
+                            S.y[at][1] = y;
+                        }
+                    }
+                    group_sync(grp);
+                    if (active) tile_gather(S, 0, all, gi, gj, du, dv, wing);
+                    group_sync(grp);
+                }
+            }
+            if (active) {
+                C o[9], rho, u, v;
+                collide_moments<C>(kf, g, q, true, (C)du, (C)dv, o, rho, u, v);
+                put_node<T, C>(kf, fout, fl, gi, gj, o, rho, u, v);
+            }
+        };
+        if (duty)
+            for (int c = c0; c < ntile; c += G) {
+                if (c > c0) {
+                    if (tile >= 0) forces(a);
+                    group_sync(grp);
+                    prepare(c);
+                }
+                if (tile >= 0) update();
+            }
+        // the group's part of the step is handed on
+        group_sync(grp);
+        if (gt == 0) red_release(L.sync + SYNC_STEP, 1u);
+        if (!good[grp]) return;
+        if (duty && c0 < ntile && tile >= 0) forces(a);
+        if (s + 1 == L.nsteps) return;
+        // what the next step needs ahead of its start
+        a = step_args(L.ib, L.step0 + s + 1);
+        ntile = tiles_of(a);
+        mctas = marker_ctas(ntile);
+        k0 = cta < mctas ? warp * mctas + cta : n;
+        if (k0 < n) il = interp_lane(a, k0, lane);
+        if (!duty && c0 < ntile) prepare(c0);
+        if (gt == 0) good[grp] = wait_step(L.sync, L.base + (unsigned)(NG * G) * (unsigned)(s + 1), a.status);
+        group_sync(grp);
+        if (!good[grp]) return;
+    }
+}
+
+size_t loop_smem(const lbm_handle *h)
+{
+    const size_t nb = (size_t)(h->nseg + BS - 1) / BS;
+    const size_t solve = sizeof(double) * (nb * BS * GW + 2 * nb * BS) + 16;
+    return std::max(solve, NT / TILE_THREADS * sizeof(GroupSmem));
+}
+
+template <typename T, typename C, bool CONS0>
+int launch_loop_t(lbm_handle *h, const IBArgs &ib, int nsteps, void *const *fields, cudaStream_t st)
+{
+    LoopArgs<C> L;
+    L.ib = ib;
+    L.kf = make_kf_args<C>(h, nullptr, nullptr, nullptr, KF_OUTER);
+    L.f[0] = h->fbuf[h->cur];
+    L.f[1] = h->fbuf[h->cur ^ 1];
+    for (int s = 0; s < LOOP_STEPS; ++s) L.fields[s] = s < nsteps ? (C *)fields[s] : nullptr;
+    L.step0 = h->n;
+    L.nsteps = nsteps;
+    L.sync = h->d_sync;
+    const size_t smem = loop_smem(h);
+    auto kernel = step_loop<T, C, CONS0>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
+    // one group's threads for every 256 nodes (or pairs), so that the group
+    // without tiles does the lattice alone where the SMs suffice; fewer than
+    // 24 CTAs leave tiles to share one (96x64: 10.0 us a step on 6 CTAs, 9.1
+    // on 24 and on 132)
+    const int want = (h->nx * h->ny / (sizeof(T) == 8 ? 1 : 2) + TILE_THREADS - 1) / TILE_THREADS;
+    const int ctas = std::min(1 + std::max(want, 24), h->loop_ctas);
+    // every launch adds the same number to the step counter, whatever it
+    // waited for; after one that gave up the counters start over (loop_reset)
+    L.base = h->sync_base;
+    void *args[] = {&L};
+    if (cudaLaunchCooperativeKernel((const void *)kernel, dim3(ctas), dim3(NT), args, smem, st) != cudaSuccess) return -1;
+    h->sync_base += (unsigned)(NT / TILE_THREADS * (ctas - 1) * nsteps);
+    h->launches += 4ll * nsteps;   // interpolation, solve, lattice, correction tiles of each step
+    return 0;
+}
+
+}  // namespace
+
+int loop_sync_words() { return SYNC_WORDS; }
+
+cudaError_t loop_reset(lbm_handle *h)
+{
+    h->sync_base = 0;
+    return cudaMemsetAsync(h->d_sync, 0, SYNC_WORDS * sizeof(unsigned), h->stream);
+}
+
+// Whether a handle's steps run as step_loop launches.
+bool loop_fits(const lbm_handle *h)
+{
+    if (h->loop_ctas < 2 || h->nseg <= 0 || h->nslots / 2 > LOOP_STEPS) return false;
+    if (loop_smem(h) > LOOP_SMEM) return false;
+    // the loop's lattice update moves at most some 5 TB/s and 3 nodes a step
+    // and clock, the staged kernel more: 2400x1200 in FP32 (210 MB) 62 us a step
+    // here and 68 there, 2800x1400 (282 MB) 81 and 78; FP64 1600x800 (184 MB) 51
+    // and 61, 2048x1024 (302 MB) 87 and 79; 2800x1400 in FP16, bound by the
+    // nodes and not by their 141 MB, 58 and 59
+    return 18ll * std::max<long long>(4, (long long)h->elem) * h->plane <= 220000000ll;
+}
+
+// `nsteps` steps from step h->n on (within one slot half), step s with its
+// fields written to fields[s] unless null
+int launch_loop(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t st)
+{
+    IBArgs ib;
+    ib_args_write(h, nullptr, 0, &ib);
+    const bool c0 = h->s[0] == 0.0 && h->s[3] == 0.0 && h->s[5] == 0.0;
+    switch (h->prec) {
+    case LBM_PREC_FP32:
+        return c0 ? launch_loop_t<float, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<float, float, false>(h, ib, nsteps, fields, st);
+    case LBM_PREC_FP64:
+        return c0 ? launch_loop_t<double, double, true>(h, ib, nsteps, fields, st) : launch_loop_t<double, double, false>(h, ib, nsteps, fields, st);
+    case LBM_PREC_FP16:
+        return c0 ? launch_loop_t<__half, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<__half, float, false>(h, ib, nsteps, fields, st);
+    case LBM_PREC_BF16:
+        return c0 ? launch_loop_t<__nv_bfloat16, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<__nv_bfloat16, float, false>(h, ib, nsteps, fields, st);
+    }
+    return -1;
+}

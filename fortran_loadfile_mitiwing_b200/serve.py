@@ -42,7 +42,7 @@ _MAXW = 8                  # LBM_MAXW
 _NPART = 3 * _MAXW + 3     # per-tile partials of the correction
 _TILE_INTS = 257           # per-tile list: count + 256 markers
 _BS, _GW = 16, 48          # block size and factor row width of the marker solve
-_FBATCH = 4                # steps per factorization batch (LBM_IB_BATCH)
+_FBATCH = 8                # steps per factorization batch (LBM_IB_BATCH)
 _MASS_BLOCKS = 296         # CTAs of the mass check (kf_kernel.cu)
 
 
@@ -79,7 +79,7 @@ def patch_extent(case):
 def estimate_device_bytes(case):
     """Device bytes a case holds while it is stepped: lattice buffers, fields
     and edge values (lbm_create), step table and contour, and the
-    immersed-boundary scratch of 2 x 4 step slots (first step)."""
+    immersed-boundary scratch of 2 x 8 step slots (first step)."""
     p = case.params
     nx, ny = p.nx, p.ny
     elem = _elem_bytes(p.precision)
@@ -92,7 +92,7 @@ def estimate_device_bytes(case):
     total = 2 * elem * (9 * pitch * ny + 2 * _FPAD)          # populations, two buffers
     total += 2 * 3 * cs * nx * ny                              # fields, two slots
     total += cs * (6 * ny + 36)                                # edge values
-    total += 4 + 4 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 2 * 16 + 8 * row_len * _RING
+    total += 4 + 4 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 16 * _NSLOT_MAX + 4 * 64 + 8 * row_len * _RING
     total += 8 * (_MASS_BLOCKS + 1) + 4                        # mass check: partials and sum, counter
     if nwing:
         dt = p.scale * p.uu
@@ -103,10 +103,10 @@ def estimate_device_bytes(case):
         nb = (ns + _BS - 1) // _BS
         pw, ph = patch_extent(case)
         nblk = max(1, (pw + 15) // 16) * max(1, (ph + 15) // 16)
-        # right-hand sides, solution and tile partials: one set per step parity
-        total += S * _MARKER_BYTES * ns + 2 * 2 * 8 * 2 * ns + S * 8 * ns * ns
+        # right-hand sides, solution and tile partials: one set per slot
+        total += S * _MARKER_BYTES * ns + S * 2 * 8 * 2 * ns + S * 8 * ns * ns
         total += 2 * K * 8 * nb * _BS * _BS + S * 8 * nb * _BS * _GW + S * 2 * 4 + S * 4
-        total += 2 * 8 * max(_NPART * nblk, 2 * ((ns + 7) // 8))
+        total += S * 8 * max(_NPART * nblk, 2 * ((ns + 7) // 8))
         total += S * 4 * _TILE_INTS * nblk + S * 4 + S * 4 * nblk
         total += S * 4 * ns + S * 8 * ns + 8 + K * 4
     return int(total)

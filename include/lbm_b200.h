@@ -248,9 +248,13 @@ LBM_API int lbm_get_timing(lbm_t *h, double *step_ms, double *ib_ms, double *lat
 LBM_API int lbm_residual_device(const void *u, const void *v, const void *u0, const void *v0,
                                 int nx, int ny, int precision, void *stream, double *err);
 
-/* number of CUDA kernels this handle has launched since lbm_create (all
- * entry points: steps, population transfers, residuals). No counterpart in
- * the reference, which has no device code. */
+/* number of CUDA kernels run for this handle since lbm_create (all entry
+ * points: steps, population transfers, residuals). A launch that works for
+ * several cases counts for each of them, and one that runs several steps of a
+ * small lattice counts the kernels it runs in place of (per step:
+ * interpolation, solve, lattice, correction tiles, force row), so the count
+ * of a run does not depend on how its kernels were launched. No counterpart
+ * in the reference, which has no device code. */
 LBM_API int lbm_get_launch_count(const lbm_t *h, long long *count);
 
 /* current step counter n of the driver loop (1 before the first step). */
