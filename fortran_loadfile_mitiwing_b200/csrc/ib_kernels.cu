@@ -1133,11 +1133,20 @@ __global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *
     force_row(a, BATCH ? a.ring_row : ring_slot);
 }
 
-// the force rows of consecutive steps (CTA b: step step0 + b), headers included
-__global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, int step0, int ring0)
+// arguments of case z of a batch's loop launch (they begin its entry)
+__device__ __forceinline__ const IBArgs &loop_case(const void *batch, size_t stride)
 {
-    const int step = step0 + (int)blockIdx.x, rr = ring0 + (int)blockIdx.x;
-    const IBArgs a = step_args(a0, step);
+    return *reinterpret_cast<const IBArgs *>((const char *)batch + blockIdx.z * stride);
+}
+
+// the force rows of consecutive steps, headers included: CTA b the step b
+// after the arguments' (of slot 0), into the row b after theirs
+template <bool BATCH>
+__global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, const void *batch, size_t stride)
+{
+    const IBArgs &base = BATCH ? loop_case(batch, stride) : a0;
+    const int step = base.cur_step + (int)blockIdx.x, rr = base.ring_row + (int)blockIdx.x;
+    const IBArgs a = step_args(base, step);
     if (threadIdx.x == 0 && rr >= 0 && rr < a.ring_rows) {
         double time;
         const double *row = motion_row(a, step, &time);
@@ -1152,11 +1161,8 @@ __global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, int step
 // half-bandwidth; deterministic two-level sum (CTA partials, last CTA).
 // Flags LBM_ST_SOLVER unless it is below 1e-6, or LBM_ST_NONFINITE when the
 // right-hand side itself is not finite (the flow at the markers diverged).
-template <bool BATCH>
-__global__ void __launch_bounds__(256) ib_residual(const IBArgs a0, const IBArgs *batch)
+__device__ __forceinline__ void solve_residual(const IBArgs &a)
 {
-    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
-    if (BATCH && !a.check_res) return;   // this case's step is not checked
     __shared__ double red[8][2];
     __shared__ bool amlast;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1226,6 +1232,23 @@ __global__ void __launch_bounds__(256) ib_residual(const IBArgs a0, const IBArgs
             atomicOr(a.status, LBM_ST_SOLVER);
         *a.counter = 0u;
     }
+}
+
+template <bool BATCH>
+__global__ void __launch_bounds__(256) ib_residual(const IBArgs a0, const IBArgs *batch)
+{
+    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
+    if (BATCH && !a.check_res) return;   // this case's step is not checked
+    solve_residual(a);
+}
+
+// the step t after the loop launch's first; due for every case, or (if not)
+// for those whose last step it is
+__global__ void __launch_bounds__(256) ib_residual_steps(const void *batch, size_t stride, int t, bool due)
+{
+    const IBArgs &base = loop_case(batch, stride);
+    if (!due && !base.check_res) return;
+    solve_residual(step_args(base, base.cur_step + t));
 }
 
 // The correction tiles of the step (the 16 x 16 tiles of the patch
@@ -1523,8 +1546,10 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st)
 
 int launch_check_steps(lbm_handle *h, int step0, int count, int ring_slot, bool last, cudaStream_t st)
 {
-    const IBArgs a = make_args(h, nullptr, 0);
-    ib_forces_steps<<<count, 256, 0, st>>>(a, step0, ring_slot);
+    IBArgs a = make_args(h, nullptr, 0);
+    a.cur_step = step0;
+    a.ring_row = ring_slot;
+    ib_forces_steps<false><<<count, 256, 0, st>>>(a, nullptr, 0);
     h->launches += count;   // a force row each
     for (int t = 0; t < count; ++t) {
         if (!check_due(step0 + t) && !(last && t == count - 1)) continue;
@@ -1672,5 +1697,20 @@ int launch_check_batch(lbm_handle *const *hs, int ncase, const void *dargs, int 
     if (!residual) return cudaGetLastError() == cudaSuccess ? 0 : -1;   // no case checks this step
     ib_residual<true><<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(IBArgs{}, d);
     for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
+    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+int launch_check_steps_batch(lbm_handle *const *hs, int ncase, const void *dargs, size_t stride, int count, unsigned due,
+                             bool last, cudaStream_t st)
+{
+    const int ns = max_seg(hs, ncase);
+    ib_forces_steps<true><<<dim3(count, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs, stride);
+    for (int c = 0; c < ncase; ++c) hs[c]->launches += count;
+    for (int t = 0; t < count; ++t) {
+        const bool d = (due >> t) & 1u;
+        if (!d && !(last && t == count - 1)) continue;
+        ib_residual_steps<<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(dargs, stride, t, d);
+        for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
+    }
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

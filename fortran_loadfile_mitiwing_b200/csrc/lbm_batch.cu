@@ -12,6 +12,11 @@
 // slots and factorization state, kept in its handle), and may be added and
 // removed between runs: the base of the serving loop.
 //
+// A batch of small lattices at one phase of their factorization batches runs as
+// step_loop launches instead (loop_shares): each case gets CTAs of its own and
+// up to a factorization batch of steps is one launch, in the stream code and in
+// the graphs.
+//
 // Every kernel computes each case exactly as the single-case launches do, so
 // a case's results in a batch are bit-for-bit those of running it alone.
 //
@@ -45,6 +50,11 @@ constexpr int kArgRing = 8;
 // that segments of a run share their structure) and instantiated graphs kept
 constexpr int kGraphSteps = 16;
 constexpr int kGraphCache = 8;
+// argument buffers of step_loop launches in flight, entries of their CTA maps,
+// and such launches in a graph segment at most
+constexpr int kLoopRing = 4;
+constexpr int kLoopMap = 256;
+constexpr int kLoopChunks = 3;
 
 size_t round256(size_t x) { return (x + 255) & ~(size_t)255; }
 }
@@ -83,6 +93,11 @@ struct lbm_batch {
     void *d_fargs[kFactorRing] = {}, *h_fargs[kFactorRing] = {};
     cudaEvent_t ev_fup[kFactorRing] = {};
     int fring = 0;
+    // step_loop launches: the cases' arguments, then the CTA map; ev_lup: the
+    // upload is done, ev_luse: the launch and its checks
+    void *d_loop[kLoopRing] = {}, *h_loop[kLoopRing] = {};
+    cudaEvent_t ev_lup[kLoopRing] = {}, ev_luse[kLoopRing] = {};
+    int lring = 0;
     cudaEvent_t ev_group[kGroupRing] = {};
     long long gseq = 0;   // factorization launches so far
     size_t ib_sz = 0, kf_sz = 0;
@@ -157,6 +172,11 @@ void free_arrays(lbm_batch *b)
         if (b->h_fargs[r]) cudaFreeHost(b->h_fargs[r]);
         b->d_fargs[r] = b->h_fargs[r] = nullptr;
     }
+    for (int r = 0; r < kLoopRing; ++r) {
+        if (b->d_loop[r]) cudaFree(b->d_loop[r]);
+        if (b->h_loop[r]) cudaFreeHost(b->h_loop[r]);
+        b->d_loop[r] = b->h_loop[r] = nullptr;
+    }
     // the graphs name these buffers
     for (auto &g : b->gcache)
         if (g.exec) cudaGraphExecDestroy(g.exec);
@@ -193,6 +213,9 @@ void free_batch(lbm_batch *b)
         if (b->ev_fup[r]) cudaEventDestroy(b->ev_fup[r]);
     for (int r = 0; r < kGroupRing; ++r)
         if (b->ev_group[r]) cudaEventDestroy(b->ev_group[r]);
+    for (int r = 0; r < kLoopRing; ++r)
+        for (cudaEvent_t e : {b->ev_lup[r], b->ev_luse[r]})
+            if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : {b->ev_ib, b->ev_done, b->ev_fready, b->ev_side, b->ev_t0, b->ev_t1, b->ev_interp,
                           b->ev_gdone[0], b->ev_gdone[1], b->ev_gpre, b->ev_bcheck[0], b->ev_bcheck[1], b->ev_cpre})
         if (e) cudaEventDestroy(e);
@@ -203,6 +226,9 @@ void free_batch(lbm_batch *b)
     if (b->fstream) cudaStreamDestroy(b->fstream);
     if (b->cstream) cudaStreamDestroy(b->cstream);
 }
+
+// bytes of the arguments and the CTA map of one step_loop launch of nc cases
+size_t loop_launch_bytes(int prec, int nc) { return round256(nc * loop_args_size(prec)) + kLoopMap * sizeof(int4); }
 
 // argument arrays for `ncase` cases and `ntab` case-table entries (grown, never shrunk)
 int reserve(lbm_batch *b, int ncase, int ntab)
@@ -225,10 +251,16 @@ int reserve(lbm_batch *b, int ncase, int ntab)
         BCK(cudaMalloc(&b->d_fargs[r], nc * b->ib_sz), "alloc");
         BCK(cudaMallocHost(&b->h_fargs[r], nc * b->ib_sz), "alloc");
     }
+    for (int r = 0; r < kLoopRing; ++r) {
+        BCK(cudaMalloc(&b->d_loop[r], loop_launch_bytes(b->prec, nc)), "alloc");
+        BCK(cudaMallocHost(&b->h_loop[r], loop_launch_bytes(b->prec, nc)), "alloc");
+    }
     // a graph segment's arguments: per step the flow-chain and lattice
     // arguments of every case, and up to two factorization launches per step
     b->seg_bytes = round256((size_t)kGraphSteps * nc * b->ib_sz) + round256((size_t)kGraphSteps * nc * b->kf_sz) +
                    round256((size_t)2 * kGraphSteps * nc * b->ib_sz);
+    b->seg_bytes = std::max(b->seg_bytes, round256((size_t)2 * kLoopChunks * nc * b->ib_sz) +
+                                              kLoopChunks * loop_launch_bytes(b->prec, nc));
     for (int q = 0; q < 2; ++q) {
         BCK(cudaMalloc(&b->d_seg[q], b->seg_bytes), "alloc");
         BCK(cudaMallocHost(&b->h_seg[q], b->seg_bytes), "alloc");
@@ -344,6 +376,9 @@ int lbm_batch_create(lbm_t *const *cases, int count, lbm_batch_t **out)
     for (int r = 0; r < kGroupRing; ++r)
         if ((e = cudaEventCreateWithFlags(&b->ev_group[r], cudaEventDisableTiming)) != cudaSuccess)
             return fail(e, "event");
+    for (int r = 0; r < kLoopRing; ++r)
+        for (cudaEvent_t *ev : {&b->ev_lup[r], &b->ev_luse[r]})
+            if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
     for (int c = 0; c < count; ++c) {
         const int rc = add_case(b, cases[c]);
         if (rc) {
@@ -541,9 +576,94 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
     };
     std::vector<lbm_handle *> act, prev_act;
     std::vector<int> act_idx;
+    std::vector<int> share, all_share;   // step_loop CTAs of each active case (empty: launches per stage)
     int tcur = -1, ntab = 0;           // table buffer in use, its entries
+    std::vector<long long> waited;
     bool cons0 = true;                 // every case's conserved-moment relaxation rates are zero
     for (lbm_handle *h : b->cases) cons0 = cons0 && h->s[0] == 0.0 && h->s[3] == 0.0 && h->s[5] == 0.0;
+    // the active cases' step_loop arguments for m steps, and the CTA map, into
+    // dst; the cases' counters and steps go on
+    auto loop_write = [&](char *dst, int m, int ring_row, bool fields_end) {
+        const size_t lsz = loop_args_size(b->prec);
+        int4 *map = (int4 *)(dst + round256(act.size() * lsz));
+        // fields of the last two steps of the call and of every case that ends
+        // (all active cases keep them then)
+        bool keep[LBM_NSLOT_MAX] = {};
+        for (int t = 0; t < m && fields_end; ++t) {
+            keep[t] = step + t >= nsteps - 2;
+            for (size_t c = 0; c < act.size(); ++c) keep[t] = keep[t] || act[c]->n + t >= last_step[act_idx[c]] - 1;
+        }
+        int at = 0;
+        for (size_t c = 0; c < act.size(); ++c) {
+            lbm_handle *h = act[c];
+            void *fields[LBM_NSLOT_MAX] = {};
+            for (int t = 0; t < m; ++t)
+                if (keep[t]) {
+                    const int fs = h->fields_slot ^ 1;
+                    fields[t] = h->d_fields[fs];
+                    h->fields_slot = fs;
+                    h->fields_step[fs] = h->n + t;
+                }
+            const bool last = fields_end && (step + m == nsteps || h->n + m - 1 >= last_step[act_idx[c]]);
+            loop_args_write(h, m, fields, ring_row, last, dst + c * lsz);
+            loop_account(h, share[c], m);
+            for (int q = 0; q < share[c]; ++q) map[at++] = make_int4((int)c, q, share[c], 0);
+        }
+    };
+    auto loop_due = [&](int m) {
+        unsigned due = 0;
+        for (int t = 0; t < m; ++t)
+            if (check_due(act[0]->n + t)) due |= 1u << t;   // the cases are at one phase
+        return due;
+    };
+    auto advance = [&](int m) {
+        for (size_t c = 0; c < act.size(); ++c) {
+            lbm_handle *h = act[c];
+            if (m & 1) h->cur ^= 1;
+            h->n += m;
+            h->steps_done += m;
+            done[act_idx[c]] += m;
+        }
+    };
+    // m steps of the active cases as one step_loop launch from the host
+    auto loop_chunk = [&](int m) -> int {
+        int r0 = factor_needed(act, act_idx, false);
+        if (r0) return r0;
+        waited.clear();
+        for (lbm_handle *h : act) {
+            const long long g = h->fgroup[(h->n / K) & 1];
+            if (g > seq_start && std::find(waited.begin(), waited.end(), g) == waited.end()) {
+                BCK(cudaStreamWaitEvent(b->main, b->ev_group[g % kGroupRing], 0), "wait");
+                waited.push_back(g);
+            }
+        }
+        // the next batch's factorization, beside this launch
+        if ((r0 = factor_needed(act, act_idx, true))) return r0;
+        const int r = b->lring;
+        b->lring = (b->lring + 1) % kLoopRing;
+        BCK(cudaEventSynchronize(b->ev_lup[r]), "sync upload");
+        const unsigned due = loop_due(m);
+        char *hb = (char *)b->h_loop[r], *db = (char *)b->d_loop[r];
+        loop_write(hb, m, pending, true);
+        bool last = step + m == nsteps;
+        for (size_t c = 0; c < act.size(); ++c) last = last || act[c]->n + m - 1 >= last_step[act_idx[c]];
+        const size_t lsz = loop_args_size(b->prec), off = round256(act.size() * lsz);
+        BCK(cudaStreamWaitEvent(b->main, b->ev_luse[r], 0), "wait");
+        BCK(cudaMemcpyAsync(db, hb, off + kLoopMap * sizeof(int4), cudaMemcpyHostToDevice, b->main), "upload");
+        BCK(cudaEventRecord(b->ev_lup[r], b->main), "event");
+        if (launch_loop_multi(act.data(), (int)act.size(), share, m, cons0, db, (const int4 *)(db + off), b->main))
+            return berr(b, LBM_ERR_CUDA, std::string("batch: launch step loop: ") + cudaGetErrorString(cudaGetLastError()));
+        BCK(cudaEventRecord(b->ev_done, b->main), "event");
+        BCK(cudaStreamWaitEvent(b->cstream, b->ev_done, 0), "wait");
+        if (launch_check_steps_batch(act.data(), (int)act.size(), db, lsz, m, due, last, b->cstream))
+            return berr(b, LBM_ERR_CUDA, "batch: launch check");
+        BCK(cudaEventRecord(b->ev_luse[r], b->cstream), "event");
+        BCK(cudaEventRecord(b->ev_bcheck[0], b->cstream), "event");
+        BCK(cudaEventRecord(b->ev_bcheck[1], b->cstream), "event");
+        BCK(cudaEventRecord(b->ev_side, b->cstream), "event");
+        advance(m);
+        return LBM_OK;
+    };
     // One CUDA graph segment of kGraphSteps steps from `step` (the caller has
     // checked that it may run one: the same active cases and case table as
     // the step before, no fields, room in the force ring). The host plans the
@@ -560,6 +680,8 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         int cur = -1, next = -1;    // factorization groups before / after the flow chain
         std::vector<int> waits;     // groups of this segment the flow chain waits for
         bool residual = false;      // some case checks its solve residual
+        int m = 0;                  // steps of a step_loop launch, and those of them to check
+        unsigned due = 0;
     };
     auto graph_segment = [&]() -> int {
         const int G = kGraphSteps, na = (int)act.size();
@@ -567,10 +689,12 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         b->gset ^= 1;
         BCK(cudaEventSynchronize(b->ev_gdone[sb]), "sync segment");   // the last graph that read this buffer
         char *hs = (char *)b->h_seg[sb], *ds = (char *)b->d_seg[sb];
+        const bool loop = !share.empty();
+        const size_t lone = loop_launch_bytes(b->prec, na);
         const size_t off_k = round256((size_t)G * na * b->ib_sz);
-        const size_t off_f = off_k + round256((size_t)G * na * b->kf_sz);
+        const size_t off_f = loop ? kLoopChunks * lone : off_k + round256((size_t)G * na * b->kf_sz);
         std::vector<GroupPlan> groups;
-        std::vector<StepPlan> plan(G);
+        std::vector<StepPlan> plan(G), chunks;
         const long long seq_seg = b->gseq;   // groups numbered above it are the segment's own
         // a factorization group, chosen as factor_needed chooses it
         auto plan_factor = [&](bool next) -> int {
@@ -596,7 +720,23 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             groups.push_back(std::move(g));
             return (int)groups.size() - 1;
         };
-        for (int t = 0; t < G; ++t) {
+        for (int t = 0; t < G && loop;) {
+            StepPlan p;
+            p.m = std::min(K - act[0]->n % K, G - t);
+            p.cur = plan_factor(false);
+            for (int c = 0; c < na; ++c) {
+                const long long g = act[c]->fgroup[(act[c]->n / K) & 1];
+                const int gi = (int)(g - seq_seg - 1);
+                if (g > seq_seg && std::find(p.waits.begin(), p.waits.end(), gi) == p.waits.end()) p.waits.push_back(gi);
+            }
+            p.next = plan_factor(true);
+            p.due = loop_due(p.m);
+            loop_write(hs + chunks.size() * lone, p.m, pending + t, false);
+            advance(p.m);
+            t += p.m;
+            chunks.push_back(std::move(p));
+        }
+        for (int t = 0; t < G && !loop; ++t) {
             StepPlan &p = plan[t];
             p.cur = plan_factor(false);
             // groups from before the segment are complete when the graph starts
@@ -631,11 +771,12 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         // the structure: what sets grid sizes, kernel variants, buffer
         // addresses and the graph's edges
         std::vector<long long> sig = {sb, G, na, b->prec, cons0, b->after_interp, tcur, ntab, K, (long long)used,
-                                      b->ctas_per_sm};
+                                      b->ctas_per_sm, (long long)loop};
         for (lbm_handle *h : act)
             sig.insert(sig.end(), {(long long)(uintptr_t)h, h->nseg, h->patch_gx(), h->patch_gy(), h->static_order});
-        for (const StepPlan &p : plan) {
-            sig.insert(sig.end(), {p.cur, p.next, (long long)p.residual, (long long)p.waits.size()});
+        sig.insert(sig.end(), share.begin(), share.end());
+        for (const StepPlan &p : loop ? chunks : plan) {
+            sig.insert(sig.end(), {p.cur, p.next, (long long)p.residual, (long long)p.m, (long long)p.due, (long long)p.waits.size()});
             sig.insert(sig.end(), p.waits.begin(), p.waits.end());
         }
         for (const GroupPlan &g : groups) {
@@ -665,7 +806,22 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 return LBM_OK;
             };
             int erc = LBM_OK;
-            for (int t = 0; t < G; ++t) {
+            for (size_t q = 0; q < chunks.size(); ++q) {   // step_loop launches
+                const StepPlan &p = chunks[q];
+                if (p.cur >= 0 && (erc = factor(p.cur, q > 0))) return erc;
+                if (p.next >= 0 && (erc = factor(p.next, q > 0))) return erc;
+                for (int gi : p.waits) BCK(cudaStreamWaitEvent(b->main, E[9 + gi], 0), "wait");
+                const char *la = ds + q * lone;
+                const size_t lsz = loop_args_size(b->prec);
+                if (launch_loop_multi(act.data(), na, share, p.m, cons0, la, (const int4 *)(la + round256(na * lsz)), b->main))
+                    return berr(b, LBM_ERR_CUDA, "batch: launch step loop");
+                BCK(cudaEventRecord(E[7], b->main), "event");
+                BCK(cudaStreamWaitEvent(b->cstream, E[7], 0), "wait");
+                if (launch_check_steps_batch(act.data(), na, la, lsz, p.m, p.due, false, b->cstream))
+                    return berr(b, LBM_ERR_CUDA, "batch: launch check");
+                BCK(cudaEventRecord(E[6], b->cstream), "event");
+            }
+            for (int t = 0; t < G && !loop; ++t) {
                 const StepPlan &p = plan[t];
                 if (p.cur >= 0 && (erc = factor(p.cur, t > 0))) return erc;
                 if (t > 0) BCK(cudaStreamWaitEvent(b->side, E[7], 0), "wait");
@@ -754,7 +910,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         BCK(cudaEventRecord(b->ev_gdone[sb], b->side), "event");
         BCK(cudaEventRecord(b->ev_done, b->side), "event");
         BCK(cudaEventRecord(b->ev_side, b->side), "event");
-        BCK(cudaEventRecord(b->ev_tuse[tcur], b->side), "event");
+        if (tcur >= 0) BCK(cudaEventRecord(b->ev_tuse[tcur], b->side), "event");
         BCK(cudaEventRecord(b->ev_bcheck[0], b->side), "event");
         BCK(cudaEventRecord(b->ev_bcheck[1], b->side), "event");
         for (const GroupPlan &g : groups) BCK(cudaEventRecord(b->ev_group[g.seq % kGroupRing], b->side), "event");
@@ -768,7 +924,6 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
     BCK(cudaEventRecord(b->ev_t0, b->main), "event");
     b->last_ms = 0.0;
     b->last_steps = 0;
-    std::vector<long long> waited;
     std::vector<int> tkey, tkey_now;   // grids of the active cases the current table was built for
     const int ring_cap = b->cases[0]->ring_cap;
     for (; step < nsteps; ++step) {
@@ -781,11 +936,16 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 act_idx.push_back(c);
             }
         if (act.empty()) break;
+        // small lattices at one phase: step_loop launches
+        if (act != prev_act) all_share = loop_shares(act.data(), (int)act.size());
+        share = all_share;
+        for (lbm_handle *h : act)
+            if (h->n % K != act[0]->n % K) share.clear();
         // a graph segment where the next kGraphSteps steps allow one. Segments
         // start at every half of a factorization batch (of the first case),
         // so that runs of any length need two structures, not one for each
         // phase of the batch
-        if (b->graphs && act[0]->n % std::max(1, K / 2) == 0 && tcur >= 0 && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
+        if (b->graphs && act[0]->n % std::max(1, K / 2) == 0 && (tcur >= 0 || !share.empty()) && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
             pending + kGraphSteps <= ring_cap) {
             bool ok = true;
             for (size_t c = 0; c < act.size() && ok; ++c) ok = act[c]->n + kGraphSteps < last_step[act_idx[c]];
@@ -796,6 +956,17 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 if (pending == ring_cap && (rc = flush())) break;
                 continue;
             }
+        }
+        if (!share.empty()) {
+            int m = std::min({K - act[0]->n % K, nsteps - step, ring_cap - pending});
+            for (size_t c = 0; c < act.size(); ++c) m = std::min(m, last_step[act_idx[c]] - act[c]->n + 1);
+            // up to where a graph segment may start
+            if (b->graphs && K > 1 && act[0]->n % (K / 2)) m = std::min(m, K / 2 - act[0]->n % (K / 2));
+            if ((rc = loop_chunk(m))) break;
+            step += m - 1;
+            pending += m;
+            if (pending == ring_cap && (rc = flush())) break;
+            continue;
         }
         const int buf = step % kArgRing;
         // fields (rho, u, v) for the last two steps of the call and of every

@@ -241,6 +241,10 @@ int launch_check(lbm_handle *h, int slot, int ring_slot, bool residual, cudaStre
 // step0 on, after their step_loop launch; a step is checked as check_due says,
 // and the last one if `last`
 int launch_check_steps(lbm_handle *h, int step0, int count, int ring_slot, bool last, cudaStream_t st);
+// the same for a batch: dargs: the cases' loop arguments (stride bytes apart);
+// due: steps of the launch to check (bit t), by the cases' check_res its last
+int launch_check_steps_batch(lbm_handle *const *hs, int ncase, const void *dargs, size_t stride, int count, unsigned due,
+                             bool last, cudaStream_t st);
 // the solve residual is checked on every kCheckEvery-th step
 constexpr int kCheckEvery = 4;
 inline bool check_due(int step) { return (step + 1) % kCheckEvery == 0; }
@@ -249,6 +253,12 @@ bool loop_fits(const lbm_handle *h);
 int loop_sync_words();
 cudaError_t loop_reset(lbm_handle *h);   // after a launch that gave up
 int launch_loop(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t st);
+size_t loop_args_size(int prec);
+void loop_args_write(lbm_handle *h, int nsteps, void *const *fields, int ring_slot, bool check_last, void *dst);
+std::vector<int> loop_shares(lbm_handle *const *hs, int n);
+int launch_loop_multi(lbm_handle *const *hs, int n, const std::vector<int> &share, int nsteps, bool cons0,
+                      const void *dcases, const int4 *dmap, cudaStream_t st);
+void loop_account(lbm_handle *h, int ctas, int nsteps);   // of one case, for each launch
 // batches of cases stepped together (lbm_batch.cu)
 int handle_prepare_ib(lbm_handle *h);                    // immersed-boundary buffers (once per geometry)
 int handle_error(lbm_handle *h, int code, const char *msg);

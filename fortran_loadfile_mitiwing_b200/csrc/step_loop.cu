@@ -377,17 +377,34 @@ __device__ __forceinline__ void solver_cta(const LoopArgs<C> &L, double *smem)
     }
 }
 
-template <typename T, typename C, bool CONS0>
-__global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopArgs<C> L)
+// One case (MULTI false: its arguments are L0, its CTAs the grid), or a batch
+// of cases (CTA b: entry b of `map`, {case, its CTA, its CTAs}), which share
+// the launch and nothing else.
+template <typename T, typename C, bool CONS0, bool MULTI>
+__global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopArgs<C> L0, const LoopArgs<C> *cases,
+                                                   const int4 *map)
 {
     constexpr int NW = NT / 32, NG = NT / TILE_THREADS;
     extern __shared__ __align__(128) double smem[];
-    if (blockIdx.x == 0) {
+    // a batch's arguments are read in shared memory: in global memory every
+    // store might alias them
+    __shared__ __align__(16) uint32_t lw[MULTI ? sizeof(LoopArgs<C>) / 4 : 1];
+    int me = blockIdx.x, all = gridDim.x;
+    if (MULTI) {
+        const int4 m = map[blockIdx.x];
+        me = m.y;
+        all = m.z;
+        const uint32_t *src = reinterpret_cast<const uint32_t *>(cases + m.x);
+        for (int w = threadIdx.x; w < (int)(sizeof(LoopArgs<C>) / 4); w += NT) lw[w] = src[w];
+        __syncthreads();
+    }
+    const LoopArgs<C> &L = MULTI ? *reinterpret_cast<const LoopArgs<C> *>(lw) : L0;
+    if (me == 0) {
         solver_cta<C>(L, smem);
         return;
     }
     __shared__ int good[NG];
-    const int cta = blockIdx.x - 1, G = gridDim.x - 1;
+    const int cta = me - 1, G = all - 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid / TILE_THREADS, gt = tid % TILE_THREADS;
     if (gt == 0) good[grp] = 1;
@@ -586,36 +603,73 @@ size_t loop_smem(const lbm_handle *h)
     return std::max(solve, NT / TILE_THREADS * sizeof(GroupSmem));
 }
 
-template <typename T, typename C, bool CONS0>
-int launch_loop_t(lbm_handle *h, const IBArgs &ib, int nsteps, void *const *fields, cudaStream_t st)
+// CTAs beside the solver that a case's lattice can use: one group's threads
+// for every 256 nodes (or pairs), so that the group without tiles does the
+// lattice alone where the SMs suffice; fewer than 24 CTAs leave tiles to
+// share one (96x64: 10.0 us a step on 6 CTAs, 9.1 on 24 and on 132)
+int loop_want(const lbm_handle *h)
+{
+    const int units = h->nx * h->ny / (h->elem == 8 ? 1 : 2);
+    return std::max((units + TILE_THREADS - 1) / TILE_THREADS, 24);
+}
+
+template <typename C>
+LoopArgs<C> loop_args(lbm_handle *h, int nsteps, void *const *fields, int ring_slot, bool check_last)
 {
     LoopArgs<C> L;
-    L.ib = ib;
+    ib_args_write(h, nullptr, 0, &L.ib);
+    L.ib.ring_row = ring_slot;
+    L.ib.check_res = check_last;
     L.kf = make_kf_args<C>(h, nullptr, nullptr, nullptr, KF_OUTER);
     L.f[0] = h->fbuf[h->cur];
     L.f[1] = h->fbuf[h->cur ^ 1];
-    for (int s = 0; s < LOOP_STEPS; ++s) L.fields[s] = s < nsteps ? (C *)fields[s] : nullptr;
+    for (int s = 0; s < LOOP_STEPS; ++s) L.fields[s] = fields && s < nsteps ? (C *)fields[s] : nullptr;
     L.step0 = h->n;
     L.nsteps = nsteps;
     L.sync = h->d_sync;
-    const size_t smem = loop_smem(h);
-    auto kernel = step_loop<T, C, CONS0>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
-    // one group's threads for every 256 nodes (or pairs), so that the group
-    // without tiles does the lattice alone where the SMs suffice; fewer than
-    // 24 CTAs leave tiles to share one (96x64: 10.0 us a step on 6 CTAs, 9.1
-    // on 24 and on 132)
-    const int want = (h->nx * h->ny / (sizeof(T) == 8 ? 1 : 2) + TILE_THREADS - 1) / TILE_THREADS;
-    const int ctas = std::min(1 + std::max(want, 24), h->loop_ctas);
     // every launch adds the same number to the step counter, whatever it
     // waited for; after one that gave up the counters start over (loop_reset)
     L.base = h->sync_base;
-    void *args[] = {&L};
-    if (cudaLaunchCooperativeKernel((const void *)kernel, dim3(ctas), dim3(NT), args, smem, st) != cudaSuccess) return -1;
+    return L;
+}
+
+// the launch of `ctas` CTAs for a case is accounted for
+void loop_done(lbm_handle *h, int ctas, int nsteps)
+{
     h->sync_base += (unsigned)(NT / TILE_THREADS * (ctas - 1) * nsteps);
     h->launches += 4ll * nsteps;   // interpolation, solve, lattice, correction tiles of each step
+}
+
+template <typename T, typename C, bool CONS0>
+int launch_loop_t(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t st)
+{
+    LoopArgs<C> L = loop_args<C>(h, nsteps, fields, 0, false);
+    const size_t smem = loop_smem(h);
+    auto kernel = step_loop<T, C, CONS0, false>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
+    const int ctas = std::min(1 + loop_want(h), h->loop_ctas);
+    const LoopArgs<C> *cases = nullptr;
+    const int4 *map = nullptr;
+    void *args[] = {&L, &cases, &map};
+    if (cudaLaunchCooperativeKernel((const void *)kernel, dim3(ctas), dim3(NT), args, smem, st) != cudaSuccess) return -1;
+    loop_done(h, ctas, nsteps);
     return 0;
 }
+
+template <typename T, typename C, bool CONS0>
+int launch_loop_multi_t(int ctas, size_t smem, const void *dcases, const int4 *dmap, cudaStream_t st)
+{
+    auto kernel = step_loop<T, C, CONS0, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
+    LoopArgs<C> none{};
+    const LoopArgs<C> *cases = (const LoopArgs<C> *)dcases;
+    void *args[] = {&none, &cases, &dmap};
+    return cudaLaunchCooperativeKernel((const void *)kernel, dim3(ctas), dim3(NT), args, smem, st) == cudaSuccess ? 0 : -1;
+}
+
+// bytes by which the lattices of a loop are measured: 2-byte storage counts as
+// 4-byte (its update is bound by the nodes)
+long long loop_bytes(const lbm_handle *h) { return 18ll * std::max<long long>(4, (long long)h->elem) * h->plane; }
 
 }  // namespace
 
@@ -630,32 +684,96 @@ cudaError_t loop_reset(lbm_handle *h)
 // Whether a handle's steps run as step_loop launches.
 bool loop_fits(const lbm_handle *h)
 {
-    if (h->loop_ctas < 2 || h->nseg <= 0 || h->nslots / 2 > LOOP_STEPS) return false;
-    if (loop_smem(h) > LOOP_SMEM) return false;
+    if (h->loop_ctas < 2 || h->nseg <= 0 || h->nslots / 2 > LOOP_STEPS || loop_smem(h) > LOOP_SMEM) return false;
     // the loop's lattice update moves at most some 5 TB/s and 3 nodes a step
     // and clock, the staged kernel more: 2400x1200 in FP32 (210 MB) 62 us a step
     // here and 68 there, 2800x1400 (282 MB) 81 and 78; FP64 1600x800 (184 MB) 51
     // and 61, 2048x1024 (302 MB) 87 and 79; 2800x1400 in FP16, bound by the
     // nodes and not by their 141 MB, 58 and 59
-    return 18ll * std::max<long long>(4, (long long)h->elem) * h->plane <= 220000000ll;
+    return loop_bytes(h) <= 220000000ll;
 }
 
 // `nsteps` steps from step h->n on (within one slot half), step s with its
 // fields written to fields[s] unless null
 int launch_loop(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t st)
 {
-    IBArgs ib;
-    ib_args_write(h, nullptr, 0, &ib);
     const bool c0 = h->s[0] == 0.0 && h->s[3] == 0.0 && h->s[5] == 0.0;
     switch (h->prec) {
     case LBM_PREC_FP32:
-        return c0 ? launch_loop_t<float, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<float, float, false>(h, ib, nsteps, fields, st);
+        return c0 ? launch_loop_t<float, float, true>(h, nsteps, fields, st) : launch_loop_t<float, float, false>(h, nsteps, fields, st);
     case LBM_PREC_FP64:
-        return c0 ? launch_loop_t<double, double, true>(h, ib, nsteps, fields, st) : launch_loop_t<double, double, false>(h, ib, nsteps, fields, st);
+        return c0 ? launch_loop_t<double, double, true>(h, nsteps, fields, st) : launch_loop_t<double, double, false>(h, nsteps, fields, st);
     case LBM_PREC_FP16:
-        return c0 ? launch_loop_t<__half, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<__half, float, false>(h, ib, nsteps, fields, st);
+        return c0 ? launch_loop_t<__half, float, true>(h, nsteps, fields, st) : launch_loop_t<__half, float, false>(h, nsteps, fields, st);
     case LBM_PREC_BF16:
-        return c0 ? launch_loop_t<__nv_bfloat16, float, true>(h, ib, nsteps, fields, st) : launch_loop_t<__nv_bfloat16, float, false>(h, ib, nsteps, fields, st);
+        return c0 ? launch_loop_t<__nv_bfloat16, float, true>(h, nsteps, fields, st) : launch_loop_t<__nv_bfloat16, float, false>(h, nsteps, fields, st);
     }
     return -1;
 }
+
+// ---- a batch of cases --------------------------------------------------------
+
+size_t loop_args_size(int prec) { return prec == LBM_PREC_FP64 ? sizeof(LoopArgs<double>) : sizeof(LoopArgs<float>); }
+
+void loop_args_write(lbm_handle *h, int nsteps, void *const *fields, int ring_slot, bool check_last, void *dst)
+{
+    if (h->prec == LBM_PREC_FP64)
+        *(LoopArgs<double> *)dst = loop_args<double>(h, nsteps, fields, ring_slot, check_last);
+    else
+        *(LoopArgs<float> *)dst = loop_args<float>(h, nsteps, fields, ring_slot, check_last);
+}
+
+// The CTAs of each case when `hs` run as one step_loop launch (empty: they
+// do not): one solver and at least one more, the rest by lattice size. The
+// launches per stage cost a batch some 45 us a step whatever its size.
+std::vector<int> loop_shares(lbm_handle *const *hs, int n)
+{
+    std::vector<int> share;
+    if (n < 1) return share;
+    const int total = hs[0]->loop_ctas;
+    long long bytes = 0;
+    double units = 0.0;
+    for (int c = 0; c < n; ++c) {
+        if (!loop_fits(hs[c])) return share;
+        bytes += loop_bytes(hs[c]);
+        units += (double)loop_want(hs[c]);
+    }
+    if (2 * n > total || bytes > 150000000ll) return share;
+    share.assign(n, 0);
+    int used = 0;
+    for (int c = 0; c < n; ++c) {
+        const int want = loop_want(hs[c]);
+        share[c] = 1 + std::max(1, std::min(want, (int)((total - 2 * n) * (want / units)) + 1));
+        used += share[c];
+    }
+    return used <= total ? share : std::vector<int>();
+}
+
+int launch_loop_multi(lbm_handle *const *hs, int n, const std::vector<int> &share, int nsteps, bool cons0,
+                      const void *dcases, const int4 *dmap, cudaStream_t st)
+{
+    size_t smem = 0;
+    int ctas = 0;
+    for (int c = 0; c < n; ++c) {
+        smem = std::max(smem, loop_smem(hs[c]));
+        ctas += share[c];
+    }
+    int rc = -1;
+    switch (hs[0]->prec) {
+    case LBM_PREC_FP32:
+        rc = cons0 ? launch_loop_multi_t<float, float, true>(ctas, smem, dcases, dmap, st) : launch_loop_multi_t<float, float, false>(ctas, smem, dcases, dmap, st);
+        break;
+    case LBM_PREC_FP64:
+        rc = cons0 ? launch_loop_multi_t<double, double, true>(ctas, smem, dcases, dmap, st) : launch_loop_multi_t<double, double, false>(ctas, smem, dcases, dmap, st);
+        break;
+    case LBM_PREC_FP16:
+        rc = cons0 ? launch_loop_multi_t<__half, float, true>(ctas, smem, dcases, dmap, st) : launch_loop_multi_t<__half, float, false>(ctas, smem, dcases, dmap, st);
+        break;
+    case LBM_PREC_BF16:
+        rc = cons0 ? launch_loop_multi_t<__nv_bfloat16, float, true>(ctas, smem, dcases, dmap, st) : launch_loop_multi_t<__nv_bfloat16, float, false>(ctas, smem, dcases, dmap, st);
+        break;
+    }
+    return rc;
+}
+
+void loop_account(lbm_handle *h, int ctas, int nsteps) { loop_done(h, ctas, nsteps); }

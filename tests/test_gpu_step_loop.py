@@ -80,3 +80,40 @@ def test_dense_solve(gpu_lib):
     with Batch([member]) as b:
         rows_b = b.run(11)[0]
     same(alone, member, alone.run(11), rows_b)
+
+
+@pytest.mark.parametrize("graphs", [True, False], ids=["graphs", "stream"])
+@pytest.mark.parametrize("precision", ["fp32", "fp64", "fp16"])
+def test_batch_of_small_cases(gpu_lib, precision, graphs):
+    """Cases of different sizes at one phase share step_loop launches, from the
+    host and inside graph segments; each gives what it gives alone, over runs
+    that begin at every phase of a factorization batch, and with a case that
+    ends inside a run."""
+    shapes = SHAPES[:5] + [SHAPES[6]]
+    steps = (3, 40, 21, 1, 30)
+    ends = [200, 200, 60, 200, 200, 200]
+    alone = [make(s, precision, gpu_lib, n) for s, n in zip(shapes, ends)]
+    member = [make(s, precision, gpu_lib, n) for s, n in zip(shapes, ends)]
+    with Batch(member) as b:
+        b.set_graphs(graphs)
+        for k in steps:
+            rows = b.run(k)
+            for a, r in zip(alone, rows):
+                np.testing.assert_array_equal(a.run(k), r)
+        assert b.graph_stats()[0] > 0 or not graphs
+    for a, m, n in zip(alone, member, ends):
+        same(a, m, np.zeros(0), np.zeros(0), fields=n == 200)
+
+
+def test_batch_of_many_tiny_cases(gpu_lib):
+    """As many cases as one launch takes (two CTAs each), and more."""
+    for count in (66, 70):
+        kw = [dict(seed=c, heave=0.1 + 0.002 * c) for c in range(count)]
+        alone = [Lbm.from_case(cases.small_case(n_steps=60, **k), gpu_lib) for k in kw]
+        member = [Lbm.from_case(cases.small_case(n_steps=60, **k), gpu_lib) for k in kw]
+        with Batch(member) as b:
+            rows = b.run(27)
+        for a, m, r in zip(alone, member, rows):
+            same(a, m, a.run(27), r)
+        for h in alone + member:
+            h.close()
