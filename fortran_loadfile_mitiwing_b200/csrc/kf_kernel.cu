@@ -655,7 +655,7 @@ constexpr int MASS_BLOCKS = 296, MASS_THREADS = 256;
 template <typename T>
 __global__ void __launch_bounds__(MASS_THREADS) mass_kernel(const T *__restrict__ f, int nx, int ny, int pitch,
                                                             long long plane, double *__restrict__ part,
-                                                            unsigned *__restrict__ counter)
+                                                            unsigned *__restrict__ counter, double *__restrict__ total)
 {
     __shared__ double red[MASS_THREADS / 32];
     __shared__ bool amlast;
@@ -685,29 +685,29 @@ __global__ void __launch_bounds__(MASS_THREADS) mass_kernel(const T *__restrict_
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int b = 0; b < (int)gridDim.x; ++b) t += __ldcg(part + b);
-        part[MASS_BLOCKS] = t;
+        *total = t;
         *counter = 0u;
     }
 }
 
 }  // namespace
 
-// the deviation sum of the populations in `fsrc` into h->d_mass[MASS_BLOCKS],
+// the deviation sum of the populations in `fsrc` into the handle's head,
 // on stream st (the caller copies it back)
 int launch_mass(lbm_handle *h, const void *fsrc, cudaStream_t st)
 {
     switch (h->prec) {
     case LBM_PREC_FP32:
-        mass_kernel<float><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const float *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount);
+        mass_kernel<float><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const float *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount, &h->d_head->mass);
         break;
     case LBM_PREC_FP64:
-        mass_kernel<double><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const double *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount);
+        mass_kernel<double><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const double *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount, &h->d_head->mass);
         break;
     case LBM_PREC_FP16:
-        mass_kernel<__half><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const __half *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount);
+        mass_kernel<__half><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const __half *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount, &h->d_head->mass);
         break;
     case LBM_PREC_BF16:
-        mass_kernel<__nv_bfloat16><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const __nv_bfloat16 *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount);
+        mass_kernel<__nv_bfloat16><<<MASS_BLOCKS, MASS_THREADS, 0, st>>>((const __nv_bfloat16 *)fsrc, h->nx, h->ny, h->pitch, h->plane, h->d_mass, h->d_mcount, &h->d_head->mass);
         break;
     default: return -1;
     }
@@ -715,7 +715,7 @@ int launch_mass(lbm_handle *h, const void *fsrc, cudaStream_t st)
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-int mass_slots() { return MASS_BLOCKS + 1; }
+int mass_slots() { return MASS_BLOCKS; }
 
 // Dynamic shared memory of a batched lattice launch that holds at most
 // `ctas_per_sm` CTAs on an SM (0: the kernel's own ring, as many CTAs as the

@@ -550,22 +550,21 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
     int rc = LBM_OK, pending = 0, step = 0;
     // copies the force rows of the steps since the last flush (ring rows
     // 0 .. rows-1, each case its own count) and reads the cases' status
-    auto flush = [&]() -> int {
+    auto flush = [&](bool mass) -> int {
         BCK(cudaStreamWaitEvent(b->main, b->ev_side, 0), "wait");
-        for (int c = 0; c < nc; ++c) {
-            lbm_handle *h = b->cases[c];
-            const int rows = done[c] - start[c];
-            if (force_rows && force_rows[c] && rows > 0)
-                BCK(cudaMemcpyAsync(force_rows[c] + (size_t)start[c] * h->row_len, h->d_ring,
-                                    sizeof(double) * h->row_len * rows, cudaMemcpyDeviceToHost, b->main),
-                    "copy force rows");
-        }
+        auto rows_to = [&](int c) {
+            return force_rows && force_rows[c] && done[c] > start[c] ? force_rows[c] + (size_t)start[c] * b->cases[c]->row_len
+                                                                     : nullptr;
+        };
+        for (int c = 0; c < nc; ++c)
+            if (handle_fetch(b->cases[c], b->main, mass && done[c] > 0, done[c] - start[c], rows_to(c)))
+                return berr(b, LBM_ERR_CUDA, std::string("batch: ") + b->cases[c]->err);
         BCK(cudaStreamSynchronize(b->main), "sync");
         pending = 0;
         int st0 = LBM_OK;
         for (int c = 0; c < nc; ++c) {
+            const int st = handle_fetched(b->cases[c], mass && done[c] > 0, done[c] - start[c], rows_to(c));
             start[c] = done[c];
-            const int st = handle_status(b->cases[c]);
             if (st) b->status[c] = st;
             if (st && !st0) {
                 st0 = st;
@@ -953,7 +952,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 if ((rc = graph_segment())) break;
                 step += kGraphSteps - 1;
                 pending += kGraphSteps;
-                if (pending == ring_cap && (rc = flush())) break;
+                if (pending == ring_cap && (rc = flush(false))) break;
                 continue;
             }
         }
@@ -965,7 +964,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             if ((rc = loop_chunk(m))) break;
             step += m - 1;
             pending += m;
-            if (pending == ring_cap && (rc = flush())) break;
+            if (pending == ring_cap && (rc = flush(false))) break;
             continue;
         }
         const int buf = step % kArgRing;
@@ -1089,7 +1088,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         pending++;
         // force rows to the host every ring's worth of steps
         if (pending == ring_cap) {
-            if ((rc = flush())) break;
+            if ((rc = flush(false))) break;
         }
     }
     // device time of the steps: from before the first step's launches to the
@@ -1098,30 +1097,10 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         BCK(cudaStreamWaitEvent(b->main, b->ev_side, 0), "wait");
         BCK(cudaEventRecord(b->ev_t1, b->main), "event");
     }
-    // the rows of the last steps (also when every case ended before nsteps)
-    if (pending > 0 && rc == LBM_OK) rc = flush();
-    // the global mass of every case that ran, at the end of the run (FP64 on
-    // the device; a non-finite mass fails that case)
-    if (rc == LBM_OK) {
-        std::vector<double> dsum(nc, 0.0);
-        for (int c = 0; c < nc && rc == LBM_OK; ++c)
-            if (done[c] > 0) rc = handle_mass_launch(b->cases[c], b->main, &dsum[c]);
-        if (rc == LBM_OK) {
-            BCK(cudaStreamSynchronize(b->main), "sync mass");
-            for (int c = 0; c < nc; ++c) {
-                const int st = done[c] > 0 ? handle_mass_result(b->cases[c], dsum[c]) : LBM_OK;
-                if (st) {
-                    b->status[c] = st;
-                    if (rc == LBM_OK) {
-                        rc = st;
-                        b->err = std::string("batch: case ") + std::to_string(c) + ": " + b->cases[c]->err;
-                    }
-                }
-            }
-        } else {
-            b->err = std::string("batch: mass check: ") + b->cases[0]->err;
-        }
-    }
+    // the rows of the last steps (also when every case ended before nsteps),
+    // and the global mass of every case that ran, at the end of the run (FP64
+    // on the device; a non-finite mass fails that case)
+    if (rc == LBM_OK) rc = flush(true);
     // leave every stream idle: the cases' own calls follow on their streams
     sync_streams(b);
     if (step > 0 && rc == LBM_OK) {

@@ -389,27 +389,48 @@ int status_error(unsigned st, std::string &msg)
 
 namespace {
 
-int check_status(lbm_handle *h)
+// Pinned host memory of a handle: what a call reads back goes there in one copy
+// (a copy into pageable memory holds up the host for some 10 us; a step call
+// made two). Blocks of destroyed handles are kept for the next ones, up to
+// kHostBlocks of them.
+constexpr size_t kHostBlock = 16384;
+constexpr size_t kHostBlocks = 64;
+std::mutex g_host_mu;
+std::vector<void *> g_host_free;
+
+void *host_block()
 {
-    unsigned st = 0;
-    CK(cudaMemcpyAsync(&st, h->d_status, sizeof st, cudaMemcpyDeviceToHost, h->stream), "read status");
-    CK(cudaStreamSynchronize(h->stream), "step sync");
-    if (!st) return LBM_OK;
-    CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream), "clear status");
-    if (st & LBM_ST_TIMEOUT) CK(loop_reset(h), "reset step loop");
-    std::string msg;
-    const int code = status_error(st, msg);
-    return set_err(h, code, msg.c_str());
+    {
+        std::lock_guard<std::mutex> lock(g_host_mu);
+        if (!g_host_free.empty()) {
+            void *p = g_host_free.back();
+            g_host_free.pop_back();
+            return p;
+        }
+    }
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, kHostBlock, cudaHostAllocPortable) == cudaSuccess) return p;
+    cudaGetLastError();
+    return nullptr;
 }
 
-// Global mass check: queues the FP64 deviation sum of the current populations
-// on stream st and its copy into *dsum (the caller synchronises st), then
-// mass_result turns it into the mass and checks that it is finite.
-int mass_launch(lbm_handle *h, cudaStream_t st, double *dsum)
+void host_block_free(void *p)
 {
-    if (launch_mass(h, h->fbuf[h->cur], st)) return cuda_err(h, cudaGetLastError(), "launch mass");
-    CK(cudaMemcpyAsync(dsum, h->d_mass + (mass_slots() - 1), sizeof(double), cudaMemcpyDeviceToHost, st), "copy mass");
-    return LBM_OK;
+    if (!p) return;
+    {
+        std::lock_guard<std::mutex> lock(g_host_mu);
+        if (g_host_free.size() < kHostBlocks) {
+            g_host_free.push_back(p);
+            return;
+        }
+    }
+    cudaFreeHost(p);
+}
+
+// rows that fit into the handle's block with the head
+bool rows_fit(const lbm_handle *h, int rows)
+{
+    return sizeof(RunHead) + sizeof(double) * h->row_len * (size_t)rows <= kHostBlock;
 }
 
 int mass_result(lbm_handle *h, double dsum)
@@ -419,6 +440,31 @@ int mass_result(lbm_handle *h, double dsum)
     h->last_mass_step = h->steps_done;
     if (!std::isfinite(m)) return set_err(h, LBM_ERR_NONFINITE, "mass check: non-finite populations (the flow diverged)");
     return LBM_OK;
+}
+
+int fetch(lbm_handle *h, cudaStream_t st, bool mass, int rows, double *dst)
+{
+    // the global mass check: the FP64 deviation sum of the current populations
+    if (mass && launch_mass(h, h->fbuf[h->cur], st)) return cuda_err(h, cudaGetLastError(), "launch mass");
+    const bool fit = dst && rows_fit(h, rows);
+    const size_t bytes = sizeof(double) * h->row_len * (size_t)rows;
+    CK(cudaMemcpyAsync(h->hblock, h->d_head, sizeof(RunHead) + (fit ? bytes : 0), cudaMemcpyDeviceToHost, st), "read status");
+    if (dst && !fit) CK(cudaMemcpyAsync(dst, h->d_ring, bytes, cudaMemcpyDeviceToHost, st), "copy force rows");
+    return LBM_OK;
+}
+
+int fetched(lbm_handle *h, bool mass, int rows, double *dst)
+{
+    const RunHead *head = (const RunHead *)h->hblock;
+    if (dst && rows_fit(h, rows)) memcpy(dst, head + 1, sizeof(double) * h->row_len * (size_t)rows);
+    if (const unsigned st = head->status) {
+        CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream), "clear status");
+        if (st & LBM_ST_TIMEOUT) CK(loop_reset(h), "reset step loop");
+        std::string msg;
+        const int code = status_error(st, msg);
+        return set_err(h, code, msg.c_str());
+    }
+    return mass ? mass_result(h, head->mass) : LBM_OK;
 }
 
 // sums the event intervals of `count` step slots after the streams are idle:
@@ -511,17 +557,12 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         // the span ends with the chunk's last step; the row copy and the
         // mass check after it are per-call work, not per-step work
         if (h->timing == LBM_TIMING_SPAN) CK(cudaEventRecord(h->ev[4 * (pending - 1) + 3], h->stream), "event");
-        if (rows_out)
-            CK(cudaMemcpyAsync(rows_out + (size_t)(done - pending) * h->row_len, h->d_ring,
-                               sizeof(double) * h->row_len * pending, cudaMemcpyDeviceToHost, h->stream),
-               "copy force rows");
-        double dsum = 0.0;
         const bool mass = mass_due();
-        int st = mass ? mass_launch(h, h->stream, &dsum) : LBM_OK;
+        double *dst = rows_out ? rows_out + (size_t)(done - pending) * h->row_len : nullptr;
+        int st = fetch(h, h->stream, mass, pending, dst);
         if (st) return st;
-        st = check_status(h);
-        if (st) return st;
-        if (mass && (st = mass_result(h, dsum))) return st;
+        CK(cudaStreamSynchronize(h->stream), "step sync");
+        if ((st = fetched(h, mass, pending, dst))) return st;
         if (h->timing && (st = collect_timing(h, pending, split))) return st;
         pending = 0;
         return LBM_OK;
@@ -660,10 +701,9 @@ __global__ void arch_probe() {}
 
 // for lbm_batch.cu
 int handle_prepare_ib(lbm_handle *h) { return ensure_ib(h); }
-int handle_mass_launch(lbm_handle *h, cudaStream_t st, double *dsum) { return mass_launch(h, st, dsum); }
-int handle_mass_result(lbm_handle *h, double dsum) { return mass_result(h, dsum); }
+int handle_fetch(lbm_handle *h, cudaStream_t st, bool mass, int rows, double *dst) { return fetch(h, st, mass, rows, dst); }
+int handle_fetched(lbm_handle *h, bool mass, int rows, double *dst) { return fetched(h, mass, rows, dst); }
 int handle_error(lbm_handle *h, int code, const char *msg) { return set_err(h, code, msg); }
-int handle_status(lbm_handle *h) { return check_status(h); }
 
 // boundary reference values from the edge f0 (FP64, full f; left column,
 // right column, bottom row, top row, 9 per node): the moments
@@ -883,7 +923,6 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     for (int b = 0; b < 2; ++b)
         if ((e = dmalloc(h, &h->d_fields[b], 3 * cs * nn)) != cudaSuccess) return fail(e, "alloc fields");
     if ((e = dmalloc(h, &h->edge_c, cs * (6 * (size_t)h->ny + 36))) != cudaSuccess) return fail(e, "alloc edge");
-    if ((e = dmalloc(h, &h->d_status, sizeof(unsigned))) != cudaSuccess) return fail(e, "alloc status");
     if ((e = dmalloc(h, &h->d_counter, sizeof(unsigned))) != cudaSuccess) return fail(e, "alloc counter");
     if ((e = dmalloc(h, &h->d_pinfo, LBM_NSLOT_MAX * sizeof(PatchInfo))) != cudaSuccess) return fail(e, "alloc pinfo");
     if ((e = dmalloc(h, &h->d_red, sizeof(double) * 2 * 296)) != cudaSuccess) return fail(e, "alloc red");
@@ -893,8 +932,11 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     // solve residual and half-bandwidth, per slot
     if ((e = dmalloc(h, &h->d_solve_res, LBM_NSLOT_MAX * 2 * sizeof(double))) != cudaSuccess) return fail(e, "alloc res");
     if ((e = dmalloc(h, &h->d_sync, sizeof(unsigned) * loop_sync_words())) != cudaSuccess) return fail(e, "alloc sync");
-    if ((e = dmalloc(h, &h->d_ring, sizeof(double) * h->row_len * (size_t)h->ring_cap)) != cudaSuccess)
+    if ((e = dmalloc(h, &h->d_head, sizeof(RunHead) + sizeof(double) * h->row_len * (size_t)h->ring_cap)) != cudaSuccess)
         return fail(e, "alloc ring");
+    h->d_status = &h->d_head->status;
+    h->d_ring = (double *)(h->d_head + 1);
+    if (!(h->hblock = host_block())) return fail(cudaErrorMemoryAllocation, "alloc host block");
     if (h->npts > 0) {
         if ((e = dmalloc(h, &h->d_xb0, sizeof(double) * h->npts)) != cudaSuccess) return fail(e, "alloc xb0");
         if ((e = dmalloc(h, &h->d_yb0, sizeof(double) * h->npts)) != cudaSuccess) return fail(e, "alloc yb0");
@@ -920,7 +962,9 @@ int lbm_destroy(lbm_t *h)
     free_devp(h->d_xb0); free_devp(h->d_yb0); free_devp(h->d_arc); free_devp(h->d_mstep);
     free_ib(h);
     free_devp(h->d_pinfo); free_devp(h->d_counter);
-    free_devp(h->d_ring); free_devp(h->d_status); free_devp(h->d_solve_res); free_devp(h->d_red);
+    free_devp(h->d_head); free_devp(h->d_solve_res);
+    host_block_free(h->hblock);
+    free_devp(h->d_red);
     free_devp(h->d_mass); free_devp(h->d_mcount); free_devp(h->d_sync);
 
     free_devp(h->d_stage);
@@ -1157,11 +1201,10 @@ int lbm_mass(lbm_t *h, double *mass)
 {
     if (!h || !mass) return LBM_ERR_ARG;
     if (!h->inited) return set_err(h, LBM_ERR_STATE, "mass: not initialised");
-    double dsum = 0.0;
-    int rc = mass_launch(h, h->stream, &dsum);
-    if (rc) return rc;
+    if (launch_mass(h, h->fbuf[h->cur], h->stream)) return cuda_err(h, cudaGetLastError(), "launch mass");
+    CK(cudaMemcpyAsync(h->hblock, h->d_head, sizeof(RunHead), cudaMemcpyDeviceToHost, h->stream), "copy mass");
     CK(cudaStreamSynchronize(h->stream), "sync mass");
-    rc = mass_result(h, dsum);
+    const int rc = mass_result(h, ((const RunHead *)h->hblock)->mass);
     *mass = h->last_mass;
     return rc;
 }

@@ -99,6 +99,15 @@ struct IBArgs {
     double *solve_res;  // relative residual of the last solve
 };
 
+// What the host reads at the end of a call, at the front of the force ring on
+// the device and copied in one piece to pinned memory (host_block): the status
+// word, the deviation sum of the mass check, then force rows.
+struct RunHead {
+    unsigned status;
+    unsigned pad;
+    double mass;
+};
+
 struct lbm_handle {
     lbm_params p;
     int nx = 0, ny = 0, pitch = 0;
@@ -192,10 +201,12 @@ struct lbm_handle {
     unsigned sync_base = 0;   // their step counter after the launches so far
     double *d_partial = nullptr;
     unsigned *d_counter = nullptr;
-    double *d_ring = nullptr;
+    RunHead *d_head = nullptr;   // allocation of the head and the force ring
+    double *d_ring = nullptr;    // behind it
+    void *hblock = nullptr;      // kHostBlock bytes of pinned memory
     int ring_cap = 0;
     int row_len = 0;
-    unsigned *d_status = nullptr;
+    unsigned *d_status = nullptr;   // d_head->status
     double *d_solve_res = nullptr;
     // fields of the last field-writing steps (compute precision), two slots
     void *d_fields[2] = {nullptr, nullptr};
@@ -262,11 +273,11 @@ void loop_account(lbm_handle *h, int ctas, int nsteps);   // of one case, for ea
 // batches of cases stepped together (lbm_batch.cu)
 int handle_prepare_ib(lbm_handle *h);                    // immersed-boundary buffers (once per geometry)
 int handle_error(lbm_handle *h, int code, const char *msg);
-int handle_status(lbm_handle *h);                        // reads and clears the device status
-// global mass check of a case: queue the sum on st into *dsum, then (after st
-// is synchronised) check it
-int handle_mass_launch(lbm_handle *h, cudaStream_t st, double *dsum);
-int handle_mass_result(lbm_handle *h, double dsum);
+// The end of a run of steps: queue on st the mass check (if mass), and the
+// copies of the head and of `rows` force rows into dst (nullable); then, after
+// st is synchronised, the rows' last move and the status or mass error, if any
+int handle_fetch(lbm_handle *h, cudaStream_t st, bool mass, int rows, double *dst);
+int handle_fetched(lbm_handle *h, bool mass, int rows, double *dst);
 // boundary reference values from the edge f0 populations (layout of edge_f0)
 int handle_set_edges(lbm_handle *h, const double *edge_f0);
 // state of a restart file in the reference's layout: populations f(nx,ny,9),
@@ -299,7 +310,7 @@ int launch_init_lattice(lbm_handle *h, const double *du, const double *dv);
 int launch_fields_to_double(lbm_handle *h, const void *fields, double *rho, double *u, double *v);
 // global mass check (FP64, deterministic) of the populations in fsrc
 int launch_mass(lbm_handle *h, const void *fsrc, cudaStream_t st);
-int mass_slots();
+int mass_slots();   // doubles of the mass check's CTA partials
 // error code and message of a device status word
 int status_error(unsigned st, std::string &msg);
 // host <-> device copies of host arrays through the pinned staging ring

@@ -92,8 +92,8 @@ def estimate_device_bytes(case):
     total = 2 * elem * (9 * pitch * ny + 2 * _FPAD)          # populations, two buffers
     total += 2 * 3 * cs * nx * ny                              # fields, two slots
     total += cs * (6 * ny + 36)                                # edge values
-    total += 4 + 4 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 16 * _NSLOT_MAX + 4 * 64 + 8 * row_len * _RING
-    total += 8 * (_MASS_BLOCKS + 1) + 4                        # mass check: partials and sum, counter
+    total += 16 + 4 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 16 * _NSLOT_MAX + 4 * 64 + 8 * row_len * _RING
+    total += 8 * _MASS_BLOCKS + 4                        # mass check: partials and sum, counter
     if nwing:
         dt = p.scale * p.uu
         msteps = int((case.table[-1, 0] + 1e-12) / dt) + 1
