@@ -298,6 +298,7 @@ int check_case(lbm_batch *b, lbm_handle *h)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+        if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return handle_error(h, LBM_ERR_CUDA, "batch: sync");
     return LBM_OK;
 }
@@ -497,6 +498,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         if (h->fstream) cudaStreamSynchronize(h->fstream);
         if (h->side) cudaStreamSynchronize(h->side);
         if (h->cstream) cudaStreamSynchronize(h->cstream);
+        if (h->nstream) cudaStreamSynchronize(h->nstream);
         cudaStreamSynchronize(h->stream);
         int gx, gy;
         kf_tma_grid(h, &gx, &gy);

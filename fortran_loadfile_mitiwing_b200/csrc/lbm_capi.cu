@@ -182,6 +182,7 @@ void quiesce(lbm_handle *h)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (h->stream) cudaStreamSynchronize(h->stream);
 }
 
@@ -232,12 +233,24 @@ void free_ib(lbm_handle *h)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->ib_ready = 0;
     h->batch_in_half[0] = h->batch_in_half[1] = -1;
     free_devp(h->d_mk); free_devp(h->d_rhs); free_devp(h->d_B); free_devp(h->d_y); free_devp(h->d_partial);
     free_devp(h->d_bD); free_devp(h->d_bL); free_devp(h->d_gf); free_devp(h->d_fmode); free_devp(h->d_fstatus); free_devp(h->d_tiles); free_devp(h->d_nsup); free_devp(h->d_ctile);
+    free_dev(h->fmid_alloc); h->fmid = nullptr; h->pairs = 0;
+    free_devp(h->d_near); free_devp(h->d_near_list); free_devp(h->d_near_count);
     free_devp(h->d_perm); free_devp(h->d_key); free_devp(h->d_reach); free_devp(h->d_wmax);
+}
+
+// Whether a handle's steps run two at a time: lattices that step_loop does not
+// take, of 40 MB of populations or more, where the traffic saved outweighs the
+// nodes near the body that are done step by step.
+bool pairs_fit(const lbm_handle *h)
+{
+    return h->overlap && h->kf_tma && h->nseg > 0 && h->nslots % 2 == 0 && h->fbatch % 2 == 0 && !loop_fits(h) && h->nx >= 64 &&
+           h->ny >= 64 && h->plane < (1ll << 31) && 18ll * h->elem * h->plane >= 40000000ll;
 }
 
 // Allocates the immersed-boundary scratch once geometry and motion are known:
@@ -334,6 +347,15 @@ int ensure_ib(lbm_handle *h)
         CK(cudaMemcpyAsync(h->d_key, key.data(), sizeof(double) * h->nseg, cudaMemcpyHostToDevice, h->stream), "copy key");
         CK(cudaMemcpyAsync(h->d_reach, &reach, sizeof(double), cudaMemcpyHostToDevice, h->stream), "copy reach");
         CK(cudaStreamSynchronize(h->stream), "sync order");
+    }
+    if (pairs_fit(h)) {
+        const int cells = near_cells_of(h);
+        CK(dmalloc(h, &h->fmid_alloc, h->elem * (9 * (size_t)h->plane + 2 * LBM_FPAD)), "alloc f between");
+        h->fmid = (char *)h->fmid_alloc + h->elem * LBM_FPAD;
+        CK(dmalloc(h, &h->d_near, S / 2 * near_bytes(cells)), "alloc near cells");
+        CK(dmalloc(h, &h->d_near_list, S / 2 * sizeof(int) * (size_t)cells), "alloc near list");
+        CK(dmalloc(h, &h->d_near_count, S / 2 * sizeof(int)), "alloc near counts");
+        h->pairs = 1;
     }
     if (ib_configure(h) != 0) return set_err(h, LBM_ERR_CUDA, "ib_configure failed");
     h->ib_ready = 1;
@@ -537,6 +559,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             CK(cudaStreamWaitEvent(h->fstream, h->ev_inner, 0), "wait");
         }
         if (launch_factor(h, s0, s1 - s0 + 1, st)) return cuda_err(h, cudaGetLastError(), "launch factor");
+        if (h->pairs && launch_near_cells(h, s0, s1 - s0 + 1, st)) return cuda_err(h, cudaGetLastError(), "launch near cells");
         if (split) CK(cudaEventRecord(h->ev_batch[half], h->fstream), "event");
         return LBM_OK;
     };
@@ -544,6 +567,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
     // a small lattice's steps run as step_loop launches; per-kernel timing
     // needs the kernels one by one
     const bool loop = split && h->timing != LBM_TIMING_KERNELS && loop_fits(h);
+    const bool pairs = split && !loop && h->pairs && h->timing != LBM_TIMING_KERNELS;
     bool joined = loop;   // nothing queued on the side and check streams since the last flush
     // force rows, mass check, status and timing of the steps since the last flush
     auto flush = [&]() -> int {
@@ -611,6 +635,61 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             done += m;
             pending += m;
             s += m - 1;
+            if (pending == h->ring_cap || s == nsteps - 1)
+                if ((rc = flush())) return rc;
+            continue;
+        }
+        // two steps at once: an even one and the next, neither keeping fields
+        if (pairs && h->n % 2 == 0 && s + 1 < nsteps - 2 && pending + 1 < h->ring_cap &&
+            (double)h->n * dt_time <= h->mend + 1.0e-12) {
+            const int slot = pending, b = h->n / K, half = b & 1;
+            const void *fin = h->fbuf[h->cur];
+            void *fout = h->fbuf[h->cur ^ 1];
+            if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
+            if (h->timing == LBM_TIMING_SPAN && slot == 0) CK(cudaEventRecord(h->ev[0], h->stream), "event");
+            for (cudaStream_t st : {h->side, h->nstream}) {
+                CK(cudaStreamWaitEvent(st, h->ev_inner, 0), "wait");
+                CK(cudaStreamWaitEvent(st, h->ev_batch[half], 0), "wait");
+            }
+            cudaEvent_t ei = h->after_interp ? h->ev_interp : nullptr;
+            const void *src = fin;
+            for (int t = 0; t < 2; ++t) {
+                void *dst = t ? fout : h->fmid;
+                const int q = h->n % h->nslots;
+                h->pinfo_slot = q;
+                // the flow chain and the correction tiles; beside them the
+                // other nodes near the bodies (the second step's after the
+                // first step's tiles)
+                if (t) {
+                    CK(cudaStreamWaitEvent(h->side, h->ev_near[0], 0), "wait");
+                    CK(cudaStreamWaitEvent(h->nstream, h->ev_ib, 0), "wait");
+                }
+                if (launch_near(h, src, dst, h->n - t, t, h->nstream)) return cuda_err(h, cudaGetLastError(), "launch near");
+                CK(cudaEventRecord(h->ev_near[t], h->nstream), "event");
+                if (launch_flow(h, src, dst, nullptr, h->n, slot + t, q, h->side, t ? nullptr : ei)) return cuda_err(h, cudaGetLastError(), "launch ib");
+                CK(cudaEventRecord(h->ev_ib, h->side), "event");
+                CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
+                if (launch_check(h, q, slot + t, check_due(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
+                if (t == 0) {
+                    // the next batch's factorization, overlapping this batch's steps
+                    if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
+                    CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
+                    if (ei) CK(cudaStreamWaitEvent(h->stream, ei, 0), "wait");   // the solve starts first
+                    if (launch_pair(h, fin, fout, h->stream)) return cuda_err(h, cudaGetLastError(), "launch pair");
+                    h->launches += 2;   // the lattice, for both steps
+                }
+                src = dst;
+                h->n++;
+            }
+            CK(cudaEventRecord(h->ev_free[half], h->cstream), "event");
+            CK(cudaStreamWaitEvent(h->stream, h->ev_ib, 0), "wait");
+            CK(cudaStreamWaitEvent(h->stream, h->ev_near[1], 0), "wait");
+            CK(cudaEventRecord(h->ev_inner, h->stream), "event");   // both steps are complete
+            h->cur ^= 1;
+            h->steps_done += 2;
+            done += 2;
+            pending += 2;
+            s += 1;
             if (pending == h->ring_cap || s == nsteps - 1)
                 if ((rc = flush())) return rc;
             continue;
@@ -892,7 +971,10 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     if ((e = cudaStreamCreateWithPriority(&h->cstream, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(e, "check stream");
     if ((e = cudaEventCreateWithFlags(&h->ev_cjoin, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
+    if ((e = cudaStreamCreateWithPriority(&h->nstream, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
+        return fail(e, "near stream");
     for (int q = 0; q < 2; ++q) {
+        if ((e = cudaEventCreateWithFlags(&h->ev_near[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
         if ((e = cudaEventCreateWithFlags(&h->ev_batch[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
         if ((e = cudaEventCreateWithFlags(&h->ev_free[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
     }
@@ -956,6 +1038,7 @@ int lbm_destroy(lbm_t *h)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (int b = 0; b < 2; ++b) { free_dev(h->falloc[b]); h->fbuf[b] = nullptr; free_dev(h->d_fields[b]); }
     free_dev(h->edge_c);
@@ -970,6 +1053,7 @@ int lbm_destroy(lbm_t *h)
     free_devp(h->d_stage);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     // the frees above went to the pool on the main stream: once they have
     // completed, an allocation on any other stream may reuse the memory (one
@@ -981,10 +1065,12 @@ int lbm_destroy(lbm_t *h)
     if (h->ev_inner) cudaEventDestroy(h->ev_inner);
     if (h->ev_interp) cudaEventDestroy(h->ev_interp);
     for (int q = 0; q < 2; ++q) {
+        if (h->ev_near[q]) cudaEventDestroy(h->ev_near[q]);
         if (h->ev_batch[q]) cudaEventDestroy(h->ev_batch[q]);
         if (h->ev_free[q]) cudaEventDestroy(h->ev_free[q]);
     }
     if (h->ev_cjoin) cudaEventDestroy(h->ev_cjoin);
+    if (h->nstream) cudaStreamDestroy(h->nstream);
     if (h->cstream) cudaStreamDestroy(h->cstream);
     if (h->fstream) cudaStreamDestroy(h->fstream);
     if (h->side) cudaStreamDestroy(h->side);

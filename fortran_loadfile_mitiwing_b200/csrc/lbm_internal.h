@@ -198,6 +198,15 @@ struct lbm_handle {
     // on this device or in this configuration) and counters
     int loop_ctas = 0;
     unsigned *d_sync = nullptr;
+    // steps of large lattices two at a time: the state between the two steps
+    // near the bodies and at the edge, and the near cells of each pair of
+    // slots (bytes per cell, list, count)
+    int pairs = 0;
+    void *fmid_alloc = nullptr, *fmid = nullptr;
+    unsigned char *d_near = nullptr;
+    int *d_near_list = nullptr, *d_near_count = nullptr;
+    cudaStream_t nstream = nullptr;
+    cudaEvent_t ev_near[2] = {nullptr, nullptr};
     unsigned sync_base = 0;   // their step counter after the launches so far
     double *d_partial = nullptr;
     unsigned *d_counter = nullptr;
@@ -259,6 +268,12 @@ int launch_check_steps_batch(lbm_handle *const *hs, int ncase, const void *dargs
 // the solve residual is checked on every kCheckEvery-th step
 constexpr int kCheckEvery = 4;
 inline bool check_due(int step) { return (step + 1) % kCheckEvery == 0; }
+// two steps in one pass (kf_pair.cu)
+size_t near_bytes(int cells);
+int near_cells_of(const lbm_handle *h);
+int launch_near_cells(lbm_handle *h, int step0, int count, cudaStream_t st);
+int launch_pair(lbm_handle *h, const void *fin, void *fout, cudaStream_t st);
+int launch_near(lbm_handle *h, const void *fin, void *fout, int step, int phase, cudaStream_t st);
 // several steps in one launch (step_loop.cu)
 bool loop_fits(const lbm_handle *h);
 int loop_sync_words();

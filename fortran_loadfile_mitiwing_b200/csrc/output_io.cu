@@ -651,6 +651,7 @@ int lbm_save_checkpoint(lbm_t *h, const char *path)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     CkptHeader hd;
     std::vector<unsigned char> blob;
     int rc = gather_state(h, hd, blob);
@@ -676,6 +677,7 @@ int lbm_load_checkpoint(lbm_t *h, const char *path)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     cudaStreamSynchronize(h->stream);
     const unsigned char *q = blob.data();
     h->cur = 0;

@@ -76,6 +76,12 @@ def patch_extent(case):
     return (min(int(np.max(np.ceil(xhi - xlo))) + 2, p.nx), min(int(np.max(np.ceil(yhi - ylo))) + 2, p.ny))
 
 
+def _pairs(elem, pitch, nx, ny, ns):
+    """Whether the library steps such a case two steps at a time (pairs_fit)."""
+    loop = ns <= 576 and 18 * max(4, elem) * pitch * ny <= 220_000_000
+    return not loop and nx >= 64 and ny >= 64 and 18 * elem * pitch * ny >= 40_000_000
+
+
 def estimate_device_bytes(case):
     """Device bytes a case holds while it is stepped: lattice buffers, fields
     and edge values (lbm_create), step table and contour, and the
@@ -109,6 +115,9 @@ def estimate_device_bytes(case):
         total += S * 8 * max(_NPART * nblk, 2 * ((ns + 7) // 8))
         total += S * 4 * _TILE_INTS * nblk + S * 4 + S * 4 * nblk
         total += S * 4 * ns + S * 8 * ns + 8 + K * 4
+        if _pairs(elem, pitch, nx, ny, ns):                    # two steps at a time: state between, near cells
+            cells = ((nx + 15) // 16) * ((ny + 15) // 16)
+            total += elem * (9 * pitch * ny + 2 * _FPAD) + S // 2 * ((cells + 255) // 256 * 256 + 4 * cells + 4)
     return int(total)
 
 
