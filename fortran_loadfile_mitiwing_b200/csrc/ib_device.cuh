@@ -125,6 +125,7 @@ struct InterpLane {
     bool h0, h1;          // the lane has a first, a second node
     double w0, w1;        // X1(k,i) = kernel1*kernel2 (:1602)
     double ub, vb;
+    int pos;              // where its right-hand sides go (-1: nowhere)
 };
 
 __device__ __forceinline__ InterpLane interp_lane(const IBArgs &a, int k, int lane)
@@ -140,6 +141,11 @@ __device__ __forceinline__ InterpLane interp_lane(const IBArgs &a, int k, int la
     InterpLane l;
     l.ub = mp->ub;
     l.vb = mp->vb;
+    l.pos = mp->pos;
+    if (l.pos < 0 || l.pos >= a.nseg) {
+        if (lane == 0) atomicOr(a.status, LBM_ST_INDEX_INTERP);
+        l.pos = -1;
+    }
     // rows of a node number: n / nbx for n < 64 and nbx <= 6, exact
     const float rn = nn > 0 ? __frcp_rn((float)nbx) : 0.0f;
     const int r0 = (int)(((float)lane + 0.5f) * rn), r1 = (int)(((float)lane + 32.5f) * rn);
@@ -270,6 +276,45 @@ __device__ __forceinline__ void bcr_root(const double *D, int ld, double *X, int
     X[2 * i + c] = x;
 }
 
+// The solution of the marker at position pos after ib_solve, which leaves the
+// odd blocks of the first level, half of all, to whoever needs them: their back
+// substitution (bcr_backward's) waits for nothing but the even blocks, and the
+// tiles have the threads for it. Eight lanes a marker (8 m .. 8 m + 7 of the
+// warp): lane 2 p + c takes sum p of component c; the lanes 0 and 1 return the
+// components, and store them for the residual check.
+__device__ __forceinline__ double marker_solution(const IBArgs &a, int pos, int lane)
+{
+    const int c = lane & 1, part = (lane >> 1) & 3;
+    const int o = pos / BS, i = pos % BS, nb = (a.nseg + BS - 1) / BS;
+    const bool odd = pos >= 0 && (o & 1) && !a.fmode[0];
+    double s = 0.0;
+    if (odd && part < 3) {
+        const int blk = part == 0 ? o : part == 1 ? o - 1 : o + 1;
+        const double *G = a.gf + ((long long)o * BS + i) * GW + part * BS;
+        const double *x = (part == 0 ? a.rhs : a.y) + 2 * blk * BS + c;
+        const int m = blk < nb ? a.nseg - blk * BS : 0;   // past the end: 0
+        if (m >= BS) {
+#pragma unroll
+            for (int t0 = 0; t0 < BS; ++t0) {
+                const int t = (t0 + i) & (BS - 1);
+                s = rfma(G[t], x[2 * t], s);
+            }
+        } else if (blk < nb) {
+#pragma unroll
+            for (int t0 = 0; t0 < BS; ++t0) {
+                const int t = (t0 + i) & (BS - 1);
+                s = rfma(G[t], t < m ? x[2 * t] : 0.0, s);
+            }
+        }
+    }
+    const double s2 = __shfl_down_sync(0xffffffffu, s, 2, 8), s3 = __shfl_down_sync(0xffffffffu, s, 4, 8);
+    if (part != 0 || pos < 0) return 0.0;
+    if (!odd) return a.y[2 * pos + c];
+    const double x = s - s2 - s3;
+    a.y[2 * pos + c] = x;
+    return x;
+}
+
 // ---- a correction tile (TILE_THREADS threads) --------------------------------
 
 struct TileSmem {
@@ -297,9 +342,31 @@ __device__ __forceinline__ bool tile_stage(const IBArgs &a, TileSmem &S, int t, 
     }
     atomicOr(a.status, LBM_ST_INDEX_TILE);
     S.box[t] = make_int4(1, 0, 1, 0);
-    S.y[t][0] = S.y[t][1] = 0.0;
     S.wing[t] = 0;
     return false;
+}
+
+// the position of listed marker k in the solve order (-1 and a report where
+// the list or the marker holds an index out of range)
+__device__ __forceinline__ int tile_position(const IBArgs &a, int k)
+{
+    const int pos = k >= 0 && k < a.nseg ? a.mk[k].pos : -1;
+    if (pos >= 0 && pos < a.nseg) return pos;
+    atomicOr(a.status, LBM_ST_INDEX_TILE);
+    return -1;
+}
+
+// the solution of the n markers of a staged list (marker(t): its t-th), by
+// the tile's threads
+template <class F>
+__device__ __forceinline__ void tile_solve(const IBArgs &a, TileSmem &S, int n, int th, F marker)
+{
+    const int lane = th & 31;
+    for (int m0 = 0; m0 < n; m0 += TILE_THREADS / 8) {
+        const int t = m0 + (th >> 3);
+        const double x = marker_solution(a, t < n ? tile_position(a, marker(t)) : -1, lane);
+        if (t < n && (lane & 7) < 2) S.y[t][lane & 1] = x;
+    }
 }
 
 // du = D^T y at node (gi, gj) from the staged markers first .. n-1, in marker order;

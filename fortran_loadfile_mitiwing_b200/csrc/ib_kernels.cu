@@ -63,7 +63,7 @@ using namespace lbm_ib;
 #define LBM_FACTOR_THREADS 512
 #endif
 #ifndef LBM_SOLVE_THREADS
-#define LBM_SOLVE_THREADS 1024
+#define LBM_SOLVE_THREADS 512
 #endif
 #ifndef LBM_SOLVE_SMEM
 #define LBM_SOLVE_SMEM 232192
@@ -71,25 +71,17 @@ using namespace lbm_ib;
 constexpr int FACTOR_THREADS = LBM_FACTOR_THREADS;
 constexpr int BOPS_WARPS = FACTOR_THREADS / 32;   // warps running block operations
 constexpr int SOLVE_THREADS = LBM_SOLVE_THREADS;
-constexpr int STAGE_BLOCKS = 32;       // factor blocks of one level staged in shared memory by ib_solve
 constexpr int SOLVE_SMEM_BUDGET = LBM_SOLVE_SMEM;   // dynamic shared memory of ib_solve (bytes)
 
-// factor blocks ib_solve can stage next to the right-hand sides of nb blocks
-__host__ __device__ constexpr int stage_cap(int nb)
+// Levels of the reduction whose factor blocks ib_solve keeps in shared memory:
+// those from st0 on (the blocks that are multiples of st0, at index o / st0).
+// Level 1's are read once, in the forward sweep, and stay in L2, so that a
+// solve of 512 markers takes half an SM's shared memory.
+__host__ __device__ constexpr int solve_st0(int nb)
 {
-    return (SOLVE_SMEM_BUDGET - 16 - 2 * nb * BS * (int)sizeof(double)) / (BS * GW * (int)sizeof(double)) < STAGE_BLOCKS
-               ? (SOLVE_SMEM_BUDGET - 16 - 2 * nb * BS * (int)sizeof(double)) / (BS * GW * (int)sizeof(double))
-               : STAGE_BLOCKS;
-}
-// factor blocks a solve of nb blocks stages at once: level 1's odd blocks or
-// those of all the levels above it together, whichever is more (the first
-// and the second staging of the resident form), within stage_cap
-__host__ __device__ constexpr int stage_blocks(int nb)
-{
-    int upper = 0;
-    for (int st = 2; st < nb; st <<= 1) upper += (nb + st - 1) / (2 * st);
-    const int need = nb / 2 > upper ? nb / 2 : upper;
-    return need < stage_cap(nb) ? need : stage_cap(nb);
+    int st = 2;
+    while (((nb + st - 1) / st * BS * GW + 2 * nb * BS) * (int)sizeof(double) + 16 > SOLVE_SMEM_BUDGET) st *= 2;
+    return st;
 }
 constexpr int WS = BS * GP + BS * FL + BS * GP;   // workspace per warp (doubles)
 
@@ -176,7 +168,7 @@ __device__ Marker make_marker(const IBArgs &a, const double *row, int k)
     m.vb = a.uu * (-omega * ca * 0.5 * (a.xb0[p0 + 1] + a.xb0[p0]) -
                    omega * sn * 0.5 * (a.yb0[p0 + 1] + a.yb0[p0]) + sbv);
     m.wing = w;
-    m.pad = 0;
+    m.pos = -1;
     for (int t = 0; t < LBM_BOX; ++t) m.phx[t] = m.phy[t] = 0.0;
     m.i1 = 3; m.i2 = 2; m.j1 = 3; m.j2 = 2;   // empty box unless set below
     // a marker off the lattice (or not finite) is a range error before any scan
@@ -226,8 +218,8 @@ __global__ void __launch_bounds__(128) ib_geometry(const IBArgs base0, const IBA
     a.mk[k] = make_marker(a, row, k);
     // the step's right-hand sides and solution are not there yet (the step
     // loop's CTAs wait for the values themselves)
-    a.rhs[k] = a.rhs[a.nseg + k] = not_yet();
-    a.y[k] = a.y[a.nseg + k] = not_yet();
+    a.rhs[2 * k] = a.rhs[2 * k + 1] = not_yet();
+    a.y[2 * k] = a.y[2 * k + 1] = not_yet();
 }
 
 // one warp per marker: b = D u* over the support box, rhs = U_b - b
@@ -248,10 +240,11 @@ __global__ void __launch_bounds__(256) ib_interp(const IBArgs a0, const IBArgs *
     const int k = blockIdx.x * 8 + warp;
     if (k >= a.nseg) return;
     double ru, rv;
-    interp_sum<T, LdNc>(a, (const T *)a.fin, interp_lane(a, k, lane), ru, rv);
-    if (lane == 0) {
-        a.rhs[k] = ru;
-        a.rhs[a.nseg + k] = rv;
+    const InterpLane il = interp_lane(a, k, lane);
+    interp_sum<T, LdNc>(a, (const T *)a.fin, il, ru, rv);
+    if (lane == 0 && il.pos >= 0) {
+        a.rhs[2 * il.pos] = ru;
+        a.rhs[2 * il.pos + 1] = rv;
     }
 }
 
@@ -384,6 +377,7 @@ __global__ void __launch_bounds__(256) ib_assemble(const IBArgs base0, const IBA
         const int srt = (blk - 1) * BS + m;
         const Marker *mm = (srt >= 0 && srt < n) ? sorted_marker(a, srt, LBM_ST_INDEX_ASSEMBLE) : nullptr;
         bx[m] = mm ? mbox(*mm) : make_int4(1, 0, 1, 0);
+        if (mm && m >= BS) a.mk[mm - a.mk].pos = srt;
     }
     __syncthreads();
     for (int q = tid; q < 2 * BS * BS; q += blockDim.x) {
@@ -739,205 +733,136 @@ __global__ void __launch_bounds__(FACTOR_THREADS, 65536 / (FACTOR_THREADS * 128)
     if (tid == 0 && bad) atomicOr(a.status, LBM_ST_SOLVER);
 }
 
-// The flow-dependent solve of one step, one CTA (solve_threads: up to
-// SOLVE_THREADS threads),
-// with the cyclic-reduction factors of the step's slot:
+// The flow-dependent solve of one step, one CTA (solve_threads threads), with
+// the cyclic-reduction factors of the step's slot:
 //   forward, st = 1, 2, 4, ...:  r_e -= F_L(q)^T r_q + F_U(p)^T r_p  (even e)
 //   block 0:                     x_0 = D_0^-1 r_0
-//   backward, st = ..., 2, 1:    x_o = D_o^-1 r_o - F_L(o) x_p - F_U(o) x_q  (odd o)
+//   backward, st = ..., 4, 2:    x_o = D_o^-1 r_o - F_L(o) x_p - F_U(o) x_q  (odd o)
 // (F_L(q)^T = L_q^T D_q^-1 and F_U(p)^T = L_e D_p^-1 since D is symmetric.)
-// Each level reads the factor blocks of that level's odd blocks; when they
-// fit (at most stage_cap), the lanes of warp 0 bring them into shared memory
-// with bulk copies (one 6-KB block each, completion on an mbarrier) before
-// the level's arithmetic, so that the level costs one memory round trip
-// instead of one per dependent load. The levels above the first usually fit
-// together (31 blocks for 1024 markers): they then come in one round trip and
-// serve both sweeps, so that the whole solve stages three times (level 1,
-// the levels above it, level 1 again) instead of twice per level. Also writes the force row's header and reports the
-// errors of the factorization chain. Dynamic shared memory: the staged
-// blocks, then the right-hand sides in the solve order (two per marker,
-// padded to whole blocks), then the mbarrier.
+// The last backward level, half of the solution, is left to the tiles
+// (marker_solution). What is left is a chain of log2(nb) levels each way in
+// one SM, bound by latency: each level is a chain of 16 to 32 dependent
+// multiply-adds and a barrier. So nothing else waits in it: the factor blocks
+// of the levels from st0 on come into shared memory by bulk copies started
+// before the right-hand sides are read, each warp has its first-level factors
+// in registers by then, and 512 threads with 128 registers keep a level's
+// operands in flight (1024 with 64: 1.2 us a level instead of 0.5).
+// 1024 markers: 34 us -> 15 us alone. Also reports the errors of the
+// factorization chain. Dynamic shared memory: the staged blocks, the
+// right-hand sides (padded to whole blocks), the mbarrier.
 template <bool BATCH>
-__global__ void __launch_bounds__(SOLVE_THREADS, 1024 / SOLVE_THREADS) ib_solve(const IBArgs a0, const IBArgs *batch, int step_index,
-                                                          int ring_slot)
+__global__ void __launch_bounds__(SOLVE_THREADS, 1) ib_solve(const IBArgs a0, const IBArgs *batch)
 {
     const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
     extern __shared__ __align__(128) double smem[];
     const int n = a.nseg, tid = threadIdx.x, nt = blockDim.x;
     const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
-    const int nb = (n + BS - 1) / BS;
-    double *stage_buf = smem;
-    // the staged blocks the launch made room for (solve_smem: stage_blocks(nb)),
-    // read back from the dynamic shared-memory size rather than recomputed
-    uint32_t dsm;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dsm));
-    const int scap = ((int)dsm - 16 - 2 * nb * BS * (int)sizeof(double)) / (BS * GW * (int)sizeof(double));
-    double *X = smem + scap * BS * GW;
+    const int nb = (n + BS - 1) / BS, st0 = solve_st0(nb), nres = (nb + st0 - 1) / st0;
+    double *stage = smem, *X = smem + nres * BS * GW;
     uint64_t *bar = reinterpret_cast<uint64_t *>(X + 2 * nb * BS);
-    __shared__ int timed_out;
     if (tid == 0) {
-        double time;
-        const double *row = motion_row(a, BATCH ? a.cur_step : step_index, &time);
-        // batched launches take the row from the case's arguments (a CUDA
-        // graph replays one launch for many steps)
-        const int rr = BATCH ? a.ring_row : ring_slot;
-        if (rr >= 0 && rr < a.ring_rows)
-            write_header(a, row, time, rr);
-        else
-            atomicOr(a.status, LBM_ST_INDEX_SOLVE);
-        const unsigned fs = *a.fstatus;
-        if (fs) { atomicOr(a.status, fs); *a.fstatus = 0u; }
-        a.solve_res[1] = (double)a.fmode[1];
-        timed_out = 0;
         mbar_init(bar, 1);
         mbar_init_fence();
     }
     __syncthreads();
+    const bool dense = a.fmode[0] != 0;
+    const double *Gf = a.gf;
+    constexpr uint32_t kBlock = sizeof(double) * BS * GW;
+    if (warp == 0 && !dense && n > 0) {
+        if (lane == 0) mbar_expect_tx(bar, kBlock * (uint32_t)nres);
+        __syncwarp();
+        for (int m = lane; m < nres; m += 32)
+            bulk_g2s(stage + m * BS * GW, Gf + (long long)m * st0 * BS * GW, kBlock, bar);
+    }
+    if (tid == nt - 1) {
+        const unsigned fs = *a.fstatus;
+        if (fs) { atomicOr(a.status, fs); *a.fstatus = 0u; }
+        a.solve_res[1] = (double)a.fmode[1];
+    }
     if (n == 0) return;
-    if (a.fmode[0]) {   // dense factor
+    if (dense) {
         for (int s = tid; s < n; s += nt) {
-            const int k = order_at(a, s, LBM_ST_INDEX_SOLVE);
-            X[s] = k >= 0 ? a.rhs[k] : 0.0;
-            X[n + s] = k >= 0 ? a.rhs[n + k] : 0.0;
+            X[s] = a.rhs[2 * s];
+            X[n + s] = a.rhs[2 * s + 1];
         }
         __syncthreads();
         dense_tri(a, X, nt);
+        __syncthreads();
         for (int s = tid; s < n; s += nt) {
-            const int k = order_at(a, s, LBM_ST_INDEX_SOLVE);
-            if (k < 0) continue;
-            a.y[k] = X[s];
-            a.y[n + k] = X[n + s];
+            a.y[2 * s] = X[s];
+            a.y[2 * s + 1] = X[n + s];
         }
         return;
     }
-    for (int s = tid; s < nb * BS; s += nt) {
-        const int k = s < n ? order_at(a, s, LBM_ST_INDEX_SOLVE) : -1;
-        X[2 * s] = k >= 0 ? a.rhs[k] : 0.0;
-        X[2 * s + 1] = k >= 0 ? a.rhs[n + k] : 0.0;
+    // level 1: the warp's first even block's factors, then the right-hand sides
+    const int i = lane & (BS - 1), c = lane >> 4;
+    double fq[BS], fp[BS];
+    const int e1 = 2 * warp;
+    const bool q1 = e1 + 1 < nb, p1 = e1 > 0 && e1 < nb;
+#pragma unroll
+    for (int t = 0; t < BS; ++t) {
+        fq[t] = q1 ? __ldg(Gf + ((long long)(e1 + 1) * BS + t) * GW + BS + i) : 0.0;
+        fp[t] = p1 ? __ldg(Gf + ((long long)(e1 - 1) * BS + t) * GW + 2 * BS + i) : 0.0;
     }
-    const double *Gf = a.gf;
-    uint32_t parity = 0;
-    constexpr uint32_t kBlockBytes = sizeof(double) * BS * GW;
-    auto nodd_of = [&](int st) { return (nb - st + 2 * st - 1) / (2 * st); };
-    // bounded wait for the staged copies: copies that never land are
-    // reported, not waited on forever
-    auto stage_wait = [&]() {
-        int spins = 0;
-        while (!mbar_try_wait(bar, parity)) {
-            if (++spins > (1 << 22)) { timed_out = 1; break; }
-        }
-        parity ^= 1u;
-        __syncthreads();   // every thread sees the same timed_out
-    };
-    // factor blocks of the odd blocks of level st: staged (returns the base
-    // of block o at index (o/st - 1)/2), or read from global memory
-    auto stage_level = [&](int st) -> bool {
-        const int nodd = nodd_of(st);
-        if (nodd > scap) return false;
-        __syncthreads();   // previous readers of the stage buffer are done
-        if (warp == 0) {
-            if (lane == 0) mbar_expect_tx(bar, kBlockBytes * (uint32_t)nodd);
-            __syncwarp();
-            fence_proxy_async();
-            for (int m = lane; m < nodd; m += 32)
-                bulk_g2s(stage_buf + m * BS * GW, Gf + (long long)st * (2 * m + 1) * BS * GW, kBlockBytes, bar);
-        }
-        stage_wait();
-        return true;
-    };
-    // When the odd blocks of every level above the first fit in the stage
-    // buffer together, they are staged once, in one round trip, when the
-    // forward sweep reaches level 2, each level at its own base (upper_base),
-    // and stay there for the rest of the forward sweep and for the backward
-    // sweep down to level 2; only level 1 is staged twice (first and last).
-    int upper = 0;
-    for (int st = 2; st < nb; st <<= 1) upper += nodd_of(st);
-    const bool resident = nodd_of(1) <= scap && upper <= scap;
-    auto upper_base = [&](int st) {
-        int b = 0;
-        for (int s2 = 2; s2 < st; s2 <<= 1) b += nodd_of(s2);
-        return b;
-    };
-    auto stage_upper = [&]() {
-        __syncthreads();   // the first level's readers are done
-        if (warp == 0) {
-            if (lane == 0) mbar_expect_tx(bar, kBlockBytes * (uint32_t)upper);
-            __syncwarp();
-            fence_proxy_async();
-            int b = 0;
-            for (int st = 2; st < nb; st <<= 1) {
-                const int nodd = nodd_of(st);
-                for (int m = lane; m < nodd; m += 32)
-                    bulk_g2s(stage_buf + (b + m) * BS * GW, Gf + (long long)st * (2 * m + 1) * BS * GW, kBlockBytes,
-                             bar);
-                b += nodd;
-            }
-        }
-        stage_wait();
-    };
-    // the stage-buffer base (in blocks) of level st's odd blocks, staging
-    // them first where needed; -1: read them from global memory
-    auto level_base = [&](int st, bool forward) -> int {
-        if (resident && st >= 2) {
-            if (forward && st == 2) stage_upper();
-            return upper_base(st);
-        }
-        return stage_level(st) ? 0 : -1;
-    };
+    for (int s = tid; s < 2 * nb * BS; s += nt) X[s] = s < 2 * n ? a.rhs[s] : 0.0;
     __syncthreads();
-    int levels = 0;
-    for (int st = 1; st < nb; st <<= 1, ++levels) {
-        const int sbase = level_base(st, true);
-        const bool staged = sbase >= 0;
-        if (timed_out) break;
-        const int neven = (nb + 2 * st - 1) / (2 * st);
-        // one even block e per warp, F_L(q) and F_U(p) from staged blocks or
-        // from global memory
-        for (int m = warp; m < neven; m += nw) {
-            const int e = 2 * st * m, o1 = e - st, o2 = e + st;
-            const bool has_q = o2 < nb, has_p = m > 0;
-            if (staged)   // odd block st(2k+1) is staged at index sbase + k
-                bcr_forward(stage_buf + (sbase + m) * BS * GW, stage_buf + (sbase + m - 1) * BS * GW, X, e, st, has_q, has_p,
-                            lane);
-            else
-                bcr_forward(Gf + (long long)o2 * BS * GW, Gf + (long long)o1 * BS * GW, X, e, st, has_q, has_p, lane);
+    if (e1 < nb && nb > 1) {
+        double acc = 0.0;
+        if (q1) {
+#pragma unroll
+            for (int t = 0; t < BS; ++t) acc = rfma(fq[t], X[2 * ((e1 + 1) * BS + t) + c], acc);
         }
-        __syncthreads();
-    }
-    if (!timed_out) {
-        if (warp == 0) bcr_root(Gf, GW, X, lane);
-        __syncthreads();
-        for (int lv = levels - 1; lv >= 0; --lv) {
-            const int st = 1 << lv;
-            const int sbase = level_base(st, false);
-            const bool staged = sbase >= 0;
-            if (timed_out) break;
-            const int nodd = (nb - st + 2 * st - 1) / (2 * st);
-            for (int m = warp; m < nodd; m += nw) {
-                const int o = st * (2 * m + 1);
-                if (staged)
-                    bcr_backward(stage_buf + (sbase + m) * BS * GW, X, o, st, o + st < nb, lane);
-                else
-                    bcr_backward(Gf + (long long)o * BS * GW, X, o, st, o + st < nb, lane);
-            }
-            __syncthreads();
+        if (p1) {
+#pragma unroll
+            for (int t = 0; t < BS; ++t) acc = rfma(fp[t], X[2 * ((e1 - 1) * BS + t) + c], acc);
         }
+        X[2 * (e1 * BS + i) + c] -= acc;
     }
-    if (timed_out) {
+    for (int e = 2 * (warp + nw); e < nb; e += 2 * nw)
+        bcr_forward(Gf + (long long)(e + 1) * BS * GW, Gf + (long long)(e - 1) * BS * GW, X, e, 1, e + 1 < nb, true, lane);
+    // the staged blocks (bounded; copies that never land are reported, not
+    // waited on forever)
+    bool ok = true;
+    int spins = 0;
+    while (!mbar_try_wait(bar, 0))
+        if (++spins > (1 << 22)) {
+            ok = false;
+            break;
+        }
+    if (__syncthreads_or(!ok)) {
         // wait (bounded) for copies still in flight before the CTA's shared
         // memory is released, and report
         if (tid == 0) atomicOr(a.status, LBM_ST_TIMEOUT);
-        int spins = 0;
-        while (!mbar_try_wait(bar, parity ^ 1u) && ++spins < (1 << 22)) {
+        for (spins = 0; !mbar_try_wait(bar, 0) && spins < (1 << 22); ++spins) {
         }
         return;
     }
-    for (int s = tid; s < n; s += nt) {
-        const int k = order_at(a, s, LBM_ST_INDEX_SOLVE);
-        if (k < 0) continue;
-        a.y[k] = X[2 * s];
-        a.y[n + k] = X[2 * s + 1];
+    auto block = [&](int o, int st) { return st >= st0 ? stage + o / st0 * BS * GW : Gf + (long long)o * BS * GW; };
+    int st = 2;
+    for (; st < nb; st <<= 1) {
+        for (int e = 2 * st * warp; e < nb; e += 2 * st * nw) {
+            const bool q = e + st < nb, p = e > 0;
+            if (st >= st0)   // (two forms, so that staged reads are shared loads)
+                bcr_forward(stage + (e + st) / st0 * BS * GW, stage + (e - st) / st0 * BS * GW, X, e, st, q, p, lane);
+            else
+                bcr_forward(block(e + st, st), block(e - st, st), X, e, st, q, p, lane);
+        }
+        __syncthreads();
     }
+    if (warp == 0) bcr_root(stage, GW, X, lane);
+    __syncthreads();
+    for (st >>= 1; st > 1; st >>= 1) {
+        for (int o = st * (2 * warp + 1); o < nb; o += 2 * st * nw) {
+            if (st >= st0)
+                bcr_backward(stage + o / st0 * BS * GW, X, o, st, o + st < nb, lane);
+            else
+                bcr_backward(block(o, st), X, o, st, o + st < nb, lane);
+        }
+        __syncthreads();
+    }
+    // the even blocks' solution (without a first level: all there is)
+    for (int s = tid; s < 2 * n; s += nt)
+        if ((s / (2 * BS) & 1) == 0) a.y[s] = X[s];
 }
 
 // Markers whose support box meets each 16 x 16 tile of the step's patch
@@ -1074,6 +999,11 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) ib_tile_sort(const IBArgs bas
 // Needed by no kernel of the step, so it runs after the step's update.
 __device__ __forceinline__ void force_row(const IBArgs &a, int rr)
 {
+    if (threadIdx.x == 32 && rr >= 0 && rr < a.ring_rows) {
+        double time;
+        const double *row = motion_row(a, a.cur_step, &time);
+        write_header(a, row, time, rr);
+    }
     __shared__ double red[8][NPART];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nt = patch_tiles(a);
@@ -1147,11 +1077,6 @@ __global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, const vo
     const IBArgs &base = BATCH ? loop_case(batch, stride) : a0;
     const int step = base.cur_step + (int)blockIdx.x, rr = base.ring_row + (int)blockIdx.x;
     const IBArgs a = step_args(base, step);
-    if (threadIdx.x == 0 && rr >= 0 && rr < a.ring_rows) {
-        double time;
-        const double *row = motion_row(a, step, &time);
-        write_header(a, row, time, rr);
-    }
     force_row(a, rr);
 }
 
@@ -1181,17 +1106,16 @@ __device__ __forceinline__ void solve_residual(const IBArgs &a)
             if (t < 0 || t >= n) continue;
             const Marker *ml = sorted_marker(a, t, LBM_ST_INDEX_RESIDUAL);
             if (!ml) continue;
-            const int l = (int)(ml - a.mk);
             const double b = bval(ms, *ml);
-            b0 += b * a.y[l];
-            b1 += b * a.y[n + l];
+            b0 += b * a.y[2 * t];
+            b1 += b * a.y[2 * t + 1];
         }
 #pragma unroll
         for (int off = 16; off; off >>= 1) {
             b0 += __shfl_xor_sync(0xffffffffu, b0, off);
             b1 += __shfl_xor_sync(0xffffffffu, b1, off);
         }
-        const double q0 = a.rhs[ks], q1 = a.rhs[n + ks];
+        const double q0 = a.rhs[2 * s], q1 = a.rhs[2 * s + 1];
         rnum = (b0 - q0) * (b0 - q0) + (b1 - q1) * (b1 - q1);
         rden = q0 * q0 + q1 * q1;
     }
@@ -1266,6 +1190,7 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
     const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
     const KFArgs<C> &kf = BATCH ? kbatch[blockIdx.z] : kf0;
     __shared__ TileSmem S;
+    __shared__ int smark[TILE_THREADS];   // the staged markers, where a list overflows
     const int nt = patch_tiles(a);
     const int ntile = *a.nsup;
     if (ntile == 0) return;   // no correction tile
@@ -1308,11 +1233,9 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
             // markers listed for this tile by the factorization chain
             if ((int)threadIdx.x < listed) {
                 const int k = tlist[1 + threadIdx.x];
-                if (tile_stage(a, S, threadIdx.x, k)) {
-                    S.y[threadIdx.x][0] = a.y[k];
-                    S.y[threadIdx.x][1] = a.y[a.nseg + k];
-                }
+                tile_stage(a, S, threadIdx.x, k);
             }
+            tile_solve(a, S, listed, threadIdx.x, [&](int t) { return tlist[1 + t]; });
             __syncthreads();
             if (active) tile_gather(S, 0, listed, gi, gj, du, dv, wing);
         } else {
@@ -1340,11 +1263,11 @@ __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBA
                 __syncthreads();
                 if (hit) {
                     const int slot = S.wsum[warp] + __popc(bal & ((1u << lane) - 1u));
-                    if (tile_stage(a, S, slot, k)) {
-                        S.y[slot][0] = a.y[k];
-                        S.y[slot][1] = a.y[a.nseg + k];
-                    }
+                    tile_stage(a, S, slot, k);
+                    smark[slot] = k;
                 }
+                __syncthreads();
+                tile_solve(a, S, S.nlist, threadIdx.x, [&](int t) { return smark[t]; });
                 __syncthreads();
                 if (active) tile_gather(S, 0, S.nlist, gi, gj, du, dv, wing);
                 __syncthreads();
@@ -1381,7 +1304,8 @@ constexpr size_t kSolveSmemMax = SOLVE_SMEM_BUDGET;
 size_t solve_smem(int nseg)
 {
     const int nb = (nseg + BS - 1) / BS;
-    return sizeof(double) * ((size_t)stage_blocks(nb) * BS * GW + 2 * (size_t)nb * BS) + 16;
+    const int st0 = solve_st0(nb);
+    return sizeof(double) * ((size_t)((nb + st0 - 1) / st0) * BS * GW + 2 * (size_t)nb * BS) + 16;
 }
 
 // threads of the solve's CTA: one warp per even block of the first level
@@ -1461,7 +1385,7 @@ int launch_flow_t(lbm_handle *h, const void *fin, void *fout, void *fields, int 
         h->launches += 1;
     }
     if (after_interp && cudaEventRecord(after_interp, st) != cudaSuccess) return -1;
-    ib_solve<false><<<1, solve_threads(h->nseg), solve_smem(h->nseg), st>>>(a, nullptr, step_index, ring_slot);
+    ib_solve<false><<<1, solve_threads(h->nseg), solve_smem(h->nseg), st>>>(a, nullptr);
     const int grid = std::min(h->patch_gx() * h->patch_gy(), 2 * 148);   // strided over the correction tiles
     const KFArgs<C> kf = make_kf_args<C>(h, fin, fout, fields, KF_OUTER);
     if (fields)
@@ -1619,8 +1543,7 @@ int launch_flow_batch_t(lbm_handle *const *hs, int ncase, const IBArgs *dargs, c
     const int ns = max_seg(hs, ncase);
     ib_interp<T, true><<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs);
     if (after_interp && cudaEventRecord(after_interp, st) != cudaSuccess) return -1;
-    ib_solve<true><<<dim3(1, 1, ncase), solve_threads(ns), solve_smem(ns), st>>>(IBArgs{}, dargs, step_index,
-                                                                                ring_slot);
+    ib_solve<true><<<dim3(1, 1, ncase), solve_threads(ns), solve_smem(ns), st>>>(IBArgs{}, dargs);
     // CTAs per case, strided over the case's correction tiles: the patch
     // grids bound the tiles several times over (a sweep case of chord 256
     // has some 60 correction tiles in a grid of hundreds), and CTAs past a

@@ -484,12 +484,17 @@ int cells_of(const lbm_handle *h, int *cx, int *cy)
     return *cx * *cy;
 }
 
-// rows a CTA writes: 18 to 20 where the lattice has two waves of such CTAs (the
-// two rows computed twice cost 10 %), fewer on smaller lattices
+// rows a CTA writes. Two more are computed by it for the first step only, so
+// the kernel alone is fastest with 16 to 20; but the immersed-boundary kernels
+// beside it start as its CTAs leave, and the step as a whole is faster with
+// shorter ones (4096x2048, us a step with 8, 10, 12, 14, 20 rows: FP32 77.7,
+// 76.9, 76.8, 78.1, 79.8; FP16 63.3, 63.0, 65.3, 64.9, 66.8; FP64 133.6,
+// 130.3, 129.3, 128.3, 127.5). Fewer where the lattice has not two waves of
+// such CTAs.
 template <typename T> int pair_rows(const lbm_handle *h)
 {
     const int per_sm = sizeof(T) == 8 ? 2 : 4, strips = (h->nx - 2 * FRAME + pair_out<T>() - 1) / pair_out<T>();
-    int r = sizeof(T) == 2 ? 18 : 20;
+    int r = sizeof(T) == 2 ? 10 : (sizeof(T) == 4 ? 12 : 20);
     while (r > 8 && strips * ((h->ny - 2 * FRAME + r - 1) / r) < 2 * 148 * per_sm) r -= 2;
     return r;
 }

@@ -64,7 +64,7 @@ struct Marker {
     double phy[LBM_BOX];      // one-axis kernel at nodes j1..j1+5
     int i1, i2, j1, j2;       // support box, 0-based inclusive (airfoil.f90:290-321)
     int wing;                 // 0-based
-    int pad;
+    int pos;                  // position in the solve order (ib_assemble)
 };
 
 // A support box (0-based, inclusive: x..y columns, z..w rows) as make_marker

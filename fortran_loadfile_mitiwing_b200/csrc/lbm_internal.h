@@ -68,6 +68,7 @@ struct IBArgs {
     int *fmode;         // [2]: 1 if the dense factor is used, half-bandwidth
     unsigned *fstatus;  // errors of the factorization chain of the slot's step
     // per step
+    // right-hand sides and solution, pairs (x, y component) in the solve order
     double *rhs;        // [2*nseg]
     double *y;          // [2*nseg]
     double *bD, *bL;    // working diagonal and coupling blocks of the reduction

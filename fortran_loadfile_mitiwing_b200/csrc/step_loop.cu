@@ -93,14 +93,14 @@ __device__ __forceinline__ bool wait_step(unsigned *sync, unsigned target, unsig
     return false;
 }
 
-// bounded wait for the two values p[0] and p[n] of a marker (right-hand side
+// bounded wait for the two values p[0] and p[1] of a marker (right-hand sides
 // or solution); false when it gave up or another CTA did
-__device__ __forceinline__ bool wait_pair(const double *p, int n, unsigned *sync, unsigned *status, double &x, double &y)
+__device__ __forceinline__ bool wait_pair(const double *p, unsigned *sync, unsigned *status, double &x, double &y)
 {
     for (int spins = 0; spins < SPINS; ++spins) {
         long long a, b;
         asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
-        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(b) : "l"(p + n) : "memory");
+        asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(b) : "l"(p + 1) : "memory");
         if (a != (long long)LBM_NOT_YET && b != (long long)LBM_NOT_YET) {
             x = __longlong_as_double(a);
             y = __longlong_as_double(b);
@@ -333,9 +333,8 @@ __device__ __forceinline__ void solver_cta(const LoopArgs<C> &L, double *smem)
         // there (16-byte pairs; the dense solve keeps the two apart)
         const int np = dense ? n : nb * BS;
         for (int q = tid; q < np && ok; q += NT) {
-            const int k = q < n ? order_at(a, q, LBM_ST_INDEX_SOLVE) : -1;
             double x = 0.0, y = 0.0;
-            if (k >= 0) ok = wait_pair(a.rhs + k, n, L.sync, a.status, x, y);
+            if (q < n) ok = wait_pair(a.rhs + 2 * q, L.sync, a.status, x, y);
             X[dense ? q : 2 * q] = x;
             X[dense ? n + q : 2 * q + 1] = y;
         }
@@ -367,10 +366,8 @@ __device__ __forceinline__ void solver_cta(const LoopArgs<C> &L, double *smem)
             }
         }
         for (int q = tid; q < n; q += NT) {
-            const int k = order_at(a, q, LBM_ST_INDEX_SOLVE);
-            if (k < 0) continue;
-            put_value(a.y + k, X[dense ? q : 2 * q]);
-            put_value(a.y + n + k, X[dense ? n + q : 2 * q + 1]);
+            put_value(a.y + 2 * q, X[dense ? q : 2 * q]);
+            put_value(a.y + 2 * q + 1, X[dense ? n + q : 2 * q + 1]);
         }
         __syncthreads();
         if (s + 1 < L.nsteps) issue(s + 1);
@@ -475,7 +472,7 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
         mark = -1;
         if (listed <= TILE_CAP && gt < listed) {
             mark = tl[1 + gt];
-            if (!tile_stage(a, S, gt, mark)) mark = -1;
+            mark = tile_stage(a, S, gt, mark) ? tile_position(a, mark) : -1;
         }
         group_sync(grp);
         wing = 1 << 20;
@@ -492,9 +489,9 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
             if (k > k0) il = interp_lane(a, k, lane);
             double ru, rv;
             interp_sum<T, LdCg>(a, fin, il, ru, rv);
-            if (lane == 0) {
-                put_value(a.rhs + k, ru);
-                put_value(a.rhs + n + k, rv);
+            if (lane == 0 && il.pos >= 0) {
+                put_value(a.rhs + 2 * il.pos, ru);
+                put_value(a.rhs + 2 * il.pos + 1, rv);
             }
         }
         // while the solver works: the nodes outside the correction tiles, edge
@@ -517,9 +514,11 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
             if (listed <= TILE_CAP) {
                 if (mark >= 0) {
                     double x = 0.0, y = 0.0;
-                    if (!wait_pair(a.y + mark, n, L.sync, a.status, x, y)) good[grp] = 0;
+                    if (!wait_pair(a.y + 2 * mark, L.sync, a.status, x, y)) good[grp] = 0;
                     S.y[gt][0] = x;
                     S.y[gt][1] = y;
+                } else if (gt < listed) {
+                    S.y[gt][0] = S.y[gt][1] = 0.0;
                 }
                 group_sync(grp);
                 if (active) tile_sum(S, W, cnt, listed, gi, gj, gt, du, dv);
@@ -550,12 +549,11 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
                     }
                     if (hit) {
                         const int at = before + __popc(bal & ((1u << lane) - 1u));
-                        if (tile_stage(a, S, at, k)) {
-                            double x = 0.0, y = 0.0;
-                            if (!wait_pair(a.y + k, n, L.sync, a.status, x, y)) good[grp] = 0;
-                            S.y[at][0] = x;
-                            S.y[at][1] = y;
-                        }
+                        const int pos = tile_stage(a, S, at, k) ? tile_position(a, k) : -1;
+                        double x = 0.0, y = 0.0;
+                        if (pos >= 0 && !wait_pair(a.y + 2 * pos, L.sync, a.status, x, y)) good[grp] = 0;
+                        S.y[at][0] = x;
+                        S.y[at][1] = y;
                     }
                     group_sync(grp);
                     if (active) tile_gather(S, 0, all, gi, gj, du, dv, wing);
