@@ -945,8 +945,11 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         // a graph segment where the next kGraphSteps steps allow one. Segments
         // start at every half of a factorization batch (of the first case),
         // so that runs of any length need two structures, not one for each
-        // phase of the batch
-        if (b->graphs && act[0]->n % std::max(1, K / 2) == 0 && (tcur >= 0 || !share.empty()) && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
+        // phase of the batch. step_loop launches end with the batch, so a call
+        // of some batches starts at whole ones (one launch a segment), and
+        // only a shorter one at a quarter
+        const int gstart = std::max(1, share.empty() ? K / 2 : (nsteps < 4 * K ? K / 4 : K));
+        if (b->graphs && act[0]->n % gstart == 0 && (tcur >= 0 || !share.empty()) && act == prev_act && step + kGraphSteps <= nsteps - 2 &&
             pending + kGraphSteps <= ring_cap) {
             bool ok = true;
             for (size_t c = 0; c < act.size() && ok; ++c) ok = act[c]->n + kGraphSteps < last_step[act_idx[c]];
@@ -962,7 +965,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             int m = std::min({K - act[0]->n % K, nsteps - step, ring_cap - pending});
             for (size_t c = 0; c < act.size(); ++c) m = std::min(m, last_step[act_idx[c]] - act[c]->n + 1);
             // up to where a graph segment may start
-            if (b->graphs && K > 1 && act[0]->n % (K / 2)) m = std::min(m, K / 2 - act[0]->n % (K / 2));
+            if (b->graphs && act[0]->n % gstart) m = std::min(m, gstart - act[0]->n % gstart);
             if ((rc = loop_chunk(m))) break;
             step += m - 1;
             pending += m;

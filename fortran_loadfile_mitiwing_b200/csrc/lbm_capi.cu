@@ -563,6 +563,12 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         if (split) CK(cudaEventRecord(h->ev_batch[half], h->fstream), "event");
         return LBM_OK;
     };
+    // The next batch's factorization runs beside this batch's steps; a call that
+    // ends in the first half of a batch leaves it to a later one.
+    auto factor_next = [&](int b, int s) -> int {
+        if ((b + 1) * K > last_step || h->batch_in_half[(b + 1) & 1] == b + 1 || h->n % K + (nsteps - s) <= K / 2) return LBM_OK;
+        return factor_batch(b + 1);
+    };
     int done = 0, pending = 0;
     // a small lattice's steps run as step_loop launches; per-kernel timing
     // needs the kernels one by one
@@ -606,7 +612,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
             // the next batch's factorization, beside this launch (it waits for
             // the previous one, not for this one)
-            if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
+            if ((rc = factor_next(b, s))) return rc;
             void *fields[LBM_NSLOT_MAX] = {};
             for (int t = 0; t < m; ++t)
                 if (fields_every || s + t >= nsteps - 2) {
@@ -671,8 +677,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
                 CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
                 if (launch_check(h, q, slot + t, check_due(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
                 if (t == 0) {
-                    // the next batch's factorization, overlapping this batch's steps
-                    if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
+                    if ((rc = factor_next(b, s))) return rc;
                     CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
                     if (ei) CK(cudaStreamWaitEvent(h->stream, ei, 0), "wait");   // the solve starts first
                     if (launch_pair(h, fin, fout, h->stream)) return cuda_err(h, cudaGetLastError(), "launch pair");
@@ -729,8 +734,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
             if (launch_check(h, q, slot, check_res, h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
             CK(cudaEventRecord(h->ev_free[half], h->cstream), "event");
-            // the next batch's factorization, overlapping this batch's steps
-            if ((b + 1) * K <= last_step && h->batch_in_half[half ^ 1] != b + 1 && (rc = factor_batch(b + 1))) return rc;
+            if ((rc = factor_next(b, s))) return rc;
             CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");   // the step's correction tiles
             if (ei) CK(cudaStreamWaitEvent(h->stream, ei, 0), "wait");   // the solve starts first
             if (e) CK(cudaEventRecord(e[0], h->stream), "event");

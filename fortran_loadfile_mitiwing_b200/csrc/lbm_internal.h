@@ -38,7 +38,7 @@ struct KFArgs {
     unsigned *status;                  // device status word (bounded-wait timeouts)
 };
 
-#define LBM_NSLOT_MAX 16   // largest slot count of the factorization batches
+#define LBM_NSLOT_MAX 32   // largest slot count of the factorization batches
 #define LBM_FPAD 64   // elements of padding before and after the population planes
 
 #define KF_ALL 0
@@ -146,8 +146,13 @@ struct lbm_handle {
     // index only (prescribed motion). Steps are factorized in batches of
     // fbatch consecutive steps (batch b: steps b*fbatch .. b*fbatch+fbatch-1),
     // each step into slot step % nslots (nslots = 2 fbatch): the next batch
-    // is factorized while the steps of the current one run.
-    int fbatch = 8, nslots = 16;
+    // is factorized while the steps of the current one run. The chain of a
+    // batch takes some 120 us whatever its length (one CTA a step, each a
+    // serial chain), so a small lattice's steps wait for it unless the batch
+    // is long: us a step with 4, 8 and 16 steps, 1001x501 with two wings 32,
+    // 17.6, 13.7; 400x200 20, 11.8, 9.6; and 16 make a step_loop launch of
+    // 16 steps (96x64: 9.2 -> 8.0).
+    int fbatch = 16, nslots = 32;
     int batch_in_half[2] = {-1, -1};                // batch index held by each half of the slots
     Marker *d_mk = nullptr;                         // nslots x nseg
     double *d_B = nullptr;                          // nslots x nseg*nseg

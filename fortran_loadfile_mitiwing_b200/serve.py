@@ -35,14 +35,14 @@ from .solver import Batch, Lbm
 # sizes of the device structures a case holds (csrc/lbm_common.cuh, lbm_internal.h, ib_kernels.cu)
 _MARKER_BYTES = 152        # struct Marker
 _PATCHINFO_BYTES = 16      # struct PatchInfo
-_NSLOT_MAX = 16            # LBM_NSLOT_MAX
+_NSLOT_MAX = 32            # LBM_NSLOT_MAX
 _FPAD = 64                 # LBM_FPAD elements before and after the population planes
 _RING = 2048               # force rows kept on the device
 _MAXW = 8                  # LBM_MAXW
 _NPART = 3 * _MAXW + 3     # per-tile partials of the correction
 _TILE_INTS = 257           # per-tile list: count + 256 markers
 _BS, _GW = 16, 48          # block size and factor row width of the marker solve
-_FBATCH = 8                # steps per factorization batch (LBM_IB_BATCH)
+_FBATCH = 16               # steps per factorization batch (LBM_IB_BATCH)
 _MASS_BLOCKS = 296         # CTAs of the mass check (kf_kernel.cu)
 
 
@@ -85,7 +85,7 @@ def _pairs(elem, pitch, nx, ny, ns):
 def estimate_device_bytes(case):
     """Device bytes a case holds while it is stepped: lattice buffers, fields
     and edge values (lbm_create), step table and contour, and the
-    immersed-boundary scratch of 2 x 8 step slots (first step)."""
+    immersed-boundary scratch of 2 x 16 step slots (first step)."""
     p = case.params
     nx, ny = p.nx, p.ny
     elem = _elem_bytes(p.precision)
