@@ -24,9 +24,9 @@
 // chain, and what it does not need (the forces of a tile) is left for after.
 //
 // Measured on a B200, us a step, launches per stage -> here: 96x64 27.9 ->
-// 9.1; 400x200 33.5 -> 11.7 (FP64 31.7 -> 12.5); 1001x501 with two wings
-// 42 -> 18; 1280x640 42 -> 16.8; 2048x1024 in BF16 46 -> 30, where the
-// lattice's 18 us, L2 traffic by loads through registers, are most of it.
+// 8.0; 400x200 33.5 -> 9.5 (FP64 31.7 -> 11.2); 1001x501 with two wings
+// 42 -> 13.4; 1280x640 42 -> 15.4; 2048x1024 in BF16 46 -> 25.3, of which
+// 20 are the lattice (with its loads through registers 24).
 // On large lattices the staged kernel is the better one (loop_fits).
 //
 // The force rows and residual checks of the steps follow as ordinary launches
@@ -161,7 +161,65 @@ __device__ __forceinline__ bool in_tile(const IBArgs &a, const PatchInfo &r, int
 // One warp's item of the interior: with FP32 arithmetic two nodes per lane
 // (rows j, j + 1 of a column, or with 2-byte storage columns i, i + 1 of a
 // row) by the paired update, as in the staged lattice kernel; one node per
-// lane in FP64.
+// lane in FP64. An item's rows come into the warp's part of shared memory by
+// 16-byte asynchronous copies (through L2: other CTAs wrote them), some items
+// ahead: with loads into registers, of which 512 threads have 128 each, only
+// one item's were in flight and a third of the time went into waiting for them.
+template <typename T> struct Items {
+    static constexpr int AL = 16 / (int)sizeof(T);                // elements of a copy
+    static constexpr int COLS = sizeof(T) == 2 ? 64 : 32;         // of an item
+    static constexpr int ROWS = sizeof(T) == 4 ? 2 : 1;
+    static constexpr int SEG = COLS / AL;                         // copies of a row's segment, one more where it is shifted
+    static constexpr int ROW = 9 * SEG + 6;                       // copies of a row
+    static constexpr int BYTES = ROWS * ROW * 16;
+    static constexpr int STAGES = sizeof(T) == 2 ? 4 : 2;
+    // the first copy of population k's segment
+    static __host__ __device__ constexpr int at(int k)
+    {
+        int c = 0;
+        for (int q = 0; q < k; ++q) c += SEG + (lbm_ex(q) != 0);
+        return c;
+    }
+};
+
+// offsets of a row's copies from its node (i0, j), for the launch
+template <typename T> __device__ __forceinline__ void item_table(int *tab, int plane, int pitch)
+{
+    using I = Items<T>;
+    for (int c = threadIdx.x; c < I::ROW; c += NT) {
+        int k = 0, q = c;
+        while (q >= I::SEG + (lbm_ex(k) != 0)) {
+            q -= I::SEG + (lbm_ex(k) != 0);
+            ++k;
+        }
+        tab[c] = k * plane - lbm_ey(k) * pitch + (q - (lbm_ex(k) == 1)) * I::AL;   // (9 planes < 2^31 elements, loop_fits)
+    }
+}
+
+// A warp's copies of an item into its stage. The segments' ends may lie up to
+// 16 bytes outside the rows; the buffers are padded for that.
+template <typename T, typename C>
+__device__ __forceinline__ void item_issue(const KFArgs<C> &a, const T *fin, const int *tab, unsigned char *stage, int item,
+                                           int segs, int lane)
+{
+    using I = Items<T>;
+    const int r = item / segs, sg = item - r * segs, j = 1 + I::ROWS * r;
+    const T *row = fin + j * a.pitch + sg * I::COLS;
+    const int up = I::ROWS == 2 && j + 1 <= a.ny - 2 ? a.pitch : 0;   // an odd last row fills both halves
+    const uint32_t dst = smem_u32(stage);
+#pragma unroll
+    for (int t = 0; t < (I::ROWS * I::ROW + 31) / 32; ++t) {
+        const int c = 32 * t + lane;
+        if (c < I::ROWS * I::ROW) {
+            const bool second = I::ROWS == 2 && c >= I::ROW;
+            const T *src = row + tab[second ? c - I::ROW : c] + (second ? up : 0);
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + 16 * c), "l"(__cvta_generic_to_global(src)) : "memory");
+        }
+    }
+}
+__device__ __forceinline__ void copies_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
 template <typename T> struct LatticeItem {
     float2 g[9];
     int i, j;
@@ -174,48 +232,43 @@ template <> struct LatticeItem<double> {
 };
 
 template <typename T, typename C>
-__device__ __forceinline__ void item_load(LatticeItem<T> &x, const KFArgs<C> &a, const IBArgs &ib, const PatchInfo &pr,
-                                          const T *fin, int item, int segs, int lane)
+__device__ __forceinline__ void item_nodes(LatticeItem<T> &x, const KFArgs<C> &a, const IBArgs &ib, const PatchInfo &pr, int item,
+                                           int segs, int lane)
 {
     const int r = item / segs, sg = item - r * segs;
-    const int pitch = a.pitch, plane = (int)a.plane;   // 9 planes < 2^31 elements (loop_fits)
     if constexpr (sizeof(T) == 2) {
-        const int j = 1 + r, i = 2 * (32 * sg + lane);
-        x.i = i;
-        x.j = j;
-        x.w0 = i >= 1 && i <= a.nx - 2 && !in_tile(ib, pr, i, j);
-        x.w1 = i + 1 <= a.nx - 2 && !in_tile(ib, pr, i + 1, j);
-        if (!x.w0 && !x.w1) return;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const uint32_t *wk = reinterpret_cast<const uint32_t *>(fin + k * plane + (j - lbm_ey(k)) * pitch + i);
-            uint32_t w;
-            if (lbm_ex(k) == 0) w = __ldcg(wk);
-            else if (lbm_ex(k) == 1) w = __byte_perm(__ldcg(wk - 1), __ldcg(wk), 0x5432);   // columns i-1, i
-            else w = __byte_perm(__ldcg(wk), __ldcg(wk + 1), 0x5432);                       // columns i+1, i+2
-            x.g[k] = Pair2<T>::unpack(w);
-        }
-    } else if constexpr (sizeof(T) == 4) {
-        const int j = 1 + 2 * r, i = 32 * sg + lane;
-        const bool in = i >= 1 && i <= a.nx - 2, second = j + 1 <= a.ny - 2;
-        x.i = i;
-        x.j = j;
-        x.w0 = in && !in_tile(ib, pr, i, j);
-        x.w1 = in && second && !in_tile(ib, pr, i, j + 1);
-        if (!x.w0 && !x.w1) return;
-        const int up = second ? pitch : 0;   // an odd last row fills both halves
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const T *p = fin + k * plane + (j - lbm_ey(k)) * pitch + (i - lbm_ex(k));
-            x.g[k] = make_float2(__ldcg(p), __ldcg(p + up));
-        }
+        x.j = 1 + r;
+        x.i = 2 * (32 * sg + lane);
+        x.w0 = x.i >= 1 && x.i <= a.nx - 2 && !in_tile(ib, pr, x.i, x.j);
+        x.w1 = x.i + 1 <= a.nx - 2 && !in_tile(ib, pr, x.i + 1, x.j);
     } else {
-        const int j = 1 + r, i = 32 * sg + lane;
-        x.i = i;
-        x.j = j;
-        x.w0 = i >= 1 && i <= a.nx - 2 && !in_tile(ib, pr, i, j);
-        x.w1 = false;
-        if (x.w0) pull<T, C, LdCg>(fin, a.plane, pitch, i, j, x.g);
+        x.j = sizeof(T) == 4 ? 1 + 2 * r : 1 + r;
+        x.i = 32 * sg + lane;
+        const bool in = x.i >= 1 && x.i <= a.nx - 2;
+        x.w0 = in && !in_tile(ib, pr, x.i, x.j);
+        x.w1 = sizeof(T) == 4 && in && x.j + 1 <= a.ny - 2 && !in_tile(ib, pr, x.i, x.j + 1);
+    }
+}
+
+// the lane's populations from the stage
+template <typename T> __device__ __forceinline__ void item_read(LatticeItem<T> &x, const unsigned char *stage, int lane)
+{
+    using I = Items<T>;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const unsigned char *seg = stage + 16 * I::at(k);
+        if constexpr (sizeof(T) == 2) {
+            const uint32_t *w = reinterpret_cast<const uint32_t *>(seg) + lane;
+            uint32_t v;
+            if (lbm_ex(k) == 0) v = w[0];
+            else if (lbm_ex(k) == 1) v = __byte_perm(w[I::AL / 2 - 1], w[I::AL / 2], 0x5432);   // columns i-1, i
+            else v = __byte_perm(w[0], w[1], 0x5432);                                           // columns i+1, i+2
+            x.g[k] = Pair2<T>::unpack(v);
+        } else {
+            const T *e = reinterpret_cast<const T *>(seg) + lane + (lbm_ex(k) == 1 ? I::AL - 1 : (lbm_ex(k) == -1 ? 1 : 0));
+            if constexpr (sizeof(T) == 4) x.g[k] = make_float2(e[0], e[4 * I::ROW]);
+            else x.g[k] = e[0];
+        }
     }
 }
 
@@ -409,6 +462,13 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
     const KFArgs<C> &kf = L.kf;
     TileSmem &S = reinterpret_cast<GroupSmem *>(smem)[grp].tile;
     TileWeights &W = reinterpret_cast<GroupSmem *>(smem)[grp].weights;
+    // the warp's stages of the lattice update, after the groups' tiles
+    using I = Items<T>;
+    static_assert(NG * sizeof(GroupSmem) + NW * I::STAGES * I::BYTES <= LOOP_SMEM, "shared memory");
+    unsigned char *stage = reinterpret_cast<unsigned char *>(smem) + NG * sizeof(GroupSmem) + warp * I::STAGES * I::BYTES;
+    __shared__ int tab[I::ROW];
+    item_table<T>(tab, (int)kf.plane, kf.pitch);
+    __syncthreads();
     const int n = L.ib.nseg, nx = kf.nx, ny = kf.ny;
     constexpr bool XPAIR = sizeof(T) == 2, YPAIR = sizeof(T) == 4;
     const int segs = XPAIR ? (nx + 63) / 64 : (nx + 31) / 32;
@@ -499,10 +559,24 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
         const PatchInfo pr = *a.pinfo;
         const int et = duty ? TILE_THREADS + gt : gt;   // thread of the CTA, the free group first
         for (int e = (TILE_THREADS - 1 - et + (duty ? NT : 0)) * G + cta; e < nedge; e += nthr) edge_node<T, C>(kf, fin, fout, fl, e);
-        for (int it = (et >> 5) * G + cta; it < items; it += NW * G) {
+        int it = (et >> 5) * G + cta;
+#pragma unroll
+        for (int t = 0; t < I::STAGES - 1; ++t) {
+            if (it + t * NW * G < items) item_issue<T, C>(kf, fin, tab, stage + t * I::BYTES, it + t * NW * G, segs, lane);
+            copies_commit();
+        }
+        for (int q = 0; it < items; it += NW * G) {
+            const int qn = q == 0 ? I::STAGES - 1 : q - 1, ahead = it + (I::STAGES - 1) * NW * G;
+            if (ahead < items) item_issue<T, C>(kf, fin, tab, stage + qn * I::BYTES, ahead, segs, lane);
+            copies_commit();
             LatticeItem<T> x;
-            item_load<T, C>(x, kf, a, pr, fin, it, segs, lane);
+            item_nodes<T, C>(x, kf, a, pr, it, segs, lane);
+            copies_wait<I::STAGES - 1>();
+            __syncwarp();
+            item_read<T>(x, stage + q * I::BYTES, lane);
+            __syncwarp();
             item_update<T, C, CONS0>(x, kf, fout, fl);
+            q = q + 1 == I::STAGES ? 0 : q + 1;
         }
         // the update of the prepared tile; what its forces need is kept
         auto update = [&]() {
@@ -598,7 +672,9 @@ size_t loop_smem(const lbm_handle *h)
 {
     const size_t nb = (size_t)(h->nseg + BS - 1) / BS;
     const size_t solve = sizeof(double) * (nb * BS * GW + 2 * nb * BS) + 16;
-    return std::max(solve, NT / TILE_THREADS * sizeof(GroupSmem));
+    const size_t stages = h->elem == 2 ? Items<__half>::STAGES * Items<__half>::BYTES
+                          : h->elem == 4 ? Items<float>::STAGES * Items<float>::BYTES : Items<double>::STAGES * Items<double>::BYTES;
+    return std::max(solve, NT / TILE_THREADS * sizeof(GroupSmem) + NT / 32 * stages);
 }
 
 // CTAs beside the solver that a case's lattice can use: one group's threads
