@@ -24,8 +24,8 @@
 // chain, and what it does not need (the forces of a tile) is left for after.
 //
 // Measured on a B200, us a step, launches per stage -> here: 96x64 27.9 ->
-// 8.0; 400x200 33.5 -> 9.5 (FP64 31.7 -> 11.2); 1001x501 with two wings
-// 42 -> 13.4; 1280x640 42 -> 15.4; 2048x1024 in BF16 46 -> 25.3, of which
+// 8.1; 400x200 33.5 -> 9.3 (FP64 31.7 -> 10.9); 1001x501 with two wings
+// 42 -> 13.2; 1280x640 42 -> 13.6; 2048x1024 in BF16 46 -> 25.4, of which
 // 20 are the lattice (with its loads through registers 24).
 // On large lattices the staged kernel is the better one (loop_fits).
 //
@@ -49,6 +49,13 @@ constexpr int LOOP_STEPS = LBM_NSLOT_MAX / 2;   // steps of one launch at most (
 enum { SYNC_STEP = 0, SYNC_ABORT = 32, SYNC_WORDS = 64 };
 constexpr int LOOP_SMEM = 232448 - 1024;        // dynamic shared memory a CTA may use
 
+// Shares of the interior items (measured on 1280x640, 131 CTAs of which some 24
+// have a tile and each CTA some 97 items; us a step): items dealt out evenly
+// 15.4; a CTA with a tile 24, 36, 48 less 14.6, 15.0, 15.1; besides, all items
+// taken as the warps come 13.9, 13.5, 13.6; the last 2 or 4 a warp (36 less)
+// 13.6, 14.1. On 2048x1024 in BF16 (248 items a CTA) taking all costs more
+// than it saves: 25.3, 25.6 (24 less), 25.9 (all taken), 25.4 (the last 2).
+constexpr int LEAN = 36, TAIL = 2;
 constexpr int NT = 512;                         // threads of a CTA (at 1024 the 64 registers left to each spill)
 
 template <typename C> struct LoopArgs {
@@ -453,7 +460,7 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
         solver_cta<C>(L, smem);
         return;
     }
-    __shared__ int good[NG];
+    __shared__ int good[NG], taken[2];   // taken: the interior items of the step (by parity)
     const int cta = me - 1, G = all - 1;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int grp = tid / TILE_THREADS, gt = tid % TILE_THREADS;
@@ -468,6 +475,7 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
     unsigned char *stage = reinterpret_cast<unsigned char *>(smem) + NG * sizeof(GroupSmem) + warp * I::STAGES * I::BYTES;
     __shared__ int tab[I::ROW];
     item_table<T>(tab, (int)kf.plane, kf.pitch);
+    if (tid < 2) taken[tid] = 0;
     __syncthreads();
     const int n = L.ib.nseg, nx = kf.nx, ny = kf.ny;
     constexpr bool XPAIR = sizeof(T) == 2, YPAIR = sizeof(T) == 4;
@@ -545,6 +553,7 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
         T *fout = (T *)L.f[(s & 1) ^ 1];
         C *fl = L.fields[s];
         const bool duty = (s & 1) == grp;
+        if (tid == 0) taken[(s & 1) ^ 1] = 0;   // nobody takes of it before the next step
         for (int k = k0; k < n; k += NW * mctas) {
             if (k > k0) il = interp_lane(a, k, lane);
             double ru, rv;
@@ -559,24 +568,51 @@ __global__ void __launch_bounds__(NT, 1) step_loop(const __grid_constant__ LoopA
         const PatchInfo pr = *a.pinfo;
         const int et = duty ? TILE_THREADS + gt : gt;   // thread of the CTA, the free group first
         for (int e = (TILE_THREADS - 1 - et + (duty ? NT : 0)) * G + cta; e < nedge; e += nthr) edge_node<T, C>(kf, fin, fout, fl, e);
-        int it = (et >> 5) * G + cta;
+        // The CTA's interior items (`mine`): a CTA with a tile in this step has
+        // LEAN less than the others, none on a small lattice. The first `dealt`
+        // of them are dealt out to the warps; the last (TAIL a warp) go to the
+        // warps as they come, since a group that was still preparing a tile
+        // when the step began is behind.
+        const int nn = G - min(ntile, G);   // CTAs without a tile, the first ones
+        const int each = nn > 0 ? max(0, (items - LEAN * nn) / G) : (items + G - 1) / G;
+        const int mine = cta < nn ? each + (items - each * G - cta + nn - 1) / nn : each;
+        const int dealt = mine > NW ? max(0, mine / NW - TAIL) * NW : mine;
+        int turn = et >> 5;   // the free group first
+        auto take = [&]() -> int {
+            int q = turn;
+            if (q < dealt) {
+                turn += NW;
+            } else {
+                if (mine > NW) {
+                    if (lane == 0) q = atomicAdd(&taken[s & 1], 1);
+                    q = dealt + __shfl_sync(0xffffffffu, q, 0);
+                }
+                if (q >= mine) return items;
+            }
+            return q < each ? q * G + cta : each * G + (q - each) * nn + cta;
+        };
+        int it[I::STAGES];
 #pragma unroll
         for (int t = 0; t < I::STAGES - 1; ++t) {
-            if (it + t * NW * G < items) item_issue<T, C>(kf, fin, tab, stage + t * I::BYTES, it + t * NW * G, segs, lane);
+            it[t] = take();
+            if (it[t] < items) item_issue<T, C>(kf, fin, tab, stage + t * I::BYTES, it[t], segs, lane);
             copies_commit();
         }
-        for (int q = 0; it < items; it += NW * G) {
-            const int qn = q == 0 ? I::STAGES - 1 : q - 1, ahead = it + (I::STAGES - 1) * NW * G;
-            if (ahead < items) item_issue<T, C>(kf, fin, tab, stage + qn * I::BYTES, ahead, segs, lane);
+        for (int q = 0; it[0] < items;) {
+            const int qn = q == 0 ? I::STAGES - 1 : q - 1;
+            it[I::STAGES - 1] = take();
+            if (it[I::STAGES - 1] < items) item_issue<T, C>(kf, fin, tab, stage + qn * I::BYTES, it[I::STAGES - 1], segs, lane);
             copies_commit();
             LatticeItem<T> x;
-            item_nodes<T, C>(x, kf, a, pr, it, segs, lane);
+            item_nodes<T, C>(x, kf, a, pr, it[0], segs, lane);
             copies_wait<I::STAGES - 1>();
             __syncwarp();
             item_read<T>(x, stage + q * I::BYTES, lane);
             __syncwarp();
             item_update<T, C, CONS0>(x, kf, fout, fl);
             q = q + 1 == I::STAGES ? 0 : q + 1;
+#pragma unroll
+            for (int t = 0; t < I::STAGES - 1; ++t) it[t] = it[t + 1];
         }
         // the update of the prepared tile; what its forces need is kept
         auto update = [&]() {
