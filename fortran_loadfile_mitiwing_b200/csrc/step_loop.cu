@@ -795,12 +795,12 @@ cudaError_t loop_reset(lbm_handle *h)
 bool loop_fits(const lbm_handle *h)
 {
     if (h->loop_ctas < 2 || h->nseg <= 0 || h->nslots / 2 > LOOP_STEPS || loop_smem(h) > LOOP_SMEM) return false;
-    // the loop's lattice update moves at most some 5 TB/s and 3 nodes a step
-    // and clock, the staged kernel more: 2400x1200 in FP32 (210 MB) 62 us a step
-    // here and 68 there, 2800x1400 (282 MB) 81 and 78; FP64 1600x800 (184 MB) 51
-    // and 61, 2048x1024 (302 MB) 87 and 79; 2800x1400 in FP16, bound by the
-    // nodes and not by their 141 MB, 58 and 59
-    return loop_bytes(h) <= 220000000ll;
+    // Beyond these two steps in one pass (kf_pair) are faster, in FP64 earlier
+    // (the loop's lattice update is then bound by the FP64 units and the L2).
+    // us a step, here and there: FP32 2048x1024 (151 MB) 32 and 39, 2400x1200
+    // (207 MB) 41 and 42; FP16 2048x1024 26 and 37; FP64 1200x600 (104 MB) 27
+    // and 34, 1400x700 (141 MB) 37.5 and 34.6, 1600x800 (184 MB) 47 and 39.
+    return loop_bytes(h) <= (h->elem == 8 ? 125000000ll : 220000000ll);
 }
 
 // `nsteps` steps from step h->n on (within one slot half), step s with its

@@ -78,7 +78,7 @@ def patch_extent(case):
 
 def _pairs(elem, pitch, nx, ny, ns):
     """Whether the library steps such a case two steps at a time (pairs_fit)."""
-    loop = ns <= 576 and 18 * max(4, elem) * pitch * ny <= 220_000_000
+    loop = ns <= 576 and 18 * max(4, elem) * pitch * ny <= (125_000_000 if elem == 8 else 220_000_000)
     return not loop and nx >= 64 and ny >= 64 and 18 * elem * pitch * ny >= 40_000_000
 
 
