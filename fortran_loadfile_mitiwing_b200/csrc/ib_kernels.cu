@@ -12,8 +12,8 @@
 // The marker positions follow the prescribed motion, so D D^T and its
 // factorization depend on the step index only, not on the flow. The
 // launches are therefore two chains. The factorization chain of a step
-// (which the host runs one step ahead, concurrently with the previous step,
-// into one of two buffer slots):
+// (which the host runs a batch of steps ahead, beside the steps of the batch
+// before, into the slots of the other half):
 //   ib_geometry one thread per marker: position, boundary velocity, support
 //               box and one-axis kernel values (move_boundary, :1540-1606);
 //   ib_order    (several bodies only) one CTA sorts the markers along the
@@ -38,9 +38,10 @@
 //   ib_interp   one warp per marker: b = D u* over the support box and
 //               rhs = U_b - b (:1609-1629);
 //   ib_solve    one CTA: the forward and backward sweeps of the reduction
-//               over the two right-hand sides, each level's factor blocks
-//               staged in shared memory by bulk copies (or the two triangular
-//               solves of the dense factor), and the force row's header;
+//               over the two right-hand sides, the factor blocks of the
+//               levels above the first in shared memory, down to the odd
+//               blocks of the first level, which the tiles that need them
+//               solve (or the two triangular solves of the dense factor);
 //   ib_tile_update  one CTA per correction tile (a 16 x 16 tile of the
 //               patch rectangle that lists a marker): du = D^T y per node,
 //               gathered in marker order (no atomics), the lattice update of

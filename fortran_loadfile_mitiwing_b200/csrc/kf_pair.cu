@@ -5,12 +5,12 @@
 // nothing but the populations before them, so one CTA takes a node's
 // neighbourhood through both: it stages the rows of its strip as the
 // single-step kernel does, keeps the first step's results on chip (its own
-// column's in registers, the neighbour columns' through shared memory), and
-// writes only the second step's. The traffic per step is halved; the
-// arithmetic grows by the two rows and two columns around a CTA's nodes that
-// it computes for the first step only. 4096x2048, us a step, single-step
-// kernel alone -> here: FP32 104 -> 58, FP16 60 -> 47, FP64 195 -> 108; both
-// 4-byte and 2-byte forms are then bound by instruction issue.
+// column's in registers, the neighbour columns' by shuffles), and writes only
+// the second step's. The traffic per step is halved; the arithmetic grows by
+// the two rows around a CTA's nodes and the two columns around a warp's that
+// are computed for the first step only. 4096x2048, us a step, single-step
+// kernel alone -> here: FP32 104 -> 54 (85 % of the copy bandwidth), FP16
+// 60 -> 45, FP64 195 -> 104; the 2-byte form is bound by instruction issue.
 //
 // The nodes near a body go step by step: the first step's correction tiles
 // and the nodes next to them depend on the first step's solve, the second
@@ -33,10 +33,9 @@ constexpr int PT = 256;      // threads of a CTA
 constexpr int CELL = 16;     // nodes of a cell's side
 constexpr int FRAME = 2;     // nodes at the lattice's edge that kf_pair leaves (their second step needs the edge's first)
 
-// rows of a strip staged ahead. With 3 instead of 4 rows of FP32 four CTAs fit
-// on an SM instead of three: 128 -> 117 us a pair of steps on 4096x2048
-// (2: 122); FP16 no different, FP64 (two CTAs) 217 -> 220.
-template <typename T> __host__ __device__ constexpr int pair_stages() { return sizeof(T) == 8 ? 4 : 3; }
+// rows of a strip staged ahead (4096x2048, us a step with 3, 4, 5: FP32 73.4,
+// 72.0, 72.2, FP16 62.0, 60.9, 60.2: beyond 3 no more than the runs differ)
+template <typename T> __host__ __device__ constexpr int pair_stages() { return 4; }
 
 template <typename C> struct PairArgs {
     const void *fin;
@@ -50,19 +49,27 @@ template <typename C> struct PairArgs {
     unsigned *status;
 };
 
-// columns whose first step a CTA computes, and those of them it writes
-// (all but one, or with 2-byte storage one pair, at each side)
-template <typename T> __host__ __device__ constexpr int pair_cols() { return sizeof(T) == 2 ? 2 * PT : PT; }
-template <typename T> __host__ __device__ constexpr int pair_out() { return sizeof(T) == 2 ? 2 * PT - 4 : PT - 2; }
+// Columns that a CTA writes: 30 (2-byte storage: 30 pairs) of each warp. A
+// warp computes the first step of one more on either side and gets the
+// neighbours' first-step values by shuffles, so that the warps need no barrier
+// among them in the row loop. (With 254 columns a CTA, the neighbours' values
+// through shared memory and a barrier per row pair, the barrier was 40 % of
+// the stalls; 4096x2048, us a pair of steps alone, then -> now: FP32 123 ->
+// 109, FP16 100 -> 89.)
+constexpr int WOUT = 30;
+template <typename T> __host__ __device__ constexpr int pair_out() { return (sizeof(T) == 2 ? 2 : 1) * WOUT * (PT / 32); }
+// columns of the first step
+template <typename T> __host__ __device__ constexpr int pair_cols() { return pair_out<T>() + (sizeof(T) == 2 ? 4 : 2); }
 template <typename T> __host__ __device__ constexpr int pair_align() { return 16 / (int)sizeof(T); }
 // elements of a staged row segment: the columns, one or two more at each side,
 // from a 16-byte boundary on
-template <typename T> __host__ __device__ constexpr int pair_seg() { return pair_cols<T>() + 2 * pair_align<T>(); }
-// a row's neighbour values of one iteration: six planes, as pairs
-template <typename T> __host__ __device__ constexpr int pair_xch() { return sizeof(T) == 4 ? 8 : (sizeof(T) == 2 ? 4 : 8); }
+template <typename T> __host__ __device__ constexpr int pair_seg()
+{
+    return (pair_cols<T>() + pair_align<T>() - 1) / pair_align<T>() * pair_align<T>() + 2 * pair_align<T>();
+}
 template <typename T> __host__ __device__ constexpr size_t pair_smem()
 {
-    return sizeof(T) * pair_stages<T>() * 9 * pair_seg<T>() + 2 * 6 * PT * pair_xch<T>() + 2 * 8 * pair_stages<T>();
+    return sizeof(T) * pair_stages<T>() * 9 * pair_seg<T>() + 2 * 8 * pair_stages<T>();
 }
 
 // one node (or pair of nodes) of the first or second step
@@ -72,6 +79,12 @@ template <bool CONS0> __device__ __forceinline__ void pair_step(const KFArgs<flo
     collide_pair<CONS0, false>(a, g, o, r, u, v);
 }
 
+// the value of the warp's left, right neighbour column
+template <typename V> __device__ __forceinline__ V from_left(V v) { return __shfl_up_sync(0xffffffffu, v, 1); }
+template <typename V> __device__ __forceinline__ V from_right(V v) { return __shfl_down_sync(0xffffffffu, v, 1); }
+template <> __device__ __forceinline__ float2 from_left(float2 v) { return make_float2(from_left(v.x), from_left(v.y)); }
+template <> __device__ __forceinline__ float2 from_right(float2 v) { return make_float2(from_right(v.x), from_right(v.y)); }
+
 // One CTA: strip bx and row chunk by of the lattice described by p.
 template <typename T, typename C, bool CONS0>
 __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, unsigned char *sm)
@@ -79,14 +92,14 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
     constexpr int SEG = pair_seg<T>(), KS = pair_stages<T>(), NWARP = PT / 32, AL = pair_align<T>();
     constexpr bool XPAIR = sizeof(T) == 2, YPAIR = sizeof(T) == 4;
     T *buf = reinterpret_cast<T *>(sm);
-    unsigned char *xch = sm + sizeof(T) * KS * 9 * SEG;
-    uint64_t *full = reinterpret_cast<uint64_t *>(xch + 2 * 6 * PT * pair_xch<T>());
+    uint64_t *full = reinterpret_cast<uint64_t *>(sm + sizeof(T) * KS * 9 * SEG);
     uint64_t *empty = full + KS;
     const int tid = threadIdx.x, lane = tid & 31;
+    const int col = (tid >> 5) * WOUT + lane;      // of the first step (2-byte storage: pair of columns)
     // output columns from x0 on, first-step columns from x0 - 1 (x0 - 2) on
     const int x0 = FRAME + bx * pair_out<T>();
     const int xf = XPAIR ? x0 - 2 : x0 - 1;
-    const int i = xf + (XPAIR ? 2 * tid : tid);
+    const int i = xf + (XPAIR ? 2 * col : col);
     const int y0 = FRAME + by * p.rows;
     const int nout = min(p.rows, p.ny - 2 - y0);   // rows written: y0 .. y0 + nout - 1 <= ny - 3
     const int nrows = nout + 2;                    // first-step rows y0 - 1 ..
@@ -142,7 +155,7 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
         some = __syncthreads_or(some);
     }
     T *const fout = (T *)p.fout;
-    const bool out0 = tid > 0 && tid < PT - 1 && i <= p.nx - 3;
+    const bool out0 = lane > 0 && lane <= WOUT && i <= p.nx - 3;
     auto kept = [&](int ii, int j) { return some && p.near[(j >> 4) * p.cells_x + (ii >> 4)] != 0; };
     if constexpr (YPAIR) {
         float2 p0, p2, n1, n3, n5, n6;   // the iteration before: own column's planes 0, 2; neighbours' 1, 3, 5, 6
@@ -153,7 +166,7 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
             got = wait(&full[q1], (uint32_t)((r1 / KS) & 1)) && got;
             ok = ok && got;
             float2 g[9], o[9];
-            const T *b0 = buf + q0 * 9 * SEG + sh + tid, *b1 = buf + q1 * 9 * SEG + sh + tid;
+            const T *b0 = buf + q0 * 9 * SEG + sh + col, *b1 = buf + q1 * 9 * SEG + sh + col;
 #pragma unroll
             for (int k = 0; k < 9; ++k) g[k] = make_float2(b0[k * SEG - lbm_ex(k)], b1[k * SEG - lbm_ex(k)]);
             __syncwarp();
@@ -162,13 +175,11 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
                 if (r1 != r) mbar_arrive(&empty[q1]);
             }
             pair_step<CONS0>(a, g, o);
-            float2 *x = reinterpret_cast<float2 *>(xch) + ((r >> 1) & 1) * 6 * PT + tid;
-            x[0] = o[1]; x[PT] = o[3]; x[2 * PT] = o[5]; x[3 * PT] = o[6]; x[4 * PT] = o[7]; x[5 * PT] = o[8];
             refill(r);
             if (r1 != r) refill(r1);
-            if (__syncthreads_or(!ok)) break;
-            const int L = tid > 0 ? -1 : 0, R = tid < PT - 1 ? 1 : 0;
-            const float2 c1 = x[L], c3 = x[PT + R], c5 = x[2 * PT + L], c6 = x[3 * PT + R];
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const float2 c1 = from_left(o[1]), c3 = from_right(o[3]), c5 = from_left(o[5]), c6 = from_right(o[6]);
+            const float2 c7 = from_right(o[7]), c8 = from_left(o[8]);
             if (r > 0) {
                 // rows (y0 - 1 + r) - 1 and y0 - 1 + r
                 const int j = y0 - 2 + r;
@@ -179,8 +190,8 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
                 g[4] = o[4];
                 g[5] = n5;
                 g[6] = n6;
-                g[7] = x[4 * PT + R];
-                g[8] = x[5 * PT + L];
+                g[7] = c7;
+                g[8] = c8;
                 float2 w[9];
                 pair_step<CONS0>(a, g, w);
                 const bool s0 = out0 && !kept(i, j), s1 = out0 && j + 1 < y0 + nout && !kept(i, j + 1);
@@ -204,7 +215,7 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
             const int q = r % KS;
             ok = wait(&full[q], (uint32_t)((r / KS) & 1)) && ok;
             float2 g[9], o[9];
-            const uint32_t *b = reinterpret_cast<const uint32_t *>(buf + q * 9 * SEG + sh) + tid;
+            const uint32_t *b = reinterpret_cast<const uint32_t *>(buf + q * 9 * SEG + sh) + col;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
                 const uint32_t *wk = b + k * (SEG / 2);
@@ -220,13 +231,11 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
             uint32_t w[9];
 #pragma unroll
             for (int k = 0; k < 9; ++k) w[k] = Pair2<T>::pack(o[k]);
-            uint32_t *x = reinterpret_cast<uint32_t *>(xch) + (r & 1) * 6 * PT + tid;
-            x[0] = w[1]; x[PT] = w[3]; x[2 * PT] = w[5]; x[3 * PT] = w[6]; x[4 * PT] = w[7]; x[5 * PT] = w[8];
             refill(r);
-            if (__syncthreads_or(!ok)) break;
-            const int L = tid > 0 ? -1 : 0, R = tid < PT - 1 ? 1 : 0;
-            const uint32_t c1 = __byte_perm(x[L], w[1], 0x5432), c3 = __byte_perm(w[3], x[PT + R], 0x5432);
-            const uint32_t c5 = __byte_perm(x[2 * PT + L], w[5], 0x5432), c6 = __byte_perm(w[6], x[3 * PT + R], 0x5432);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const uint32_t c1 = __byte_perm(from_left(w[1]), w[1], 0x5432), c3 = __byte_perm(w[3], from_right(w[3]), 0x5432);
+            const uint32_t c5 = __byte_perm(from_left(w[5]), w[5], 0x5432), c6 = __byte_perm(w[6], from_right(w[6]), 0x5432);
+            const uint32_t c7 = __byte_perm(w[7], from_right(w[7]), 0x5432), c8 = __byte_perm(from_left(w[8]), w[8], 0x5432);
             if (r > 1) {
                 const int j = y0 - 2 + r;
                 g[0] = Pair2<T>::unpack(p0);
@@ -236,8 +245,8 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
                 g[4] = Pair2<T>::unpack(w[4]);
                 g[5] = Pair2<T>::unpack(q5b);
                 g[6] = Pair2<T>::unpack(q6b);
-                g[7] = Pair2<T>::unpack(__byte_perm(w[7], x[4 * PT + R], 0x5432));
-                g[8] = Pair2<T>::unpack(__byte_perm(x[5 * PT + L], w[8], 0x5432));
+                g[7] = Pair2<T>::unpack(c7);
+                g[8] = Pair2<T>::unpack(c8);
                 pair_step<CONS0>(a, g, o);
                 const bool s0 = out0 && !kept(i, j), s1 = s0 && i + 1 <= p.nx - 3;   // a pair lies in one cell
                 const unsigned at = (unsigned)(j * p.pitch + i);
@@ -258,23 +267,21 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
             const int q = r % KS;
             ok = wait(&full[q], (uint32_t)((r / KS) & 1)) && ok;
             C g[9], o[9], rho, u, v;
-            const T *b = buf + q * 9 * SEG + sh + tid;
+            const T *b = buf + q * 9 * SEG + sh + col;
 #pragma unroll
             for (int k = 0; k < 9; ++k) g[k] = b[k * SEG - lbm_ex(k)];
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty[q]);
             collide_interior<C, CONS0>(a, g, false, C(0), C(0), o, rho, u, v);
-            C *x = reinterpret_cast<C *>(xch) + (r & 1) * 6 * PT + tid;
-            x[0] = o[1]; x[PT] = o[3]; x[2 * PT] = o[5]; x[3 * PT] = o[6]; x[4 * PT] = o[7]; x[5 * PT] = o[8];
             refill(r);
-            if (__syncthreads_or(!ok)) break;
-            const int L = tid > 0 ? -1 : 0, R = tid < PT - 1 ? 1 : 0;
-            const C c1 = x[L], c3 = x[PT + R], c5 = x[2 * PT + L], c6 = x[3 * PT + R];
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const C c1 = from_left(o[1]), c3 = from_right(o[3]), c5 = from_left(o[5]), c6 = from_right(o[6]);
+            const C c7 = from_right(o[7]), c8 = from_left(o[8]);
             if (r > 1) {
                 const int j = y0 - 2 + r;
                 g[0] = p0; g[1] = q1; g[2] = p2b; g[3] = q3; g[4] = o[4]; g[5] = q5b; g[6] = q6b;
-                g[7] = x[4 * PT + R];
-                g[8] = x[5 * PT + L];
+                g[7] = c7;
+                g[8] = c8;
                 C w[9];
                 collide_interior<C, CONS0>(a, g, false, C(0), C(0), w, rho, u, v);
                 if (out0 && !kept(i, j)) {
@@ -298,7 +305,7 @@ __device__ __forceinline__ void pair_cta(const PairArgs<C> &p, int bx, int by, u
 }
 
 template <typename T, typename C, bool CONS0>
-__global__ void __launch_bounds__(PT, sizeof(T) == 8 ? 2 : 3) kf_pair(const __grid_constant__ PairArgs<C> p)
+__global__ void __launch_bounds__(PT, sizeof(T) == 8 ? 2 : 4) kf_pair(const __grid_constant__ PairArgs<C> p)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     pair_cta<T, C, CONS0>(p, blockIdx.x, blockIdx.y, sm);
@@ -487,14 +494,14 @@ int cells_of(const lbm_handle *h, int *cx, int *cy)
 // rows a CTA writes. Two more are computed by it for the first step only, so
 // the kernel alone is fastest with 16 to 20; but the immersed-boundary kernels
 // beside it start as its CTAs leave, and the step as a whole is faster with
-// shorter ones (4096x2048, us a step with 8, 10, 12, 14, 20 rows: FP32 77.7,
-// 76.9, 76.8, 78.1, 79.8; FP16 63.3, 63.0, 65.3, 64.9, 66.8; FP64 133.6,
-// 130.3, 129.3, 128.3, 127.5). Fewer where the lattice has not two waves of
-// such CTAs.
+// shorter ones (4096x2048, us a step with 8, 10, 12, 14, 20 rows: FP32 72.7,
+// 72.4, 72.6, 72.1, 75.0; FP16 62.1, 61.2, 60.8, 62.6, 62.1; FP64, by an
+// earlier form, 133.6, 130.3, 129.3, 128.3, 127.5). Fewer where the lattice
+// has not two waves of such CTAs.
 template <typename T> int pair_rows(const lbm_handle *h)
 {
     const int per_sm = sizeof(T) == 8 ? 2 : 4, strips = (h->nx - 2 * FRAME + pair_out<T>() - 1) / pair_out<T>();
-    int r = sizeof(T) == 2 ? 10 : (sizeof(T) == 4 ? 12 : 20);
+    int r = sizeof(T) == 8 ? 20 : 12;
     while (r > 8 && strips * ((h->ny - 2 * FRAME + r - 1) / r) < 2 * 148 * per_sm) r -= 2;
     return r;
 }

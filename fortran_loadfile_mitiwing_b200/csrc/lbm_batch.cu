@@ -65,9 +65,10 @@ struct lbm_batch {
     cudaStream_t main = nullptr, side = nullptr, fstream = nullptr;
     // the steps' force rows and residual checks run on their own stream,
     // after the step's correction tiles, so that the next step's flow chains
-    // need not wait for them (the cases keep what they read per step parity;
-    // ev_bcheck[p] marks the checks of the last step of parity p done). ev_side
-    // marks a step's flow chains and checks done.
+    // need not wait for them (the cases keep what they read per step slot;
+    // ev_bcheck[p] marks the checks of the last step of parity p done, and a
+    // step waits for those two back). ev_side marks a step's flow chains and
+    // checks done.
     cudaStream_t cstream = nullptr;
     cudaEvent_t ev_bcheck[2] = {nullptr, nullptr}, ev_cpre = nullptr;
     cudaEvent_t ev_ib = nullptr, ev_done = nullptr, ev_fready = nullptr, ev_side = nullptr;
@@ -1051,8 +1052,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             }
         }
         BCK(cudaEventRecord(b->ev_fready, b->side), "event");   // uploads done, factorizations ready
-        // the cases' buffers of this step's parity were last read by the
-        // checks two steps back
+        // the checks stay at most two steps behind
         BCK(cudaStreamWaitEvent(b->side, b->ev_bcheck[step & 1], 0), "wait");
         cudaEvent_t ei = b->after_interp ? b->ev_interp : nullptr;
         if (launch_flow_batch(act.data(), (int)act.size(), b->d_sargs[buf], b->d_kargs[buf], 0, pending, fields,
