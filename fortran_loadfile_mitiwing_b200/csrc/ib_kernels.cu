@@ -1057,11 +1057,10 @@ __device__ __forceinline__ void force_row(const IBArgs &a, int rr)
     }
 }
 
-template <bool BATCH>
-__global__ void __launch_bounds__(256) ib_forces(const IBArgs a0, const IBArgs *batch, int ring_slot)
+__global__ void __launch_bounds__(256) ib_forces(const IBArgs *batch)
 {
-    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
-    force_row(a, BATCH ? a.ring_row : ring_slot);
+    const IBArgs &a = batch[blockIdx.z];
+    force_row(a, a.ring_row);
 }
 
 // arguments of case z of a batch's loop launch (they begin its entry)
@@ -1070,31 +1069,23 @@ __device__ __forceinline__ const IBArgs &loop_case(const void *batch, size_t str
     return *reinterpret_cast<const IBArgs *>((const char *)batch + blockIdx.z * stride);
 }
 
-// the force rows of consecutive steps, headers included: CTA b the step b
-// after the arguments' (of slot 0), into the row b after theirs
-template <bool BATCH>
-__global__ void __launch_bounds__(256) ib_forces_steps(const IBArgs a0, const void *batch, size_t stride)
-{
-    const IBArgs &base = BATCH ? loop_case(batch, stride) : a0;
-    const int step = base.cur_step + (int)blockIdx.x, rr = base.ring_row + (int)blockIdx.x;
-    const IBArgs a = step_args(base, step);
-    force_row(a, rr);
-}
-
 // Residual of the step's solve, ||B y - rhs|| / ||rhs|| with B = D D^T
 // recomputed from the marker geometry (independent of the factorization):
 // one warp per row of the solve order, lanes over the couplings within the
 // half-bandwidth; deterministic two-level sum (CTA partials, last CTA).
 // Flags LBM_ST_SOLVER unless it is below 1e-6, or LBM_ST_NONFINITE when the
 // right-hand side itself is not finite (the flow at the markers diverged).
-__device__ __forceinline__ void solve_residual(const IBArgs &a)
+// The sums go behind the slot's tile partials, the counter to their end.
+__device__ __forceinline__ void solve_residual(const IBArgs &a, int blk)
 {
     __shared__ double red[8][2];
     __shared__ bool amlast;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int n = a.nseg, s = blockIdx.x * 8 + warp;
+    const int n = a.nseg, s = blk * 8 + warp;
     const int nblk = (n + 7) / 8;
-    if ((int)blockIdx.x >= nblk) return;    // batched launches size the grid for the largest case
+    double *partial = a.partial + (long long)NPART * patch_tiles(a);
+    unsigned *counter = reinterpret_cast<unsigned *>(a.partial + a.st_part - 1);
+    if (blk >= nblk) return;    // batched launches size the grid for the largest case
     const int hw = min(max((int)a.solve_res[1], 0), n);
     double rnum = 0.0, rden = 0.0;
     const int ks = s < n ? order_at(a, s, LBM_ST_INDEX_RESIDUAL) : -1;
@@ -1125,18 +1116,18 @@ __device__ __forceinline__ void solve_residual(const IBArgs &a)
     if (threadIdx.x == 0) {
         double t0 = 0, t1 = 0;
         for (int w = 0; w < 8; ++w) { t0 += red[w][0]; t1 += red[w][1]; }
-        a.partial[2 * blockIdx.x] = t0;
-        a.partial[2 * blockIdx.x + 1] = t1;
+        partial[2 * blk] = t0;
+        partial[2 * blk + 1] = t1;
         __threadfence();
-        amlast = atomicAdd(a.counter, 1u) == (unsigned)(nblk - 1);
+        amlast = atomicAdd(counter, 1u) == (unsigned)(nblk - 1);
     }
     __syncthreads();
     if (!amlast) return;
     __threadfence();
     double s0 = 0.0, s1 = 0.0;
     for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
-        s0 += __ldcg(a.partial + 2 * b);
-        s1 += __ldcg(a.partial + 2 * b + 1);
+        s0 += __ldcg(partial + 2 * b);
+        s1 += __ldcg(partial + 2 * b + 1);
     }
 #pragma unroll
     for (int off = 16; off; off >>= 1) {
@@ -1155,25 +1146,39 @@ __device__ __forceinline__ void solve_residual(const IBArgs &a)
             atomicOr(a.status, LBM_ST_NONFINITE);
         else if (!(res < 1e-6))
             atomicOr(a.status, LBM_ST_SOLVER);
-        *a.counter = 0u;
+        *counter = 0u;
     }
 }
 
-template <bool BATCH>
-__global__ void __launch_bounds__(256) ib_residual(const IBArgs a0, const IBArgs *batch)
+__global__ void __launch_bounds__(256) ib_residual(const IBArgs *batch)
 {
-    const IBArgs &a = BATCH ? batch[blockIdx.z] : a0;
-    if (BATCH && !a.check_res) return;   // this case's step is not checked
-    solve_residual(a);
+    const IBArgs &a = batch[blockIdx.z];
+    if (!a.check_res) return;   // this case's step is not checked
+    solve_residual(a, blockIdx.x);
 }
 
-// the step t after the loop launch's first; due for every case, or (if not)
-// for those whose last step it is
-__global__ void __launch_bounds__(256) ib_residual_steps(const void *batch, size_t stride, int t, bool due)
+// The force rows of `count` consecutive steps, headers included (CTA b: the
+// step b after the arguments', of slot 0, into the row b after theirs), and the
+// residual checks of the steps in `check` (bit t; `per` CTAs each), in one
+// launch: they need nothing of one another, and a call of one step waits for
+// both (us a call of one step, as kernels of their own and here: 400x200 48.5
+// and 47, 1280x640 55 and 48). With BATCH the steps
+// in `check` but not in `due` are the last ones of some cases (check_res).
+template <bool BATCH>
+__global__ void __launch_bounds__(256) ib_checks(const IBArgs a0, const void *batch, size_t stride, int count, unsigned check,
+                                                 unsigned due, int per)
 {
-    const IBArgs &base = loop_case(batch, stride);
-    if (!due && !base.check_res) return;
-    solve_residual(step_args(base, base.cur_step + t));
+    const IBArgs &base = BATCH ? loop_case(batch, stride) : a0;
+    const int b = blockIdx.x;
+    if (b < count) {
+        force_row(step_args(base, base.cur_step + b), base.ring_row + b);
+        return;
+    }
+    const int q = (b - count) / per, blk = (b - count) - q * per;
+    for (int k = 0; k < q; ++k) check &= check - 1;
+    const int t = __ffs((int)check) - 1;
+    if (t < 0 || t >= count || (BATCH && !((due >> t) & 1u) && !base.check_res)) return;
+    solve_residual(step_args(base, base.cur_step + t), blk);
 }
 
 // The correction tiles of the step (the 16 x 16 tiles of the patch
@@ -1366,7 +1371,7 @@ IBArgs make_args(lbm_handle *h, const void *fin, int slot)
     a.nsup = h->d_nsup + slot;
     a.ctile = h->d_ctile + slot * (a.st_tiles / (TILE_CAP + 1));
     a.patch_wmax = h->patch_wmax; a.patch_hmax = h->patch_hmax;
-    a.partial = h->d_partial + slot * a.st_part; a.counter = h->d_counter;
+    a.partial = h->d_partial + slot * a.st_part;
     a.force_ring = h->d_ring; a.row_len = h->row_len;
     a.ring_row = 0; a.ring_rows = h->ring_cap;
     a.status = h->d_status; a.solve_res = h->d_solve_res + 2 * slot;
@@ -1397,16 +1402,16 @@ int launch_flow_t(lbm_handle *h, const void *fin, void *fout, void *fields, int 
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// the residual check of the step's solve (needed by no later kernel of the step)
-template <typename T, typename C>
-int launch_check_t(lbm_handle *h, int slot, int ring_slot, bool residual, cudaStream_t st)
+// the force rows of `count` steps from step0 on and the residual checks of
+// those in `check`
+int launch_checks(lbm_handle *h, int step0, int count, int ring_slot, unsigned check, cudaStream_t st)
 {
-    IBArgs a = make_args(h, nullptr, slot);
-    ib_forces<false><<<1, 256, 0, st>>>(a, nullptr, ring_slot);
-    h->launches += 1;
-    if (h->nseg == 0 || !residual) return cudaGetLastError() == cudaSuccess ? 0 : -1;
-    ib_residual<false><<<(h->nseg + 7) / 8, 256, 0, st>>>(a, nullptr);
-    h->launches += 1;
+    IBArgs a = make_args(h, nullptr, 0);
+    a.cur_step = step0;
+    a.ring_row = ring_slot;
+    const int per = (h->nseg + 7) / 8, checks = per > 0 ? __builtin_popcount(check) : 0;
+    ib_checks<false><<<count + checks * per, 256, 0, st>>>(a, nullptr, 0, count, check, check, std::max(per, 1));
+    h->launches += count + checks;   // a force row of each step, a check
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1471,24 +1476,16 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st)
 
 int launch_check_steps(lbm_handle *h, int step0, int count, int ring_slot, bool last, cudaStream_t st)
 {
-    IBArgs a = make_args(h, nullptr, 0);
-    a.cur_step = step0;
-    a.ring_row = ring_slot;
-    ib_forces_steps<false><<<count, 256, 0, st>>>(a, nullptr, 0);
-    h->launches += count;   // a force row each
-    for (int t = 0; t < count; ++t) {
-        if (!check_due(step0 + t) && !(last && t == count - 1)) continue;
-        const IBArgs b = make_args(h, nullptr, (step0 + t) % h->nslots);
-        ib_residual<false><<<(h->nseg + 7) / 8, 256, 0, st>>>(b, nullptr);
-        h->launches += 1;
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : -1;
+    unsigned check = 0;
+    for (int t = 0; t < count; ++t)
+        if (check_due(step0 + t) || (last && t == count - 1)) check |= 1u << t;
+    return launch_checks(h, step0, count, ring_slot, check, st);
 }
 
-// force row and residual check of the step held in `slot`, after its flow chain
-int launch_check(lbm_handle *h, int slot, int ring_slot, bool residual, cudaStream_t st)
+// force row and residual check of one step, after its flow chain
+int launch_check(lbm_handle *h, int step, int ring_slot, bool residual, cudaStream_t st)
 {
-    return launch_check_t<float, float>(h, slot, ring_slot, residual, st ? st : h->stream);
+    return launch_checks(h, step, 1, ring_slot, residual ? 1u : 0u, st);
 }
 
 // flow chain of step `step_index`: interpolation, solve with the factor of
@@ -1616,10 +1613,10 @@ int launch_check_batch(lbm_handle *const *hs, int ncase, const void *dargs, int 
     if (ncase <= 0) return 0;
     const IBArgs *d = (const IBArgs *)dargs;
     const int ns = max_seg(hs, ncase);
-    ib_forces<true><<<dim3(1, 1, ncase), 256, 0, st>>>(IBArgs{}, d, ring_slot);
+    ib_forces<<<dim3(1, 1, ncase), 256, 0, st>>>(d);
     for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
     if (!residual) return cudaGetLastError() == cudaSuccess ? 0 : -1;   // no case checks this step
-    ib_residual<true><<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(IBArgs{}, d);
+    ib_residual<<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(d);
     for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -1628,13 +1625,9 @@ int launch_check_steps_batch(lbm_handle *const *hs, int ncase, const void *dargs
                              bool last, cudaStream_t st)
 {
     const int ns = max_seg(hs, ncase);
-    ib_forces_steps<true><<<dim3(count, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs, stride);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += count;
-    for (int t = 0; t < count; ++t) {
-        const bool d = (due >> t) & 1u;
-        if (!d && !(last && t == count - 1)) continue;
-        ib_residual_steps<<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(dargs, stride, t, d);
-        for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
-    }
+    const unsigned check = due | (last ? 1u << (count - 1) : 0u);
+    const int per = (ns + 7) / 8, checks = __builtin_popcount(check);
+    ib_checks<true><<<dim3(count + checks * per, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs, stride, count, check, due, per);
+    for (int c = 0; c < ncase; ++c) hs[c]->launches += count + checks;
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -312,9 +312,9 @@ int ensure_ib(lbm_handle *h)
     CK(cudaMemsetAsync(h->d_fmode, 0, S * 2 * sizeof(int), h->stream), "clear factor mode");
     CK(cudaMemsetAsync(h->d_fstatus, 0, S * sizeof(unsigned), h->stream), "clear factor status");
     const int nblk = h->patch_gx() * h->patch_gy();
-    // partials of the spread (per patch tile) and of the residual check (per 8
-    // markers), per slot
-    const size_t npart = std::max((size_t)ib_partials_per_block() * nblk, 2 * (size_t)((ns + 7) / 8));
+    // partials of the spread (per patch tile), of the residual check (per 8
+    // markers) and the check's counter, per slot
+    const size_t npart = (size_t)ib_partials_per_block() * nblk + 2 * (size_t)((ns + 7) / 8) + 1;
     h->part_stride = npart;
     CK(dmalloc(h, &h->d_partial, S * sizeof(double) * npart), "alloc partials");
     h->tiles_slot = (size_t)ib_tile_ints() * nblk;
@@ -675,7 +675,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
                 if (launch_flow(h, src, dst, nullptr, h->n, slot + t, q, h->side, t ? nullptr : ei)) return cuda_err(h, cudaGetLastError(), "launch ib");
                 CK(cudaEventRecord(h->ev_ib, h->side), "event");
                 CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
-                if (launch_check(h, q, slot + t, check_due(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
+                if (launch_check(h, h->n, slot + t, check_due(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
                 if (t == 0) {
                     if ((rc = factor_next(b, s))) return rc;
                     CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
@@ -732,7 +732,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             // the force row and the residual check on their own stream; the
             // slot half is free for the next factorization after them
             CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
-            if (launch_check(h, q, slot, check_res, h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
+            if (launch_check(h, h->n, slot, check_res, h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
             CK(cudaEventRecord(h->ev_free[half], h->cstream), "event");
             if ((rc = factor_next(b, s))) return rc;
             CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");   // the step's correction tiles
@@ -750,7 +750,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             if (e) CK(cudaEventRecord(e[0], h->stream), "event");
             if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
             if (launch_flow(h, fin, fout, fields, h->n, slot, q, h->stream)) return cuda_err(h, cudaGetLastError(), "launch ib");
-            if (launch_check(h, q, slot, check_res, h->stream)) return cuda_err(h, cudaGetLastError(), "launch check");
+            if (launch_check(h, h->n, slot, check_res, h->stream)) return cuda_err(h, cudaGetLastError(), "launch check");
             if (e) {
                 CK(cudaEventRecord(e[1], h->stream), "event");
                 CK(cudaEventRecord(e[2], h->stream), "event");
@@ -1009,7 +1009,6 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     for (int b = 0; b < 2; ++b)
         if ((e = dmalloc(h, &h->d_fields[b], 3 * cs * nn)) != cudaSuccess) return fail(e, "alloc fields");
     if ((e = dmalloc(h, &h->edge_c, cs * (6 * (size_t)h->ny + 36))) != cudaSuccess) return fail(e, "alloc edge");
-    if ((e = dmalloc(h, &h->d_counter, sizeof(unsigned))) != cudaSuccess) return fail(e, "alloc counter");
     if ((e = dmalloc(h, &h->d_pinfo, LBM_NSLOT_MAX * sizeof(PatchInfo))) != cudaSuccess) return fail(e, "alloc pinfo");
     if ((e = dmalloc(h, &h->d_red, sizeof(double) * 2 * 296)) != cudaSuccess) return fail(e, "alloc red");
     if ((e = dmalloc(h, &h->d_mass, sizeof(double) * mass_slots())) != cudaSuccess) return fail(e, "alloc mass");
@@ -1048,7 +1047,7 @@ int lbm_destroy(lbm_t *h)
     free_dev(h->edge_c);
     free_devp(h->d_xb0); free_devp(h->d_yb0); free_devp(h->d_arc); free_devp(h->d_mstep);
     free_ib(h);
-    free_devp(h->d_pinfo); free_devp(h->d_counter);
+    free_devp(h->d_pinfo); 
     free_devp(h->d_head); free_devp(h->d_solve_res);
     host_block_free(h->hblock);
     free_devp(h->d_red);

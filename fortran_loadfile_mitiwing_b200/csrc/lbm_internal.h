@@ -90,7 +90,6 @@ struct IBArgs {
     int *nsup;          // number of correction tiles (tiles listing a marker) of the slot's step
     int *ctile;         // their tile indices, in no particular order
     double *partial;    // per-block force partials
-    unsigned *counter;  // last-block counter
     double *force_ring; // [ring_cap][row_len]
     int row_len;
     // batched launches: the force-ring row of this case's step (the rows
@@ -215,7 +214,6 @@ struct lbm_handle {
     cudaEvent_t ev_near[2] = {nullptr, nullptr};
     unsigned sync_base = 0;   // their step counter after the launches so far
     double *d_partial = nullptr;
-    unsigned *d_counter = nullptr;
     RunHead *d_head = nullptr;   // allocation of the head and the force ring
     double *d_ring = nullptr;    // behind it
     void *hblock = nullptr;      // kHostBlock bytes of pinned memory
@@ -262,7 +260,7 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st);
 // after_interp (nullable): recorded on st once the interpolation is done
 int launch_flow(lbm_handle *h, const void *fin, void *fout, void *fields, int step_index, int ring_slot, int slot,
                 cudaStream_t st, cudaEvent_t after_interp = nullptr);
-int launch_check(lbm_handle *h, int slot, int ring_slot, bool residual, cudaStream_t st);
+int launch_check(lbm_handle *h, int step, int ring_slot, bool residual, cudaStream_t st);
 // force rows (headers included) and residual checks of the `count` steps from
 // step0 on, after their step_loop launch; a step is checked as check_due says,
 // and the last one if `last`

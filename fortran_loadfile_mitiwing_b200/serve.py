@@ -98,7 +98,7 @@ def estimate_device_bytes(case):
     total = 2 * elem * (9 * pitch * ny + 2 * _FPAD)          # populations, two buffers
     total += 2 * 3 * cs * nx * ny                              # fields, two slots
     total += cs * (6 * ny + 36)                                # edge values
-    total += 16 + 4 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 16 * _NSLOT_MAX + 4 * 64 + 8 * row_len * _RING
+    total += 16 + _NSLOT_MAX * _PATCHINFO_BYTES + 8 * 2 * 296 + 16 * _NSLOT_MAX + 4 * 64 + 8 * row_len * _RING
     total += 8 * _MASS_BLOCKS + 4                        # mass check: partials and sum, counter
     if nwing:
         dt = p.scale * p.uu
@@ -112,7 +112,7 @@ def estimate_device_bytes(case):
         # right-hand sides, solution and tile partials: one set per slot
         total += S * _MARKER_BYTES * ns + S * 2 * 8 * 2 * ns + S * 8 * ns * ns
         total += 2 * K * 8 * nb * _BS * _BS + S * 8 * nb * _BS * _GW + S * 2 * 4 + S * 4
-        total += S * 8 * max(_NPART * nblk, 2 * ((ns + 7) // 8))
+        total += S * 8 * (_NPART * nblk + 2 * ((ns + 7) // 8) + 1)
         total += S * 4 * _TILE_INTS * nblk + S * 4 + S * 4 * nblk
         total += S * 4 * ns + S * 8 * ns + 8 + K * 4
         if _pairs(elem, pitch, nx, ny, ns):                    # two steps at a time: state between, near cells

@@ -19,6 +19,10 @@ SHAPES = {
     "odd": (1301, 655, 290, (511, 329), 580, 1, dict(pitch_deg=25.0)),
     "strip": (1274, 701, 300, (499, 350), 600, 1, dict(heave=0.3, delta=LBM_DELTA_SMOOTH)),
     "wings": (1403, 603, 160, (400, 301), 310, 2, {}),
+    "full": (1204, 640, 290, (500, 321), 580, 1, {}),   # strips of 240 (480) columns without a remainder, with one of a column
+    "one": (1205, 641, 290, (500, 321), 580, 1, {}),
+    "full2": (1924, 640, 290, (500, 321), 580, 1, {}),
+    "one2": (1925, 641, 290, (500, 321), 580, 1, {}),
     "wide": (2051, 1031, 300, (700, 515), 590, 1, dict(pitch_deg=20.0)),
     "edge": (1283, 641, 290, (82, 28), 580, 1, dict(heave=0.005, pitch_deg=0.0)),   # cells at the left and lower edge
 }
@@ -39,7 +43,8 @@ def same(alone, member, rows_a, rows_b):
 
 @pytest.mark.parametrize("name,precision", [("even", "fp32"), ("odd", "fp32"), ("strip", "fp32"), ("wings", "fp32"),
                                             ("edge", "fp32"), ("odd", "fp64"), ("strip", "fp64"), ("wide", "fp16"),
-                                            ("wide", "bf16")])
+                                            ("wide", "bf16"), ("full", "fp32"), ("one", "fp32"), ("one", "fp64"),
+                                            ("full2", "fp16"), ("one2", "bf16")])
 def test_pairs_equal_single_steps(gpu_lib, name, precision):
     alone, member = make(name, precision, gpu_lib), make(name, precision, gpu_lib)
     held = alone.device_bytes()
