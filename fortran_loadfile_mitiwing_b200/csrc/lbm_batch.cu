@@ -236,7 +236,10 @@ int reserve(lbm_batch *b, int ncase, int ntab)
 {
     if (ncase <= b->cap && ntab <= b->table_cap) return LBM_OK;
     sync_streams(b);
-    const int nc = std::max(ncase, b->cap), nt = std::max(ntab, b->table_cap);
+    // half as much again, so that adding cases one by one (lbm_batch_create
+    // does) allocates the some 60 arrays a few times and not once a case
+    const int nc = ncase <= b->cap ? b->cap : std::max(ncase, b->cap + b->cap / 2 + 8);
+    const int nt = ntab <= b->table_cap ? b->table_cap : std::max(ntab, b->table_cap + b->table_cap / 2);
     free_arrays(b);
     for (int q = 0; q < kArgRing; ++q) {
         BCK(cudaMalloc(&b->d_sargs[q], nc * b->ib_sz), "alloc");
