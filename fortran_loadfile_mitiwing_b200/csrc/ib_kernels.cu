@@ -49,8 +49,9 @@
 //               moment sums (:1645-1675, solution.f90:327-336) in FP64 with a
 //               deterministic two-level reduction. The lattice kernel skips
 //               these nodes and updates all others;
-//   ib_forces   the force row from the tiles' partials, and
-//   ib_residual the solve's residual, both after the step's update.
+//   ib_checks   the force row from the tiles' partials and the solve's
+//               residual, after the step's update (ib_forces and ib_residual
+//               in batches that run stage by stage).
 
 #include <math.h>
 
@@ -1162,8 +1163,8 @@ __global__ void __launch_bounds__(256) ib_residual(const IBArgs *batch)
 // residual checks of the steps in `check` (bit t; `per` CTAs each), in one
 // launch: they need nothing of one another, and a call of one step waits for
 // both (us a call of one step, as kernels of their own and here: 400x200 48.5
-// and 47, 1280x640 55 and 48). With BATCH the steps
-// in `check` but not in `due` are the last ones of some cases (check_res).
+// and 47, 1280x640 55 and 48). With BATCH the steps in `check` but not in `due`
+// are the last ones of some cases (check_res).
 template <bool BATCH>
 __global__ void __launch_bounds__(256) ib_checks(const IBArgs a0, const void *batch, size_t stride, int count, unsigned check,
                                                  unsigned due, int per)

@@ -1,12 +1,12 @@
-"""Small lattices run several steps per launch (csrc/step_loop.cu); batches
-run one launch per stage. Both call the same node, marker and tile functions
-in the same order, so a case alone must give exactly what it gives in a batch
-of one: force rows, populations and fields, bit for bit. The cases are where
+"""Small lattices run several steps per launch (csrc/step_loop.cu), alone and in
+batches; with per-kernel timing on, a case runs one launch per stage. All call
+the same node, marker and tile functions in the same order, so they must give
+the same force rows, populations and fields, bit for bit. The cases are where
 the loop's work division can go wrong: odd sizes (a last row pair or column
 pair with one node), sizes at and beside a warp's and a row pair's width, one
 and two wings, marker counts around the 16-marker blocks and at the largest
 count one launch's solver holds (576; the next one runs kernel by kernel),
-and step counts around the 8 steps of a launch."""
+and step counts around the 16 steps of a launch."""
 import numpy as np
 import pytest
 
@@ -14,6 +14,7 @@ from fortran_loadfile_mitiwing_b200 import Batch, Lbm, cases
 from fortran_loadfile_mitiwing_b200._abi import LBM_DELTA_SMOOTH
 
 pytestmark = pytest.mark.gpu
+LBM_TIMING_KERNELS = 1
 
 SHAPES = [
     # nx, ny, chord, pivot, markers, wings, kwargs
@@ -46,14 +47,17 @@ def same(alone, member, rows_a, rows_b, fields=True):
 @pytest.mark.parametrize("precision", ["fp32", "fp64", "fp16", "bf16"])
 @pytest.mark.parametrize("shape", SHAPES, ids=lambda s: f"{s[0]}x{s[1]}-{s[4]}x{s[5]}")
 def test_loop_equals_kernel_by_kernel(gpu_lib, shape, precision):
-    alone, member = make(shape, precision, gpu_lib), make(shape, precision, gpu_lib)
+    alone, member, staged = (make(shape, precision, gpu_lib) for _ in range(3))
     with Batch([member]) as b:
         b.set_graphs(False)
         rows_b = b.run(21)[0]
-    same(alone, member, alone.run(21), rows_b)
+    assert gpu_lib.lbm_set_timing(staged.h, LBM_TIMING_KERNELS) == 0
+    rows = alone.run(21)
+    same(alone, member, rows, rows_b)
+    same(alone, staged, rows, staged.run(21))
 
 
-@pytest.mark.parametrize("chunks", [(1, 1, 1), (7, 8, 9), (2, 16, 3), (8, 8, 5)], ids=str)
+@pytest.mark.parametrize("chunks", [(1, 1, 1), (7, 8, 9), (2, 16, 3), (8, 8, 5), (15, 16, 17), (33, 14)], ids=str)
 def test_call_lengths(gpu_lib, chunks):
     alone, member = make(SHAPES[1], "fp32", gpu_lib), make(SHAPES[1], "fp32", gpu_lib)
     rows = np.concatenate([alone.run(k) for k in chunks] + [alone.evolution()[None]])
