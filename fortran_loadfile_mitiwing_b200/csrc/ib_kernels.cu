@@ -79,10 +79,15 @@ constexpr int SOLVE_SMEM_BUDGET = LBM_SOLVE_SMEM;   // dynamic shared memory of 
 // those from st0 on (the blocks that are multiples of st0, at index o / st0).
 // Level 1's are read once, in the forward sweep, and stay in L2, so that a
 // solve of 512 markers takes half an SM's shared memory.
+// shared memory of a solve of nb blocks that keeps the levels from st on
+__host__ __device__ constexpr int solve_bytes(int nb, int st)
+{
+    return ((nb + st - 1) / st * BS * GW + 2 * nb * BS) * (int)sizeof(double) + 16;
+}
 __host__ __device__ constexpr int solve_st0(int nb)
 {
     int st = 2;
-    while (((nb + st - 1) / st * BS * GW + 2 * nb * BS) * (int)sizeof(double) + 16 > SOLVE_SMEM_BUDGET) st *= 2;
+    while (solve_bytes(nb, st) > SOLVE_SMEM_BUDGET) st *= 2;
     return st;
 }
 constexpr int WS = BS * GP + BS * FL + BS * GP;   // workspace per warp (doubles)
@@ -762,6 +767,14 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) ib_solve(const IBArgs a0, co
     const int nb = (n + BS - 1) / BS, st0 = solve_st0(nb), nres = (nb + st0 - 1) / st0;
     double *stage = smem, *X = smem + nres * BS * GW;
     uint64_t *bar = reinterpret_cast<uint64_t *>(X + 2 * nb * BS);
+    if (BATCH) {   // a launch for several cases has room for each of them (launch_flow_batch_t)
+        uint32_t have;
+        asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(have));
+        if (solve_bytes(nb, st0) > (int)have) {
+            if (tid == 0) atomicOr(a.status, LBM_ST_INDEX_SOLVE);
+            return;
+        }
+    }
     if (tid == 0) {
         mbar_init(bar, 1);
         mbar_init_fence();
@@ -1311,8 +1324,17 @@ constexpr size_t kSolveSmemMax = SOLVE_SMEM_BUDGET;
 size_t solve_smem(int nseg)
 {
     const int nb = (nseg + BS - 1) / BS;
-    const int st0 = solve_st0(nb);
-    return sizeof(double) * ((size_t)((nb + st0 - 1) / st0) * BS * GW + 2 * (size_t)nb * BS) + 16;
+    return (size_t)solve_bytes(nb, solve_st0(nb));
+}
+
+// Of a launch for several cases: the largest need among them, which is not
+// that of the most markers (68 blocks keep every level above the first and
+// take 226,320 bytes, 69 blocks every second one of those and 128,272).
+size_t solve_smem(lbm_handle *const *hs, int n)
+{
+    size_t m = 0;
+    for (int c = 0; c < n; ++c) m = std::max(m, solve_smem(hs[c]->nseg));
+    return m;
 }
 
 // threads of the solve's CTA: one warp per even block of the first level
@@ -1542,7 +1564,7 @@ int launch_flow_batch_t(lbm_handle *const *hs, int ncase, const IBArgs *dargs, c
     const int ns = max_seg(hs, ncase);
     ib_interp<T, true><<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs);
     if (after_interp && cudaEventRecord(after_interp, st) != cudaSuccess) return -1;
-    ib_solve<true><<<dim3(1, 1, ncase), solve_threads(ns), solve_smem(ns), st>>>(IBArgs{}, dargs);
+    ib_solve<true><<<dim3(1, 1, ncase), solve_threads(ns), solve_smem(hs, ncase), st>>>(IBArgs{}, dargs);
     // CTAs per case, strided over the case's correction tiles: the patch
     // grids bound the tiles several times over (a sweep case of chord 256
     // has some 60 correction tiles in a grid of hundreds), and CTAs past a
