@@ -236,7 +236,7 @@ void free_ib(lbm_handle *h)
     if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->ib_ready = 0;
-    h->batch_in_half[0] = h->batch_in_half[1] = -1;
+    forget_batches(h);
     free_devp(h->d_mk); free_devp(h->d_rhs); free_devp(h->d_B); free_devp(h->d_y); free_devp(h->d_partial);
     free_devp(h->d_bD); free_devp(h->d_bL); free_devp(h->d_gf); free_devp(h->d_fmode); free_devp(h->d_fstatus); free_devp(h->d_tiles); free_devp(h->d_nsup); free_devp(h->d_ctile);
     free_dev(h->fmid_alloc); h->fmid = nullptr; h->pairs = 0;
@@ -559,8 +559,25 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             CK(cudaStreamWaitEvent(h->fstream, h->ev_inner, 0), "wait");
         }
         if (launch_factor(h, s0, s1 - s0 + 1, st)) return cuda_err(h, cudaGetLastError(), "launch factor");
-        if (h->pairs && launch_near_cells(h, s0, s1 - s0 + 1, st)) return cuda_err(h, cudaGetLastError(), "launch near cells");
+        if (h->pairs) {
+            if (launch_near_cells(h, s0, s1 - s0 + 1, st)) return cuda_err(h, cudaGetLastError(), "launch near cells");
+            h->near_in_half[half] = b;
+        }
         if (split) CK(cudaEventRecord(h->ev_batch[half], h->fstream), "event");
+        return LBM_OK;
+    };
+    // The near cells of batch b where its half was factorized without them, by
+    // an lbm_batch (whose run has ended: nothing of its is queued). They
+    // replace those of the batch two back, which the factor stream waits for
+    // as factor_batch does.
+    auto near_batch = [&](int b) -> int {
+        const int half = b & 1;
+        const int s0 = std::max(1, b * K), s1 = std::min(b * K + K - 1, last_step);
+        CK(cudaStreamWaitEvent(h->fstream, h->ev_free[half], 0), "wait");
+        CK(cudaStreamWaitEvent(h->fstream, h->ev_inner, 0), "wait");
+        if (launch_near_cells(h, s0, s1 - s0 + 1, h->fstream)) return cuda_err(h, cudaGetLastError(), "launch near cells");
+        h->near_in_half[half] = b;
+        CK(cudaEventRecord(h->ev_batch[half], h->fstream), "event");
         return LBM_OK;
     };
     // The next batch's factorization runs beside this batch's steps; a call that
@@ -652,6 +669,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             const void *fin = h->fbuf[h->cur];
             void *fout = h->fbuf[h->cur ^ 1];
             if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
+            if (h->near_in_half[half] != b && (rc = near_batch(b))) return rc;
             if (h->timing == LBM_TIMING_SPAN && slot == 0) CK(cudaEventRecord(h->ev[0], h->stream), "event");
             for (cudaStream_t st : {h->side, h->nstream}) {
                 CK(cudaStreamWaitEvent(st, h->ev_inner, 0), "wait");
@@ -782,6 +800,11 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
 // attributes tell which architecture the library's device code is for
 __global__ void arch_probe() {}
 
+void forget_batches(lbm_handle *h)
+{
+    for (int q = 0; q < 2; ++q) h->batch_in_half[q] = h->near_in_half[q] = h->fgroup[q] = -1;
+}
+
 // for lbm_batch.cu
 int handle_prepare_ib(lbm_handle *h) { return ensure_ib(h); }
 int handle_fetch(lbm_handle *h, cudaStream_t st, bool mass, int rows, double *dst) { return fetch(h, st, mass, rows, dst); }
@@ -876,8 +899,7 @@ int handle_restore(lbm_handle *h, const double *f, const double *u, const double
     h->fields_slot = 0;
     h->fields_step[0] = cycle;
     h->fields_step[1] = -1;
-    h->batch_in_half[0] = h->batch_in_half[1] = -1;
-    h->fgroup[0] = h->fgroup[1] = -1;
+    forget_batches(h);
     return LBM_OK;
 }
 
@@ -1204,8 +1226,7 @@ int lbm_init(lbm_t *h, const double *du, const double *dv)
     h->steps_done = 0;
     // the patch rectangles were cleared above: the factorization slots are
     // filled again from the first step
-    h->batch_in_half[0] = h->batch_in_half[1] = -1;
-    h->fgroup[0] = h->fgroup[1] = -1;
+    forget_batches(h);
     h->inited = 1;
     return LBM_OK;
 }

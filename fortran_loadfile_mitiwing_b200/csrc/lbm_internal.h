@@ -153,6 +153,9 @@ struct lbm_handle {
     // 16 steps (96x64: 9.2 -> 8.0).
     int fbatch = 16, nslots = 32;
     int batch_in_half[2] = {-1, -1};                // batch index held by each half of the slots
+    // batch whose near cells (below) each half holds: only the handle's own
+    // two-step runs make them, a run in an lbm_batch factorizes without
+    int near_in_half[2] = {-1, -1};
     Marker *d_mk = nullptr;                         // nslots x nseg
     double *d_B = nullptr;                          // nslots x nseg*nseg
     int *d_fmode = nullptr;                         // nslots x 2
@@ -278,6 +281,7 @@ int near_cells_of(const lbm_handle *h);
 int launch_near_cells(lbm_handle *h, int step0, int count, cudaStream_t st);
 int launch_pair(lbm_handle *h, const void *fin, void *fout, cudaStream_t st);
 int launch_near(lbm_handle *h, const void *fin, void *fout, int step, int phase, cudaStream_t st);
+void forget_batches(lbm_handle *h);   // the slots hold no factorization that later steps may use
 // several steps in one launch (step_loop.cu)
 bool loop_fits(const lbm_handle *h);
 int loop_sync_words();

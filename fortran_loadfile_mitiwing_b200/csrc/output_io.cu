@@ -698,8 +698,7 @@ int lbm_load_checkpoint(lbm_t *h, const char *path)
     h->fields_step[0] = (int)hd.fields_step[0];
     h->fields_step[1] = (int)hd.fields_step[1];
     // the factorization slots are filled again for the restored step
-    h->batch_in_half[0] = h->batch_in_half[1] = -1;
-    h->fgroup[0] = h->fgroup[1] = -1;
+    forget_batches(h);
     return LBM_OK;
 }
 
