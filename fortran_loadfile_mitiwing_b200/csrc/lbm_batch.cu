@@ -50,13 +50,19 @@ constexpr int kArgRing = 8;
 // that segments of a run share their structure) and instantiated graphs kept
 constexpr int kGraphSteps = 16;
 constexpr int kGraphCache = 8;
-// argument buffers of step_loop launches in flight, entries of their CTA maps,
-// and such launches in a graph segment at most
+// argument buffers of step_loop launches in flight, entries of their CTA maps
 constexpr int kLoopRing = 4;
 constexpr int kLoopMap = 256;
-constexpr int kLoopChunks = 3;
 
 size_t round256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// step_loop launches of a graph segment that begins `phase` steps into a
+// factorization batch of K: each ends with the batch
+int loop_chunks(int phase, int K)
+{
+    const int first = K - phase;
+    return first >= kGraphSteps ? 1 : 1 + (kGraphSteps - first + K - 1) / K;
+}
 }
 
 struct lbm_batch {
@@ -263,8 +269,12 @@ int reserve(lbm_batch *b, int ncase, int ntab)
     // arguments of every case, and up to two factorization launches per step
     b->seg_bytes = round256((size_t)kGraphSteps * nc * b->ib_sz) + round256((size_t)kGraphSteps * nc * b->kf_sz) +
                    round256((size_t)2 * kGraphSteps * nc * b->ib_sz);
-    b->seg_bytes = std::max(b->seg_bytes, round256((size_t)2 * kLoopChunks * nc * b->ib_sz) +
-                                              kLoopChunks * loop_launch_bytes(b->prec, nc));
+    // or the arguments of its step_loop launches (the most a segment has
+    // begins with the last step of a batch), with up to two factorization
+    // launches for each
+    const size_t chunks = loop_chunks(b->fbatch - 1, b->fbatch);
+    b->seg_bytes = std::max(b->seg_bytes, chunks * loop_launch_bytes(b->prec, nc) +
+                                              round256((size_t)2 * chunks * nc * b->ib_sz));
     for (int q = 0; q < 2; ++q) {
         BCK(cudaMalloc(&b->d_seg[q], b->seg_bytes), "alloc");
         BCK(cudaMallocHost(&b->h_seg[q], b->seg_bytes), "alloc");
@@ -697,7 +707,10 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         const bool loop = !share.empty();
         const size_t lone = loop_launch_bytes(b->prec, na);
         const size_t off_k = round256((size_t)G * na * b->ib_sz);
-        const size_t off_f = loop ? kLoopChunks * lone : off_k + round256((size_t)G * na * b->kf_sz);
+        const int nchunk = loop ? loop_chunks(act[0]->n % K, K) : 0;
+        const size_t off_f = loop ? nchunk * lone : off_k + round256((size_t)G * na * b->kf_sz);
+        if (off_f + (size_t)2 * (loop ? nchunk : G) * na * b->ib_sz > b->seg_bytes)
+            return berr(b, LBM_ERR_STATE, "batch: a graph segment's arguments exceed their buffer");
         std::vector<GroupPlan> groups;
         std::vector<StepPlan> plan(G), chunks;
         const long long seq_seg = b->gseq;   // groups numbered above it are the segment's own
