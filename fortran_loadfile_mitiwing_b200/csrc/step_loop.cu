@@ -47,7 +47,11 @@ using namespace lbm_node;
 constexpr int LOOP_STEPS = LBM_NSLOT_MAX / 2;   // steps of one launch at most (a slot half)
 // counters, each on a line of its own
 enum { SYNC_STEP = 0, SYNC_ABORT = 32, SYNC_WORDS = 64 };
-constexpr int LOOP_SMEM = 232448 - 1024;        // dynamic shared memory a CTA may use
+// dynamic shared memory a CTA may use: a block's 227 KB less the kernel's
+// static part (up to 1536 bytes, for batches in FP64). The kernels' limit is
+// set to it, the same for every handle: the attribute is the process's, and
+// another thread may set it between this one's setting and its launch.
+constexpr int LOOP_SMEM = 232448 - 1536;
 
 // Shares of the interior items (measured on 1280x640, 131 CTAs of which some 24
 // have a tile and each CTA some 97 items; us a step): items dealt out evenly
@@ -756,7 +760,7 @@ int launch_loop_t(lbm_handle *h, int nsteps, void *const *fields, cudaStream_t s
     LoopArgs<C> L = loop_args<C>(h, nsteps, fields, 0, false);
     const size_t smem = loop_smem(h);
     auto kernel = step_loop<T, C, CONS0, false>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) != cudaSuccess) return -1;
     const int ctas = std::min(1 + loop_want(h), h->loop_ctas);
     const LoopArgs<C> *cases = nullptr;
     const int4 *map = nullptr;
@@ -770,7 +774,7 @@ template <typename T, typename C, bool CONS0>
 int launch_loop_multi_t(int ctas, size_t smem, const void *dcases, const int4 *dmap, cudaStream_t st)
 {
     auto kernel = step_loop<T, C, CONS0, true>;
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return -1;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LOOP_SMEM) != cudaSuccess) return -1;
     LoopArgs<C> none{};
     const LoopArgs<C> *cases = (const LoopArgs<C> *)dcases;
     void *args[] = {&none, &cases, &dmap};
