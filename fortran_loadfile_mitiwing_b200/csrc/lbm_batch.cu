@@ -514,6 +514,9 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         if (h->cstream) cudaStreamSynchronize(h->cstream);
         if (h->nstream) cudaStreamSynchronize(h->nstream);
         cudaStreamSynchronize(h->stream);
+        // what its slots hold is complete; the launches that filled them may
+        // be numbered by another batch
+        h->fgroup[0] = h->fgroup[1] = -1;
         int gx, gy;
         kf_tma_grid(h, &gx, &gy);
         need += gx * gy;
