@@ -800,9 +800,12 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
 // attributes tell which architecture the library's device code is for
 __global__ void arch_probe() {}
 
+// The errors of the steps discarded go with them: the next user of a slot
+// would report what no step of its own has seen.
 void forget_batches(lbm_handle *h)
 {
     for (int q = 0; q < 2; ++q) h->batch_in_half[q] = h->near_in_half[q] = h->fgroup[q] = -1;
+    if (h->d_fstatus) cudaMemsetAsync(h->d_fstatus, 0, sizeof(unsigned) * h->nslots, h->stream);
 }
 
 // for lbm_batch.cu
