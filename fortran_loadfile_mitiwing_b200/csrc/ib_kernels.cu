@@ -612,6 +612,10 @@ __global__ void __launch_bounds__(FACTOR_THREADS, 65536 / (FACTOR_THREADS * 128)
         const int w = *a.wmax;
         bad = 0;
         dense = (w > BS || a.force_dense) ? 1 : 0;
+        if (dense && !a.B) {   // dense_possible rules this out
+            atomicOr(a.status, LBM_ST_INDEX_FACTOR);
+            dense = 0;
+        }
         a.fmode[0] = dense;
         a.fmode[1] = w;
         *a.wmax = 0;   // for the next assembly
@@ -1369,13 +1373,13 @@ IBArgs make_args(lbm_handle *h, const void *fin, int slot)
     a.static_order = h->static_order;
     a.st_mk = (long long)ns;
     a.st_perm = h->static_order ? 0 : (long long)ns;
-    a.st_B = (long long)(ns * ns);
+    a.st_B = h->d_B ? (long long)(ns * ns) : 0;
     a.wk_blocks = (long long)h->work_blocks;
     a.wk_gf = (long long)h->gf_slot;
     a.mk = h->d_mk + slot * ns;
     a.perm = h->d_perm + slot * a.st_perm;
     a.key = h->d_key + slot * a.st_perm;
-    a.B = h->d_B + slot * ns * ns;
+    a.B = h->d_B + slot * a.st_B;
     a.fmode = h->d_fmode + 2 * slot;
     a.fstatus = h->d_fstatus + slot;
     a.pinfo = h->d_pinfo + slot;

@@ -253,6 +253,157 @@ bool pairs_fit(const lbm_handle *h)
            h->ny >= 64 && h->plane < (1ll << 31) && 18ll * h->elem * h->plane >= 40000000ll;
 }
 
+// Whether some step of the motion may need the dense factor of the marker
+// system: a coupling of more than kBand places in the solve order (ib_factor),
+// that is two markers whose support boxes (at most 5 lattice units from first
+// to last node) share a node with kBand others or more between them. The
+// factor takes 8 nseg^2 bytes a step slot and next to no case uses it (a
+// contour with a marker per lattice unit has couplings of some 14 places), so
+// it is allocated only where this bound does not rule it out.
+constexpr int kBand = 16;
+constexpr double kSpan = 5.0 + 1.0e-6;   // lattice units; positions are rounded
+
+// One body: its order is fixed in its own frame, where two markers that couple
+// are at most 5 sqrt(2) units apart whatever its angle.
+bool band_exceeded(const std::vector<double> &x, const std::vector<double> &y)
+{
+    const int n = (int)x.size();
+    std::vector<int> at(n);
+    for (int k = 0; k < n; ++k) at[k] = k;
+    std::stable_sort(at.begin(), at.end(), [&](int p, int q) { return x[p] < x[q]; });
+    const double reach = sqrt(2.0) * kSpan;
+    for (int p = 0; p < n; ++p)
+        for (int q = p + kBand + 1; q < n && x[at[q]] - x[at[p]] <= reach; ++q)
+            if (hypot(x[at[q]] - x[at[p]], y[at[q]] - y[at[p]]) <= reach) return true;
+    return false;
+}
+
+// A body of several, over the angles of its motion: sampled so densely that no
+// marker moves more than kMove relative to another between two samples.
+constexpr double kMove = 1.0;
+struct BodyRange {
+    std::vector<double> x, y;    // markers in the body's frame, lattice units
+    double a0 = 1e300, a1 = -1e300;
+    int samples = 0;
+    double lo[2], hi[2];         // extent along x and y about the pivot, over all angles,
+    double in_lo[2], in_hi[2];   // and what it covers at every angle
+    void keys(int t, int d, std::vector<double> &v) const
+    {
+        const double a = samples > 1 ? a0 + (a1 - a0) * t / (samples - 1) : a0, ca = cos(a), sn = d == 0 ? sin(a) : -sin(a);
+        const std::vector<double> &p = d == 0 ? x : y, &q = d == 0 ? y : x;
+        v.resize(p.size());
+        for (size_t k = 0; k < p.size(); ++k) v[k] = ca * p[k] + sn * q[k];
+    }
+    void extents()
+    {
+        std::vector<double> v;
+        for (int d = 0; d < 2; ++d) {
+            lo[d] = in_hi[d] = 1e300;
+            hi[d] = in_lo[d] = -1e300;
+            for (int t = 0; t < samples; ++t) {
+                keys(t, d, v);
+                const auto m = std::minmax_element(v.begin(), v.end());
+                lo[d] = std::min(lo[d], *m.first - kMove);
+                hi[d] = std::max(hi[d], *m.second + kMove);
+                in_lo[d] = std::max(in_lo[d], *m.first + kMove);
+                in_hi[d] = std::min(in_hi[d], *m.second - kMove);
+            }
+        }
+    }
+    // the most markers within kSpan along an axis
+    int most(int d) const
+    {
+        std::vector<double> v;
+        int m = 0;
+        for (int t = 0; t < samples; ++t) {
+            keys(t, d, v);
+            std::sort(v.begin(), v.end());
+            size_t p = 0;
+            for (size_t q = 0; q < v.size(); ++q) {
+                while (v[q] - v[p] > kSpan + kMove) ++p;
+                m = std::max(m, (int)(q - p) + 1);
+            }
+        }
+        return m;
+    }
+};
+
+// Several bodies: the order follows the longer axis of all markers; a coupling
+// spans no more places than a window of kSpan along it holds markers, of the
+// bodies that can be in it together.
+bool dense_possible(const lbm_handle *h)
+{
+    if (h->nseg > 0 && (h->p.flags & LBM_FLAG_DENSE_SOLVE)) return true;
+    if (h->nseg <= kBand + 1) return false;
+    const int nw = h->nwing;
+    std::vector<BodyRange> body(nw);
+    for (int w = 0; w < nw; ++w)
+        for (int k = 0; k < h->spw; ++k) {
+            const int q = w * h->ppw + k;
+            body[w].x.push_back(0.5 * (h->hx0[q] + h->hx0[q + 1]) / h->p.scale);
+            body[w].y.push_back(0.5 * (h->hy0[q] + h->hy0[q + 1]) / h->p.scale);
+        }
+    if (nw == 1) return band_exceeded(body[0].x, body[0].y);
+    // angles, and from pivot p to pivot q > p the least and the largest distance
+    double c0[2][LBM_MAXW][LBM_MAXW], c1[2][LBM_MAXW][LBM_MAXW];
+    for (int d = 0; d < 2; ++d)
+        for (int p = 0; p < nw; ++p)
+            for (int q = 0; q < nw; ++q) {
+                c0[d][p][q] = 1e300;
+                c1[d][p][q] = -1e300;
+            }
+    for (int s = 0; s < h->msteps; ++s) {
+        const double *row = &h->mstep_host[(size_t)s * h->mcols];
+        for (int p = 0; p < nw; ++p) {
+            body[p].a0 = std::min(body[p].a0, row[1 + 9 * p]);
+            body[p].a1 = std::max(body[p].a1, row[1 + 9 * p]);
+            for (int d = 0; d < 2; ++d)
+                for (int q = p; q < nw; ++q) {
+                    const double c = (row[4 + 3 * d + 9 * q] - row[4 + 3 * d + 9 * p]) / h->p.scale;
+                    c0[d][p][q] = std::min(c0[d][p][q], c);
+                    c1[d][p][q] = std::max(c1[d][p][q], c);
+                }
+        }
+    }
+    for (BodyRange &b : body) {
+        double r = 0.0;
+        for (size_t k = 0; k < b.x.size(); ++k) r = std::max(r, hypot(b.x[k], b.y[k]));
+        const double samples = std::ceil(r * (b.a1 - b.a0) / kMove) + 1.0;
+        if (!(samples >= 1.0 && samples <= 1000.0)) return true;   // (turns of a large body: not worth the time)
+        b.samples = (int)samples;
+        b.extents();
+    }
+    double cloud_min[2] = {0.0, 0.0}, cloud_max[2] = {0.0, 0.0};   // extent of all markers
+    for (int d = 0; d < 2; ++d)
+        for (int p = 0; p < nw; ++p)
+            for (int q = 0; q < nw; ++q) {
+                if (q < p) {
+                    c0[d][p][q] = -c1[d][q][p];
+                    c1[d][p][q] = -c0[d][q][p];
+                }
+                cloud_min[d] = std::max(cloud_min[d], c0[d][p][q] + body[q].in_hi[d] - body[p].in_lo[d]);
+                cloud_max[d] = std::max(cloud_max[d], c1[d][p][q] + body[q].hi[d] - body[p].lo[d]);
+            }
+    for (int d = 0; d < 2; ++d) {
+        if (cloud_max[d] < cloud_min[d ^ 1]) continue;   // never the longer axis
+        std::vector<int> most(nw);
+        for (int p = 0; p < nw; ++p) {
+            int same = p;   // a body of the same contour and angles
+            for (int q = 0; q < p && same == p; ++q)
+                if (body[q].x == body[p].x && body[q].y == body[p].y && body[q].a0 == body[p].a0 && body[q].a1 == body[p].a1) same = q;
+            most[p] = same < p ? most[same] : body[p].most(d);
+        }
+        for (int p = 0; p < nw; ++p) {
+            int window = 0;
+            for (int q = 0; q < nw; ++q)
+                if (c0[d][p][q] + body[q].lo[d] - body[p].hi[d] <= kSpan && body[p].lo[d] - c1[d][p][q] - body[q].hi[d] <= kSpan)
+                    window += most[q];
+            if (window > kBand + 1) return true;
+        }
+    }
+    return false;
+}
+
 // Allocates the immersed-boundary scratch once geometry and motion are known:
 // the correction patch is sized by the largest per-step rectangle of the
 // bodies' bounding discs over the whole motion table.
@@ -302,7 +453,7 @@ int ensure_ib(lbm_handle *h)
     CK(dmalloc(h, &h->d_mk, S * sizeof(Marker) * ns), "alloc markers");
     CK(dmalloc(h, &h->d_rhs, S * sizeof(double) * 2 * ns), "alloc rhs");
     CK(dmalloc(h, &h->d_y, S * sizeof(double) * 2 * ns), "alloc y");
-    CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
+    if (dense_possible(h)) CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
     ib_factor_scratch(ns, &h->work_blocks, &h->gf_slot);
     CK(dmalloc(h, &h->d_bD, K * sizeof(double) * h->work_blocks), "alloc block D");
     CK(dmalloc(h, &h->d_bL, K * sizeof(double) * h->work_blocks), "alloc block L");

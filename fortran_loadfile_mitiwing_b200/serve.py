@@ -30,6 +30,7 @@ import time
 
 import numpy as np
 
+from ._abi import LBM_FLAG_DENSE_SOLVE
 from .solver import Batch, Lbm
 
 # sizes of the device structures a case holds (csrc/lbm_common.cuh, lbm_internal.h, ib_kernels.cu)
@@ -82,6 +83,33 @@ def _pairs(elem, pitch, nx, ny, ns):
     return not loop and nx >= 64 and ny >= 64 and 18 * elem * pitch * ny >= 40_000_000
 
 
+def _dense(case):
+    """Whether a case holds the dense factors of the marker system
+    (dense_possible, csrc/lbm_capi.cu): asked for, or a coupling of more than
+    16 places in the solve order cannot be ruled out. For several bodies the
+    library looks at their motion; here they count as if it could not."""
+    p = case.params
+    ns = p.wing_count * (p.points_per_wing - 1)
+    if ns > 0 and p.flags & LBM_FLAG_DENSE_SOLVE:
+        return True
+    if ns <= _BS + 1:
+        return False
+    if p.wing_count > 1:
+        return True
+    x, y = (np.asarray(c, dtype=np.float64) for c in case.contours[0])
+    x, y = 0.5 * (x[:-1] + x[1:]) / p.scale, 0.5 * (y[:-1] + y[1:]) / p.scale
+    order = np.argsort(x, kind="stable")
+    x, y = x[order], y[order]
+    reach = math.sqrt(2.0) * (5.0 + 1.0e-6)
+    for k in range(_BS + 1, ns):
+        dx = x[k:] - x[:-k]
+        if not np.any(dx <= reach):
+            return False
+        if np.any(np.hypot(dx, y[k:] - y[:-k]) <= reach):
+            return True
+    return False
+
+
 def estimate_device_bytes(case):
     """Device bytes a case holds while it is stepped: lattice buffers, fields
     and edge values (lbm_create), step table and contour, and the
@@ -110,7 +138,7 @@ def estimate_device_bytes(case):
         pw, ph = patch_extent(case)
         nblk = max(1, (pw + 15) // 16) * max(1, (ph + 15) // 16)
         # right-hand sides, solution and tile partials: one set per slot
-        total += S * _MARKER_BYTES * ns + S * 2 * 8 * 2 * ns + S * 8 * ns * ns
+        total += S * _MARKER_BYTES * ns + S * 2 * 8 * 2 * ns + (S * 8 * ns * ns if _dense(case) else 0)
         total += 2 * K * 8 * nb * _BS * _BS + S * 8 * nb * _BS * _GW + S * 2 * 4 + S * 4
         total += S * 8 * (_NPART * nblk + 2 * ((ns + 7) // 8) + 1)
         total += S * 4 * _TILE_INTS * nblk + S * 4 + S * 4 * nblk
