@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(FACTOR_THREADS, 65536 / (FACTOR_THREADS * 128)
         const int w = *a.wmax;
         bad = 0;
         dense = (w > BS || a.force_dense) ? 1 : 0;
-        if (dense && !a.B) {   // dense_possible rules this out
+        if (dense && !a.B) {   // ensure_ib rules this out
             atomicOr(a.status, LBM_ST_INDEX_FACTOR);
             dense = 0;
         }

@@ -312,7 +312,7 @@ int check_case(lbm_batch *b, lbm_handle *h)
     if (h->fstream) cudaStreamSynchronize(h->fstream);
     if (h->side) cudaStreamSynchronize(h->side);
     if (h->cstream) cudaStreamSynchronize(h->cstream);
-        if (h->nstream) cudaStreamSynchronize(h->nstream);
+    if (h->nstream) cudaStreamSynchronize(h->nstream);
     if (cudaStreamSynchronize(h->stream) != cudaSuccess) return handle_error(h, LBM_ERR_CUDA, "batch: sync");
     return LBM_OK;
 }

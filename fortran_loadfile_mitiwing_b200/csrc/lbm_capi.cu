@@ -263,78 +263,98 @@ bool pairs_fit(const lbm_handle *h)
 constexpr int kBand = 16;
 constexpr double kSpan = 5.0 + 1.0e-6;   // lattice units; positions are rounded
 
-// One body: its order is fixed in its own frame, where two markers that couple
-// are at most 5 sqrt(2) units apart whatever its angle.
-bool band_exceeded(const std::vector<double> &x, const std::vector<double> &y)
+// The solve order of one rigid body, kept for the whole run: by body-frame
+// chordwise position (two markers whose support boxes overlap are less than
+// 5 sqrt(2) lattice units apart in any orientation). key: the positions.
+void body_order(const lbm_handle *h, std::vector<int> &perm, std::vector<double> &key)
 {
-    const int n = (int)x.size();
-    std::vector<int> at(n);
-    for (int k = 0; k < n; ++k) at[k] = k;
-    std::stable_sort(at.begin(), at.end(), [&](int p, int q) { return x[p] < x[q]; });
-    const double reach = sqrt(2.0) * kSpan;
+    const int n = h->nseg;
+    std::vector<double> x(n);
+    perm.resize(n);
+    key.resize(n);
+    for (int k = 0; k < n; ++k) {
+        perm[k] = k;
+        x[k] = 0.5 * (h->hx0[k] + h->hx0[k + 1]);
+    }
+    std::stable_sort(perm.begin(), perm.end(), [&](int p, int q) { return x[p] < x[q]; });
+    for (int q = 0; q < n; ++q) key[q] = x[perm[q]];
+}
+
+// One body in its order
+bool band_exceeded(const lbm_handle *h, const std::vector<int> &perm, const std::vector<double> &key)
+{
+    const int n = h->nseg;
+    const double reach = sqrt(2.0) * kSpan * h->p.scale;
+    auto y = [&](int q) { return 0.5 * (h->hy0[perm[q]] + h->hy0[perm[q] + 1]); };
     for (int p = 0; p < n; ++p)
-        for (int q = p + kBand + 1; q < n && x[at[q]] - x[at[p]] <= reach; ++q)
-            if (hypot(x[at[q]] - x[at[p]], y[at[q]] - y[at[p]]) <= reach) return true;
+        for (int q = p + kBand + 1; q < n && key[q] - key[p] <= reach; ++q)
+            if (hypot(key[q] - key[p], y(q) - y(p)) <= reach) return true;
     return false;
 }
 
-// A body of several, over the angles of its motion: sampled so densely that no
-// marker moves more than kMove relative to another between two samples.
-constexpr double kMove = 1.0;
+// A body of several, over the angles of its motion
 struct BodyRange {
     std::vector<double> x, y;    // markers in the body's frame, lattice units
-    double a0 = 1e300, a1 = -1e300;
-    int samples = 0;
+    double a0 = 1e300, a1 = -1e300, r = 0.0;   // angles, distance of the farthest marker
     double lo[2], hi[2];         // extent along x and y about the pivot, over all angles,
     double in_lo[2], in_hi[2];   // and what it covers at every angle
-    void keys(int t, int d, std::vector<double> &v) const
+    // samples of the angle between the nearest of which and any other angle no
+    // marker moves more than `move` relative to another
+    double samples(double move) const { return std::ceil(r * (a1 - a0) / move) + 1.0; }
+    // positions along an axis, f(position) for each marker of sample t of n
+    template <class F> void each(int t, int n, int d, F f) const
     {
-        const double a = samples > 1 ? a0 + (a1 - a0) * t / (samples - 1) : a0, ca = cos(a), sn = d == 0 ? sin(a) : -sin(a);
-        const std::vector<double> &p = d == 0 ? x : y, &q = d == 0 ? y : x;
-        v.resize(p.size());
-        for (size_t k = 0; k < p.size(); ++k) v[k] = ca * p[k] + sn * q[k];
+        const double a = n > 1 ? a0 + (a1 - a0) * t / (n - 1) : a0, ca = cos(a), sn = d == 0 ? sin(a) : -sin(a);
+        const double *p = d == 0 ? x.data() : y.data(), *q = d == 0 ? y.data() : x.data();
+        for (size_t k = 0; k < x.size(); ++k) f(ca * p[k] + sn * q[k]);
     }
     void extents()
     {
-        std::vector<double> v;
+        const double move = std::max(1.0, r * (a1 - a0) / 15.0);
+        const int n = (int)samples(move);
         for (int d = 0; d < 2; ++d) {
             lo[d] = in_hi[d] = 1e300;
             hi[d] = in_lo[d] = -1e300;
-            for (int t = 0; t < samples; ++t) {
-                keys(t, d, v);
-                const auto m = std::minmax_element(v.begin(), v.end());
-                lo[d] = std::min(lo[d], *m.first - kMove);
-                hi[d] = std::max(hi[d], *m.second + kMove);
-                in_lo[d] = std::max(in_lo[d], *m.first + kMove);
-                in_hi[d] = std::min(in_hi[d], *m.second - kMove);
+            for (int t = 0; t < n; ++t) {
+                double v0 = 1e300, v1 = -1e300;
+                each(t, n, d, [&](double v) {
+                    v0 = v < v0 ? v : v0;
+                    v1 = v > v1 ? v : v1;
+                });
+                lo[d] = std::min(lo[d], v0 - move);
+                hi[d] = std::max(hi[d], v1 + move);
+                in_lo[d] = std::max(in_lo[d], v0 + move);
+                in_hi[d] = std::min(in_hi[d], v1 - move);
             }
         }
     }
-    // the most markers within kSpan along an axis
+    // a bound on the markers within kSpan along an axis: those of 13 successive
+    // bins of half a unit, which hold any window of kSpan + kMove
+    static constexpr double kMove = 0.9;
     int most(int d) const
     {
-        std::vector<double> v;
+        std::vector<int> bin((size_t)(4.0 * r) + 16);
+        const int n = (int)samples(kMove);
         int m = 0;
-        for (int t = 0; t < samples; ++t) {
-            keys(t, d, v);
-            std::sort(v.begin(), v.end());
-            size_t p = 0;
-            for (size_t q = 0; q < v.size(); ++q) {
-                while (v[q] - v[p] > kSpan + kMove) ++p;
-                m = std::max(m, (int)(q - p) + 1);
+        for (int t = 0; t < n; ++t) {
+            std::fill(bin.begin(), bin.end(), 0);
+            each(t, n, d, [&](double v) { ++bin[(size_t)(2.0 * (v + r) + 1.0)]; });   // |v| <= r, but for rounding
+            int sum = 0;
+            for (size_t q = 0; q < bin.size(); ++q) {
+                sum += bin[q] - (q >= 13 ? bin[q - 13] : 0);
+                m = std::max(m, sum);
             }
         }
         return m;
     }
+    bool same(const BodyRange &o) const { return x == o.x && y == o.y && a0 == o.a0 && a1 == o.a1; }
 };
 
 // Several bodies: the order follows the longer axis of all markers; a coupling
 // spans no more places than a window of kSpan along it holds markers, of the
 // bodies that can be in it together.
-bool dense_possible(const lbm_handle *h)
+bool window_exceeded(const lbm_handle *h)
 {
-    if (h->nseg > 0 && (h->p.flags & LBM_FLAG_DENSE_SOLVE)) return true;
-    if (h->nseg <= kBand + 1) return false;
     const int nw = h->nwing;
     std::vector<BodyRange> body(nw);
     for (int w = 0; w < nw; ++w)
@@ -343,7 +363,6 @@ bool dense_possible(const lbm_handle *h)
             body[w].x.push_back(0.5 * (h->hx0[q] + h->hx0[q + 1]) / h->p.scale);
             body[w].y.push_back(0.5 * (h->hy0[q] + h->hy0[q + 1]) / h->p.scale);
         }
-    if (nw == 1) return band_exceeded(body[0].x, body[0].y);
     // angles, and from pivot p to pivot q > p the least and the largest distance
     double c0[2][LBM_MAXW][LBM_MAXW], c1[2][LBM_MAXW][LBM_MAXW];
     for (int d = 0; d < 2; ++d)
@@ -366,11 +385,9 @@ bool dense_possible(const lbm_handle *h)
         }
     }
     for (BodyRange &b : body) {
-        double r = 0.0;
-        for (size_t k = 0; k < b.x.size(); ++k) r = std::max(r, hypot(b.x[k], b.y[k]));
-        const double samples = std::ceil(r * (b.a1 - b.a0) / kMove) + 1.0;
-        if (!(samples >= 1.0 && samples <= 1000.0)) return true;   // (turns of a large body: not worth the time)
-        b.samples = (int)samples;
+        for (size_t k = 0; k < b.x.size(); ++k) b.r = std::max(b.r, hypot(b.x[k], b.y[k]));
+        const double n = b.samples(BodyRange::kMove);
+        if (!(n >= 1.0 && n <= 1000.0 && b.r <= 1.0e5)) return true;   // (turns of a large body: not worth the time)
         b.extents();
     }
     double cloud_min[2] = {0.0, 0.0}, cloud_max[2] = {0.0, 0.0};   // extent of all markers
@@ -388,10 +405,9 @@ bool dense_possible(const lbm_handle *h)
         if (cloud_max[d] < cloud_min[d ^ 1]) continue;   // never the longer axis
         std::vector<int> most(nw);
         for (int p = 0; p < nw; ++p) {
-            int same = p;   // a body of the same contour and angles
-            for (int q = 0; q < p && same == p; ++q)
-                if (body[q].x == body[p].x && body[q].y == body[p].y && body[q].a0 == body[p].a0 && body[q].a1 == body[p].a1) same = q;
-            most[p] = same < p ? most[same] : body[p].most(d);
+            int q = 0;
+            while (q < p && !body[q].same(body[p])) ++q;
+            most[p] = q < p ? most[q] : body[p].most(d);
         }
         for (int p = 0; p < nw; ++p) {
             int window = 0;
@@ -453,7 +469,13 @@ int ensure_ib(lbm_handle *h)
     CK(dmalloc(h, &h->d_mk, S * sizeof(Marker) * ns), "alloc markers");
     CK(dmalloc(h, &h->d_rhs, S * sizeof(double) * 2 * ns), "alloc rhs");
     CK(dmalloc(h, &h->d_y, S * sizeof(double) * 2 * ns), "alloc y");
-    if (dense_possible(h)) CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
+    std::vector<int> perm;
+    std::vector<double> key;
+    h->static_order = h->nwing == 1;
+    if (h->static_order) body_order(h, perm, key);
+    if (h->nseg > 0 && ((h->p.flags & LBM_FLAG_DENSE_SOLVE) ||
+                        (h->nseg > kBand + 1 && (h->static_order ? band_exceeded(h, perm, key) : window_exceeded(h)))))
+        CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
     ib_factor_scratch(ns, &h->work_blocks, &h->gf_slot);
     CK(dmalloc(h, &h->d_bD, K * sizeof(double) * h->work_blocks), "alloc block D");
     CK(dmalloc(h, &h->d_bL, K * sizeof(double) * h->work_blocks), "alloc block L");
@@ -474,25 +496,14 @@ int ensure_ib(lbm_handle *h)
     CK(dmalloc(h, &h->d_nsup, S * sizeof(int)), "alloc tile counts");
     CK(dmalloc(h, &h->d_ctile, S * sizeof(int) * (size_t)nblk), "alloc correction tiles");
     CK(cudaMemsetAsync(h->d_nsup, 0, S * sizeof(int), h->stream), "clear tile counts");
-    // solve order of the markers: one rigid body keeps its markers sorted by
-    // body-frame chordwise position for the whole run (two markers whose
-    // support boxes overlap are less than 5*sqrt(2) lattice units apart in any
-    // orientation); several bodies are sorted on the device every step
+    // solve order of the markers: one rigid body keeps its own; several are
+    // sorted on the device every step
     CK(dmalloc(h, &h->d_perm, S * sizeof(int) * ns), "alloc perm");
     CK(dmalloc(h, &h->d_key, S * sizeof(double) * ns), "alloc key");
     CK(dmalloc(h, &h->d_reach, sizeof(double)), "alloc reach");
     CK(dmalloc(h, &h->d_wmax, K * sizeof(int)), "alloc wmax");
     CK(cudaMemsetAsync(h->d_wmax, 0, K * sizeof(int), h->stream), "clear wmax");
-    h->static_order = h->nwing == 1;
     if (h->static_order) {
-        std::vector<int> perm(h->nseg);
-        std::vector<double> xk(h->nseg), key(h->nseg);
-        for (int k = 0; k < h->nseg; ++k) {
-            perm[k] = k;
-            xk[k] = 0.5 * (h->hx0[k] + h->hx0[k + 1]);
-        }
-        std::stable_sort(perm.begin(), perm.end(), [&](int p1, int p2) { return xk[p1] < xk[p2]; });
-        for (int q = 0; q < h->nseg; ++q) key[q] = xk[perm[q]];
         const double reach = 7.1 * h->p.scale;
         CK(cudaMemcpyAsync(h->d_perm, perm.data(), sizeof(int) * h->nseg, cudaMemcpyHostToDevice, h->stream), "copy perm");
         CK(cudaMemcpyAsync(h->d_key, key.data(), sizeof(double) * h->nseg, cudaMemcpyHostToDevice, h->stream), "copy key");
@@ -501,6 +512,13 @@ int ensure_ib(lbm_handle *h)
     }
     if (pairs_fit(h)) {
         const int cells = near_cells_of(h);
+        if (!h->nstream) {   // with the events only here, most handles do without
+            int low = 0, high = 0;
+            cudaDeviceGetStreamPriorityRange(&low, &high);
+            for (cudaEvent_t &ev : h->ev_near)
+                if (!ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), "event");
+            CK(cudaStreamCreateWithPriority(&h->nstream, cudaStreamNonBlocking, high), "near stream");
+        }
         CK(dmalloc(h, &h->fmid_alloc, h->elem * (9 * (size_t)h->plane + 2 * LBM_FPAD)), "alloc f between");
         h->fmid = (char *)h->fmid_alloc + h->elem * LBM_FPAD;
         CK(dmalloc(h, &h->d_near, S / 2 * near_bytes(cells)), "alloc near cells");
@@ -1151,10 +1169,7 @@ int lbm_create(const lbm_params *p, lbm_t **out)
     if ((e = cudaStreamCreateWithPriority(&h->cstream, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
         return fail(e, "check stream");
     if ((e = cudaEventCreateWithFlags(&h->ev_cjoin, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
-    if ((e = cudaStreamCreateWithPriority(&h->nstream, cudaStreamNonBlocking, prio_high)) != cudaSuccess)
-        return fail(e, "near stream");
     for (int q = 0; q < 2; ++q) {
-        if ((e = cudaEventCreateWithFlags(&h->ev_near[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
         if ((e = cudaEventCreateWithFlags(&h->ev_batch[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
         if ((e = cudaEventCreateWithFlags(&h->ev_free[q], cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
     }

@@ -157,7 +157,7 @@ struct lbm_handle {
     // two-step runs make them, a run in an lbm_batch factorizes without
     int near_in_half[2] = {-1, -1};
     Marker *d_mk = nullptr;                         // nslots x nseg
-    double *d_B = nullptr;                          // nslots x nseg*nseg, or null: no step needs it (dense_possible)
+    double *d_B = nullptr;                          // nslots x nseg*nseg, or null: no step needs it (ensure_ib)
     int *d_fmode = nullptr;                         // nslots x 2
     unsigned *d_fstatus = nullptr;                  // nslots
     double *d_gf = nullptr;                         // nslots x gf_slot doubles

@@ -85,7 +85,7 @@ def _pairs(elem, pitch, nx, ny, ns):
 
 def _dense(case):
     """Whether a case holds the dense factors of the marker system
-    (dense_possible, csrc/lbm_capi.cu): asked for, or a coupling of more than
+    (ensure_ib, csrc/lbm_capi.cu): asked for, or a coupling of more than
     16 places in the solve order cannot be ruled out. For several bodies the
     library looks at their motion; here they count as if it could not."""
     p = case.params
