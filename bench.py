@@ -250,7 +250,7 @@ def run_ours(args, world, rank, local):
     # steps only, so that no per-step event sits in the streams
     lib.lbm_set_timing(s.h, _abi.LBM_TIMING_SPAN)
     n0 = C.c_longlong()
-    lib.lbm_get_launch_count(s.h, C.byref(n0))
+    lib.lbm_get_device_launches(s.h, C.byref(n0))
     if world > 1:
         torch.distributed.barrier()
     torch.cuda.synchronize()
@@ -260,7 +260,7 @@ def run_ours(args, world, rank, local):
     torch.cuda.synchronize()
     clocks = sampler.stop()
     n1 = C.c_longlong()
-    lib.lbm_get_launch_count(s.h, C.byref(n1))
+    lib.lbm_get_device_launches(s.h, C.byref(n1))
     step_ms, ib_ms, kf_ms, nt = C.c_double(), C.c_double(), C.c_double(), C.c_int()
     lib.lbm_get_timing(s.h, C.byref(step_ms), None, None, C.byref(nt))
     assert nt.value == k and rows.shape[0] == k, (nt.value, rows.shape)

@@ -90,6 +90,7 @@ ABI = {
     "lbm_get_timing": (C.c_int, [_P, _D, _D, _D, C.POINTER(C.c_int)]),
     "lbm_residual_device": (C.c_int, [_P, _P, _P, _P, C.c_int, C.c_int, C.c_int, _P, _D]),
     "lbm_get_launch_count": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
+    "lbm_get_device_launches": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
     "lbm_step_index": (C.c_int, [_P]),
     "lbm_device_bytes": (C.c_int, [_P, C.POINTER(C.c_longlong)]),
     "lbm_last_error": (C.c_char_p, [_P]),

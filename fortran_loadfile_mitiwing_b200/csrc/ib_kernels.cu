@@ -1415,7 +1415,7 @@ int launch_flow_t(lbm_handle *h, const void *fin, void *fout, void *fields, int 
     IBArgs a = make_args(h, fin, slot);
     if (h->nseg > 0) {
         ib_interp<T, false><<<(h->nseg + 7) / 8, 256, 0, st>>>(a, nullptr);
-        h->launches += 1;
+        h->count(1);
     }
     if (after_interp && cudaEventRecord(after_interp, st) != cudaSuccess) return -1;
     ib_solve<false><<<1, solve_threads(h->nseg), solve_smem(h->nseg), st>>>(a, nullptr);
@@ -1425,7 +1425,7 @@ int launch_flow_t(lbm_handle *h, const void *fin, void *fout, void *fields, int 
         ib_tile_update<T, C, true, false><<<grid, 256, 0, st>>>(a, nullptr, kf, nullptr, step_index, ring_slot);
     else
         ib_tile_update<T, C, false, false><<<grid, 256, 0, st>>>(a, nullptr, kf, nullptr, step_index, ring_slot);
-    h->launches += 2;
+    h->count(2);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1438,7 +1438,7 @@ int launch_checks(lbm_handle *h, int step0, int count, int ring_slot, unsigned c
     a.ring_row = ring_slot;
     const int per = (h->nseg + 7) / 8, checks = per > 0 ? __builtin_popcount(check) : 0;
     ib_checks<false><<<count + checks * per, 256, 0, st>>>(a, nullptr, 0, count, check, check, std::max(per, 1));
-    h->launches += count + checks;   // a force row of each step, a check
+    h->count(count + checks, 1);   // a force row of each step, a check
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1497,7 +1497,7 @@ int launch_factor(lbm_handle *h, int step0, int count, cudaStream_t st)
     ib_tile_compact<false><<<dim3(1, count), 256, 0, st>>>(a, nullptr, step0);
     const int sort_ctas = std::min((h->patch_gx() * h->patch_gy() + SORT_WARPS - 1) / SORT_WARPS, SORT_CTAS);
     ib_tile_sort<false><<<dim3(sort_ctas, count), 32 * SORT_WARPS, 0, st>>>(a, nullptr, step0);
-    h->launches += h->static_order ? 6 : 7;
+    h->count(h->static_order ? 6 : 7);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1582,7 +1582,7 @@ int launch_flow_batch_t(lbm_handle *const *hs, int ncase, const IBArgs *dargs, c
         ib_tile_update<T, C, true, true><<<grid, 256, 0, st>>>(IBArgs{}, dargs, KFArgs<C>{}, kf, step_index, ring_slot);
     else
         ib_tile_update<T, C, false, true><<<grid, 256, 0, st>>>(IBArgs{}, dargs, KFArgs<C>{}, kf, step_index, ring_slot);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += 3;
+    for (int c = 0; c < ncase; ++c) hs[c]->count(3);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1608,7 +1608,7 @@ int launch_factor_batch(lbm_handle *const *hs, int ncase, const void *dargs, int
     ib_tile_compact<true><<<dim3(1, count, ncase), 256, 0, st>>>(IBArgs{}, d, step0);
     ib_tile_sort<true><<<dim3(std::min((tiles + SORT_WARPS - 1) / SORT_WARPS, SORT_CTAS), count, ncase),
                          32 * SORT_WARPS, 0, st>>>(IBArgs{}, d, step0);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += any_order ? 7 : 6;
+    for (int c = 0; c < ncase; ++c) hs[c]->count(any_order ? 7 : 6);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1641,10 +1641,10 @@ int launch_check_batch(lbm_handle *const *hs, int ncase, const void *dargs, int 
     const IBArgs *d = (const IBArgs *)dargs;
     const int ns = max_seg(hs, ncase);
     ib_forces<<<dim3(1, 1, ncase), 256, 0, st>>>(d);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
+    for (int c = 0; c < ncase; ++c) hs[c]->count(1);
     if (!residual) return cudaGetLastError() == cudaSuccess ? 0 : -1;   // no case checks this step
     ib_residual<<<dim3((ns + 7) / 8, 1, ncase), 256, 0, st>>>(d);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += 1;
+    for (int c = 0; c < ncase; ++c) hs[c]->count(1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -1655,6 +1655,6 @@ int launch_check_steps_batch(lbm_handle *const *hs, int ncase, const void *dargs
     const unsigned check = due | (last ? 1u << (count - 1) : 0u);
     const int per = (ns + 7) / 8, checks = __builtin_popcount(check);
     ib_checks<true><<<dim3(count + checks * per, 1, ncase), 256, 0, st>>>(IBArgs{}, dargs, stride, count, check, due, per);
-    for (int c = 0; c < ncase; ++c) hs[c]->launches += count + checks;
+    for (int c = 0; c < ncase; ++c) hs[c]->count(count + checks, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

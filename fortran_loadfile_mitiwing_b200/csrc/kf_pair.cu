@@ -551,6 +551,7 @@ int launch_near_t(lbm_handle *h, const void *fin, void *fout, int step, int phas
     // (a contour of 1024 markers on a chord of 512 has some 450 near cells)
     const int cell_ctas = std::min(cells, 2 * 148), edge_ctas = 24;
     kf_near<T, C, CONS0><<<cell_ctas + edge_ctas, PT, 0, st>>>(n, cell_ctas);
+    h->count(0, 1);   // (a part of the lattice)
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -574,6 +575,7 @@ int launch_near_cells(lbm_handle *h, int step0, int count, cudaStream_t st)
     ib_args_write(h, nullptr, 0, &a);
     const int cells = near_cells_of(h);
     ib_near<<<pairs, NEAR_THREADS, 0, st>>>(a, e0, h->d_near, h->d_near_list, h->d_near_count, cells, (int)near_bytes(cells));
+    h->count(0, 1);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -114,7 +114,7 @@ struct lbm_batch {
     // CUDA graph segments: two argument buffers (device and pinned host) used
     // by alternate segments, each with the event of the last graph launch
     // that read it; the instantiated graphs by segment structure, each with
-    // the kernels it launches per case (lbm_get_launch_count)
+    // the kernels it launches per case (lbm_handle::count)
     int graphs = 1;
     int gset = 0;
     size_t seg_bytes = 0;
@@ -131,7 +131,7 @@ struct lbm_batch {
     struct GraphEntry {
         std::vector<long long> sig;
         cudaGraphExec_t exec = nullptr;
-        std::vector<long long> launches;
+        std::vector<long long> launches, device_launches;
     };
     std::vector<GraphEntry> gcache;
     long long graph_steps = 0, graph_launches = 0, graph_builds = 0;   // lbm_batch_graph_stats
@@ -866,7 +866,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 if (ei) BCK(cudaStreamWaitEvent(b->main, ei, 0), "wait");   // the solves start first
                 if (launch_kf_multi(b->prec, ka, b->d_table[tcur], ntab, false, cons0, b->ctas_per_sm, b->main))
                     return berr(b, LBM_ERR_CUDA, "batch: launch lattice");
-                for (lbm_handle *h : act) h->launches += 1;
+                for (lbm_handle *h : act) h->count(1);
                 BCK(cudaStreamWaitEvent(b->main, E[5], 0), "wait");
                 BCK(cudaEventRecord(E[7], b->main), "event");   // the step is complete
             }
@@ -893,8 +893,11 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         if (!ge) {
             lbm_batch::GraphEntry e;
             e.sig = std::move(sig);
-            std::vector<long long> l0(na);
-            for (int c = 0; c < na; ++c) l0[c] = act[c]->launches;
+            std::vector<long long> l0(na), d0(na);
+            for (int c = 0; c < na; ++c) {
+                l0[c] = act[c]->launches;
+                d0[c] = act[c]->device_launches;
+            }
             cudaGraph_t graph = nullptr;
             BCK(cudaStreamBeginCapture(b->side, cudaStreamCaptureModeThreadLocal), "graph capture");
             // the capture ends whatever emit returns, so that the streams
@@ -911,9 +914,12 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
                 return erc ? erc : berr(b, LBM_ERR_CUDA, std::string("batch: graph capture: ") + cudaGetErrorString(ce));
             }
             e.launches.resize(na);
+            e.device_launches.resize(na);
             for (int c = 0; c < na; ++c) {
                 e.launches[c] = act[c]->launches - l0[c];
+                e.device_launches[c] = act[c]->device_launches - d0[c];
                 act[c]->launches = l0[c];
+                act[c]->device_launches = d0[c];
             }
             if ((int)b->gcache.size() >= kGraphCache) {
                 cudaGraphExecDestroy(b->gcache.front().exec);
@@ -924,7 +930,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
             b->graph_builds++;
         }
         BCK(cudaGraphLaunch(ge->exec, b->side), "graph launch");
-        for (int c = 0; c < na; ++c) act[c]->launches += ge->launches[c];
+        for (int c = 0; c < na; ++c) act[c]->count(ge->launches[c], ge->device_launches[c]);
         b->graph_launches++;
         b->graph_steps += G;
         // the stream code after the graph sees it as its previous step
@@ -1099,7 +1105,7 @@ int lbm_batch_run(lbm_batch_t *b, int nsteps, double *const *force_rows, int *do
         }
         BCK(cudaEventRecord(b->ev_kdone[buf], b->main), "event");
         BCK(cudaEventRecord(b->ev_tuse[tcur], b->main), "event");
-        for (lbm_handle *h : act) h->launches += 1;
+        for (lbm_handle *h : act) h->count(1);
         BCK(cudaStreamWaitEvent(b->main, b->ev_ib, 0), "wait");
         BCK(cudaEventRecord(b->ev_done, b->main), "event");   // the step is complete
         for (size_t c = 0; c < act.size(); ++c) {

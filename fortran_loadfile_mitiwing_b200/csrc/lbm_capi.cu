@@ -868,7 +868,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
                     CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
                     if (ei) CK(cudaStreamWaitEvent(h->stream, ei, 0), "wait");   // the solve starts first
                     if (launch_pair(h, fin, fout, h->stream)) return cuda_err(h, cudaGetLastError(), "launch pair");
-                    h->launches += 2;   // the lattice, for both steps
+                    h->count(2, 1);   // the lattice, for both steps
                 }
                 src = dst;
                 h->n++;
@@ -1537,6 +1537,13 @@ int lbm_get_launch_count(const lbm_t *h, long long *count)
 {
     if (!h || !count) return LBM_ERR_ARG;
     *count = h->launches;
+    return LBM_OK;
+}
+
+int lbm_get_device_launches(const lbm_t *h, long long *count)
+{
+    if (!h || !count) return LBM_ERR_ARG;
+    *count = h->device_launches;
     return LBM_OK;
 }
 

@@ -243,7 +243,15 @@ struct lbm_handle {
     std::vector<cudaEvent_t> ev, ev_side;
     double t_step = 0, t_ib = 0, t_kf = 0;
     int t_steps = 0;
-    long long launches = 0;   // kernels launched by this handle (lbm_get_launch_count)
+    // kernels run for this handle, one for each of a step's stages however they
+    // were launched (lbm_get_launch_count), and those launched (lbm_get_device_launches)
+    long long launches = 0, device_launches = 0;
+    void count(long long stages, long long launched)
+    {
+        launches += stages;
+        device_launches += launched;
+    }
+    void count(long long kernels) { count(kernels, kernels); }
     long long dev_bytes = 0;  // device memory the handle holds (lbm_device_bytes)
     long long fgroup[2] = {-1, -1};   // batch factorization launch that filled each slot half
     // driver state

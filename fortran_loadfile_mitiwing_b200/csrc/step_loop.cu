@@ -751,7 +751,7 @@ LoopArgs<C> loop_args(lbm_handle *h, int nsteps, void *const *fields, int ring_s
 void loop_done(lbm_handle *h, int ctas, int nsteps)
 {
     h->sync_base += (unsigned)(NT / TILE_THREADS * (ctas - 1) * nsteps);
-    h->launches += 4ll * nsteps;   // interpolation, solve, lattice, correction tiles of each step
+    h->count(4ll * nsteps, 1);   // interpolation, solve, lattice, correction tiles of each step
 }
 
 template <typename T, typename C, bool CONS0>

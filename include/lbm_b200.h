@@ -248,14 +248,19 @@ LBM_API int lbm_get_timing(lbm_t *h, double *step_ms, double *ib_ms, double *lat
 LBM_API int lbm_residual_device(const void *u, const void *v, const void *u0, const void *v0,
                                 int nx, int ny, int precision, void *stream, double *err);
 
-/* number of CUDA kernels run for this handle since lbm_create (all entry
- * points: steps, population transfers, residuals). A launch that works for
- * several cases counts for each of them, and one that runs several steps of a
- * small lattice counts the kernels it runs in place of (per step:
- * interpolation, solve, lattice, correction tiles, force row), so the count
- * of a run does not depend on how its kernels were launched. No counterpart
- * in the reference, which has no device code. */
+/* number of kernels run for this handle since lbm_create (all entry points:
+ * steps, population transfers, residuals), counted by the stages of the step
+ * (interpolation, solve, lattice, correction tiles, force row; residual check
+ * where due), so that the count of a run does not depend on how its stages were
+ * launched: for the launches themselves see lbm_get_device_launches. A launch
+ * that works for several cases counts for each of them. No counterpart in the
+ * reference, which has no device code. */
 LBM_API int lbm_get_launch_count(const lbm_t *h, long long *count);
+
+/* number of CUDA kernels launched for this handle since lbm_create, those that
+ * graphs launch among them. A launch that works for several cases counts for
+ * each of them; one that runs several steps or stages counts once. */
+LBM_API int lbm_get_device_launches(const lbm_t *h, long long *count);
 
 /* current step counter n of the driver loop (1 before the first step). */
 LBM_API int lbm_step_index(const lbm_t *h);
