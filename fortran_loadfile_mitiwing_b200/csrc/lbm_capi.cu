@@ -555,7 +555,7 @@ int status_error(unsigned st, std::string &msg)
         return LBM_ERR_INDEX;
     }
     if (st & LBM_ST_TIMEOUT) {
-        msg = "a bounded wait for a shared-memory copy gave up";
+        msg = "a bounded wait on the device gave up: for a shared-memory copy, or of a step_loop CTA for another";
         return LBM_ERR_CUDA;
     }
     if (st & LBM_ST_RANGE) {

@@ -34,7 +34,7 @@ __host__ __device__ constexpr int lbm_ey(int k)
 #define LBM_ST_SOLVER 2u     // IB matrix not positive definite
 #define LBM_ST_NONFINITE 4u  // NaN/Inf in forces
 #define LBM_ST_OVERFLOW 8u   // patch larger than its allocation
-#define LBM_ST_TIMEOUT 16u   // a bounded wait on a shared-memory barrier gave up
+#define LBM_ST_TIMEOUT 16u   // a bounded wait gave up: on a shared-memory barrier, or for another CTA (step_loop)
 // An index read from device memory (a solve-order position, a tile-list
 // entry, a correction-tile number, a marker's support box or wing) fell
 // outside the buffer it indexes. The kernel that saw it sets its own bit and
