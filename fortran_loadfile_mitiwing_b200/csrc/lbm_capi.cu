@@ -292,6 +292,33 @@ bool band_exceeded(const lbm_handle *h, const std::vector<int> &perm, const std:
     return false;
 }
 
+// What the rows of a step table span: angles, and displacements (x, y) of body
+// q less those of body p < q
+struct MotionRange {
+    double a0[LBM_MAXW], a1[LBM_MAXW], c0[2][LBM_MAXW][LBM_MAXW], c1[2][LBM_MAXW][LBM_MAXW];
+    MotionRange()
+    {
+        std::fill(a0, a0 + LBM_MAXW, 1e300);
+        std::fill(a1, a1 + LBM_MAXW, -1e300);
+        std::fill(&c0[0][0][0], &c0[0][0][0] + 2 * LBM_MAXW * LBM_MAXW, 1e300);
+        std::fill(&c1[0][0][0], &c1[0][0][0] + 2 * LBM_MAXW * LBM_MAXW, -1e300);
+    }
+    void add(const double *row, int nwing)
+    {
+        for (int p = 0; p < nwing; ++p) {
+            const double a = row[1 + 9 * p];
+            a0[p] = a < a0[p] ? a : a0[p];
+            a1[p] = a > a1[p] ? a : a1[p];
+            for (int d = 0; d < 2; ++d)
+                for (int q = p + 1; q < nwing; ++q) {
+                    const double c = row[4 + 3 * d + 9 * q] - row[4 + 3 * d + 9 * p];
+                    c0[d][p][q] = c < c0[d][p][q] ? c : c0[d][p][q];
+                    c1[d][p][q] = c > c1[d][p][q] ? c : c1[d][p][q];
+                }
+        }
+    }
+};
+
 // A body of several, over the angles of its motion
 struct BodyRange {
     std::vector<double> x, y;    // markers in the body's frame, lattice units
@@ -353,7 +380,7 @@ struct BodyRange {
 // Several bodies: the order follows the longer axis of all markers; a coupling
 // spans no more places than a window of kSpan along it holds markers, of the
 // bodies that can be in it together.
-bool window_exceeded(const lbm_handle *h)
+bool window_exceeded(const lbm_handle *h, const MotionRange &range)
 {
     const int nw = h->nwing;
     std::vector<BodyRange> body(nw);
@@ -363,26 +390,9 @@ bool window_exceeded(const lbm_handle *h)
             body[w].x.push_back(0.5 * (h->hx0[q] + h->hx0[q + 1]) / h->p.scale);
             body[w].y.push_back(0.5 * (h->hy0[q] + h->hy0[q + 1]) / h->p.scale);
         }
-    // angles, and from pivot p to pivot q > p the least and the largest distance
-    double c0[2][LBM_MAXW][LBM_MAXW], c1[2][LBM_MAXW][LBM_MAXW];
-    for (int d = 0; d < 2; ++d)
-        for (int p = 0; p < nw; ++p)
-            for (int q = 0; q < nw; ++q) {
-                c0[d][p][q] = 1e300;
-                c1[d][p][q] = -1e300;
-            }
-    for (int s = 0; s < h->msteps; ++s) {
-        const double *row = &h->mstep_host[(size_t)s * h->mcols];
-        for (int p = 0; p < nw; ++p) {
-            body[p].a0 = std::min(body[p].a0, row[1 + 9 * p]);
-            body[p].a1 = std::max(body[p].a1, row[1 + 9 * p]);
-            for (int d = 0; d < 2; ++d)
-                for (int q = p; q < nw; ++q) {
-                    const double c = (row[4 + 3 * d + 9 * q] - row[4 + 3 * d + 9 * p]) / h->p.scale;
-                    c0[d][p][q] = std::min(c0[d][p][q], c);
-                    c1[d][p][q] = std::max(c1[d][p][q], c);
-                }
-        }
+    for (int w = 0; w < nw; ++w) {
+        body[w].a0 = range.a0[w];
+        body[w].a1 = range.a1[w];
     }
     for (BodyRange &b : body) {
         for (size_t k = 0; k < b.x.size(); ++k) b.r = std::max(b.r, hypot(b.x[k], b.y[k]));
@@ -391,13 +401,12 @@ bool window_exceeded(const lbm_handle *h)
         b.extents();
     }
     double cloud_min[2] = {0.0, 0.0}, cloud_max[2] = {0.0, 0.0};   // extent of all markers
+    double c0[2][LBM_MAXW][LBM_MAXW], c1[2][LBM_MAXW][LBM_MAXW];   // from pivot p to pivot q, lattice units
     for (int d = 0; d < 2; ++d)
         for (int p = 0; p < nw; ++p)
             for (int q = 0; q < nw; ++q) {
-                if (q < p) {
-                    c0[d][p][q] = -c1[d][q][p];
-                    c1[d][p][q] = -c0[d][q][p];
-                }
+                c0[d][p][q] = (q > p ? range.c0[d][p][q] : q < p ? -range.c1[d][q][p] : 0.0) / h->p.scale;
+                c1[d][p][q] = (q > p ? range.c1[d][p][q] : q < p ? -range.c0[d][q][p] : 0.0) / h->p.scale;
                 cloud_min[d] = std::max(cloud_min[d], c0[d][p][q] + body[q].in_hi[d] - body[p].in_lo[d]);
                 cloud_max[d] = std::max(cloud_max[d], c1[d][p][q] + body[q].hi[d] - body[p].lo[d]);
             }
@@ -427,6 +436,7 @@ int ensure_ib(lbm_handle *h)
 {
     if (h->ib_ready) return LBM_OK;
     int wmax = 0, hmax = 0;
+    MotionRange range;
     double gx0 = 1e300, gx1 = -1e300, gy0 = 1e300, gy1 = -1e300;   // motion envelope (lattice units)
     if (h->nseg > 0) {
         std::vector<double> R(h->nwing, 0.0);
@@ -435,13 +445,15 @@ int ensure_ib(lbm_handle *h)
                 const double x = h->hx0[w * h->ppw + p], y = h->hy0[w * h->ppw + p];
                 R[w] = std::max(R[w], sqrt(x * x + y * y));
             }
+        for (double &r : R) r = r / h->p.scale + 4.0;
         for (int s = 0; s < h->msteps; ++s) {
+            if (h->nwing > 1) range.add(&h->mstep_host[(size_t)s * h->mcols], h->nwing);
             double xlo = 1e300, xhi = -1e300, ylo = 1e300, yhi = -1e300;
             for (int w = 0; w < h->nwing; ++w) {
                 const double sa = h->mstep_host[(size_t)s * h->mcols + 4 + 9 * w];
                 const double sb = h->mstep_host[(size_t)s * h->mcols + 7 + 9 * w];
                 const double cx = (sa + h->p.xc - h->p.ox) / h->p.scale, cy = (sb + h->p.yc - h->p.oy) / h->p.scale;
-                const double r = R[w] / h->p.scale + 4.0;
+                const double r = R[w];
                 xlo = std::min(xlo, cx - r); xhi = std::max(xhi, cx + r);
                 ylo = std::min(ylo, cy - r); yhi = std::max(yhi, cy + r);
             }
@@ -474,7 +486,7 @@ int ensure_ib(lbm_handle *h)
     h->static_order = h->nwing == 1;
     if (h->static_order) body_order(h, perm, key);
     if (h->nseg > 0 && ((h->p.flags & LBM_FLAG_DENSE_SOLVE) ||
-                        (h->nseg > kBand + 1 && (h->static_order ? band_exceeded(h, perm, key) : window_exceeded(h)))))
+                        (h->nseg > kBand + 1 && (h->static_order ? band_exceeded(h, perm, key) : window_exceeded(h, range)))))
         CK(dmalloc(h, &h->d_B, S * sizeof(double) * (size_t)ns * ns), "alloc B");
     ib_factor_scratch(ns, &h->work_blocks, &h->gf_slot);
     CK(dmalloc(h, &h->d_bD, K * sizeof(double) * h->work_blocks), "alloc block D");
