@@ -390,7 +390,11 @@ __device__ __forceinline__ void solver_cta(const LoopArgs<C> &L, double *smem)
                     ok = false;
                     break;
                 }
-            if (!ok) give_up(L.sync, a.status);
+            if (!ok) {   // report, then wait (bounded) for the copies still in flight
+                give_up(L.sync, a.status);
+                for (spins = 0; !mbar_try_wait(bar, parity) && spins < SPINS; ++spins) {
+                }
+            }
             parity ^= 1u;
         }
         // the right-hand sides in the solve order, each as soon as it is
