@@ -721,14 +721,16 @@ size_t loop_smem(const lbm_handle *h)
     return std::max(solve, NT / TILE_THREADS * sizeof(GroupSmem) + NT / 32 * stages);
 }
 
+// nodes (or pairs) of a lattice
+int loop_units(const lbm_handle *h) { return h->nx * h->ny / (h->elem == 8 ? 1 : 2); }
+
 // CTAs beside the solver that a case's lattice can use: one group's threads
 // for every 256 nodes (or pairs), so that the group without tiles does the
 // lattice alone where the SMs suffice; fewer than 24 CTAs leave tiles to
 // share one (96x64: 10.0 us a step on 6 CTAs, 9.1 on 24 and on 132)
 int loop_want(const lbm_handle *h)
 {
-    const int units = h->nx * h->ny / (h->elem == 8 ? 1 : 2);
-    return std::max((units + TILE_THREADS - 1) / TILE_THREADS, 24);
+    return std::max((loop_units(h) + TILE_THREADS - 1) / TILE_THREADS, 24);
 }
 
 template <typename C>
@@ -842,8 +844,18 @@ void loop_args_write(lbm_handle *h, int nsteps, void *const *fields, int ring_sl
 }
 
 // The CTAs of each case when `hs` run as one step_loop launch (empty: they
-// do not): one solver and at least one more, the rest by lattice size. The
-// launches per stage cost a batch some 45 us a step whatever its size.
+// do not): one solver and at least one more, the rest by lattice size. Launches
+// per stage cost a batch some 20 us a step and 0.5 us a case before any
+// lattice, a shared launch nothing, but it has 132 CTAs for all, which take
+// each their part of a lattice at 3.4 ns a node, however idle the others are:
+// the more cases, the fewer nodes (pairs, in FP32) a CTA may be left with.
+// us a step, launches per stage and here: 256x128, 32 cases (5461 a CTA) 54 and
+// 52, 36 (8192) 59 and 67, 48 (16384) 74 and 122; 384x192, 20 cases (7373) 59
+// and 55, 28 (12288) 74 and 81; 160x96, 40 (3840) 56 and 56, 48 (7680) 63 and
+// 89; 96x64, 48 to 66 (3072) 55 to 68 either way; FP64 160x96, 32 (5120) 57 and
+// 56, 48 (15360) 77 and 139. By bytes: 512x256, 12 cases (113 MB) 54 and 45, 16
+// (151 MB) 66 and 62, 20 (189 MB) 76 and 81; 800x400, 4 (92 MB) 43 and 31, 12
+// (276 MB) 87 and 91.
 std::vector<int> loop_shares(lbm_handle *const *hs, int n)
 {
     std::vector<int> share;
@@ -858,13 +870,15 @@ std::vector<int> loop_shares(lbm_handle *const *hs, int n)
     }
     if (2 * n > total || bytes > 150000000ll) return share;
     share.assign(n, 0);
-    int used = 0;
+    int used = 0, most = 0;   // most: nodes or pairs of a CTA
     for (int c = 0; c < n; ++c) {
         const int want = loop_want(hs[c]);
-        share[c] = 1 + std::max(1, std::min(want, (int)((total - 2 * n) * (want / units)) + 1));
+        const int work = std::max(1, std::min(want, (int)((total - 2 * n) * (want / units)) + 1));
+        share[c] = 1 + work;
         used += share[c];
+        most = std::max(most, loop_units(hs[c]) / work);
     }
-    return used <= total ? share : std::vector<int>();
+    return used <= total && most <= std::max(4000, 16000 - 310 * n) ? share : std::vector<int>();
 }
 
 int launch_loop_multi(lbm_handle *const *hs, int n, const std::vector<int> &share, int nsteps, bool cons0,
