@@ -245,8 +245,12 @@ void free_ib(lbm_handle *h)
 }
 
 // Whether a handle's steps run two at a time: lattices that step_loop does not
-// take, of 40 MB of populations or more, where the traffic saved outweighs the
-// nodes near the body that are done step by step.
+// take, of 40 MB of traffic a step or more. Below, where the flow chain is the
+// step, the two forms differ by no more than the runs do, and the state between
+// the steps would take half as much memory again. us a step, one and two at a
+// time, 580 markers: FP32 15 MB 34 and 34, 30 MB 39 and 35, 40 MB 41 and 33, 80
+// MB 39 and 37, 120 MB 49 and 37; FP16 30 MB 39 and 34, 40 MB 34 and 33, 80 MB 45
+// and 37; FP64 30 MB 33 and 33, 40 MB 34 and 33, 80 MB 34 and 36, 120 MB 46 and 37.
 bool pairs_fit(const lbm_handle *h)
 {
     return h->overlap && h->kf_tma && h->nseg > 0 && h->nslots % 2 == 0 && h->fbatch % 2 == 0 && !loop_fits(h) && h->nx >= 64 &&
