@@ -772,6 +772,8 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         return factor_batch(b + 1);
     };
     int done = 0, pending = 0;
+    // step n has a successor in the motion
+    auto goes_on = [&](int n) { return (double)n * dt_time <= h->mend + 1.0e-12; };
     // a small lattice's steps run as step_loop launches; per-kernel timing
     // needs the kernels one by one
     const bool loop = split && h->timing != LBM_TIMING_KERNELS && loop_fits(h);
@@ -808,9 +810,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             // motion hold, in one launch
             const int b = h->n / K, half = b & 1;
             int m = 1;
-            while (m < nsteps - s && (h->n + m) / K == b && pending + m < h->ring_cap &&
-                   (double)(h->n + m - 1) * dt_time <= h->mend + 1.0e-12)
-                ++m;
+            while (m < nsteps - s && (h->n + m) / K == b && pending + m < h->ring_cap && goes_on(h->n + m - 1)) ++m;
             if (h->batch_in_half[half] != b && (rc = factor_batch(b))) return rc;
             // the next batch's factorization, beside this launch (it waits for
             // the previous one, not for this one)
@@ -834,7 +834,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
                 CK(cudaStreamWaitEvent(cs, h->ev_inner, 0), "wait");
                 joined = false;
             }
-            if (launch_check_steps(h, h->n, m, pending, s + m == nsteps, cs))
+            if (launch_check_steps(h, h->n, m, pending, s + m == nsteps || !goes_on(h->n + m - 1), cs))
                 return cuda_err(h, cudaGetLastError(), "launch check");
             CK(cudaEventRecord(h->ev_free[half], cs), "event");
             if (m & 1) h->cur ^= 1;
@@ -848,8 +848,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
             continue;
         }
         // two steps at once: an even one and the next, neither keeping fields
-        if (pairs && h->n % 2 == 0 && s + 1 < nsteps - 2 && pending + 1 < h->ring_cap &&
-            (double)h->n * dt_time <= h->mend + 1.0e-12) {
+        if (pairs && h->n % 2 == 0 && s + 1 < nsteps - 2 && pending + 1 < h->ring_cap && goes_on(h->n)) {
             const int slot = pending, b = h->n / K, half = b & 1;
             const void *fin = h->fbuf[h->cur];
             void *fout = h->fbuf[h->cur ^ 1];
@@ -878,7 +877,7 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
                 if (launch_flow(h, src, dst, nullptr, h->n, slot + t, q, h->side, t ? nullptr : ei)) return cuda_err(h, cudaGetLastError(), "launch ib");
                 CK(cudaEventRecord(h->ev_ib, h->side), "event");
                 CK(cudaStreamWaitEvent(h->cstream, h->ev_ib, 0), "wait");
-                if (launch_check(h, h->n, slot + t, check_due(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
+                if (launch_check(h, h->n, slot + t, check_due(h->n) || !goes_on(h->n), h->cstream)) return cuda_err(h, cudaGetLastError(), "launch check");
                 if (t == 0) {
                     if ((rc = factor_next(b, s))) return rc;
                     CK(cudaStreamWaitEvent(h->stream, h->ev_batch[half], 0), "wait");
@@ -919,8 +918,8 @@ int run_steps(lbm_handle *h, int nsteps, double *rows_out, int *done_out, bool f
         cudaEvent_t *e = h->timing == LBM_TIMING_KERNELS ? &h->ev[4 * slot] : nullptr;
         if (h->timing == LBM_TIMING_SPAN && slot == 0) CK(cudaEventRecord(h->ev[0], h->stream), "event");
         // the solve-residual check: on every kCheckEvery-th step and on the
-        // last step of the call
-        const bool check_res = check_due(h->n) || s == nsteps - 1;
+        // last step of the call or of the motion
+        const bool check_res = check_due(h->n) || s == nsteps - 1 || !goes_on(h->n);
         if (split) {
             // side stream: the immersed-boundary chain and the correction
             // tiles; main stream: every other node, concurrently
