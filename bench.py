@@ -294,7 +294,9 @@ def run_ours(args, world, rank, local):
         "config": workload(args),
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_source": peak_kind, "bytes_per_update": bpl,
-                     "kernel": "kf_tma (fused stream/collide/boundary; every node but the IB correction tiles)",
+                     "kernel": "kf_tma (fused stream/collide/boundary of one step; every node but the IB correction tiles), "
+                               "timed kernel by kernel in a second pass; the steps timed for `value` run two at a time "
+                               "(kf_pair) on a large lattice, up to 16 in a launch (step_loop) on a small one",
                      "kernel_ms": kf_ms.value / kk, "ib_ms": ib_ms.value / kk,
                      "kernel_timing": f"CUDA events around every step's kernels over {kk} further steps "
                                       f"(step time with those events: {k2_ms.value / kk:.4f} ms)"},

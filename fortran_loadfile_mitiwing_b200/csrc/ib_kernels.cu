@@ -1205,8 +1205,8 @@ __global__ void __launch_bounds__(256) ib_checks(const IBArgs a0, const void *ba
 // atomics); then the lattice update of the tile's nodes with that velocity
 // correction (the node path of the lattice kernels); and each node's FP64
 // force and moment (boundary_condition.f90:1645-1675, solution.f90:327-336).
-// The last CTA sums the per-tile partials in tile order into the step's force
-// row. The lattice kernel updates every other node.
+// Each tile's sums go to its partials, which the check after the step adds up
+// (force_row). The lattice kernel updates every other node.
 template <typename T, typename C, bool FIELDS, bool BATCH>
 __global__ void __launch_bounds__(256) ib_tile_update(const IBArgs a0, const IBArgs *batch, const KFArgs<C> kf0,
                                                       const KFArgs<C> *kbatch, int step_index, int ring_slot)

@@ -88,8 +88,8 @@ struct IBArgs {
     long long st_tiles; // ints per slot of the tile lists
     int patch_wmax, patch_hmax;  // largest patch rectangle (the tile grid covers it)
     int *nsup;          // number of correction tiles (tiles listing a marker) of the slot's step
-    int *ctile;         // their tile indices, in no particular order
-    double *partial;    // per-block force partials
+    int *ctile;         // their tile indices, ascending (ib_tile_compact)
+    double *partial;    // force partials per patch tile, then those of the residual check and its counter
     double *force_ring; // [ring_cap][row_len]
     int row_len;
     // batched launches: the force-ring row of this case's step (the rows
