@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <mutex>
+#include <type_traits>
 #include <unordered_map>
 #include <vector>
 
@@ -450,22 +451,28 @@ int ensure_ib(lbm_handle *h)
                 R[w] = std::max(R[w], sqrt(x * x + y * y));
             }
         for (double &r : R) r = r / h->p.scale + 4.0;
-        for (int s = 0; s < h->msteps; ++s) {
-            if (h->nwing > 1) range.add(&h->mstep_host[(size_t)s * h->mcols], h->nwing);
-            double xlo = 1e300, xhi = -1e300, ylo = 1e300, yhi = -1e300;
-            for (int w = 0; w < h->nwing; ++w) {
-                const double sa = h->mstep_host[(size_t)s * h->mcols + 4 + 9 * w];
-                const double sb = h->mstep_host[(size_t)s * h->mcols + 7 + 9 * w];
-                const double cx = (sa + h->p.xc - h->p.ox) / h->p.scale, cy = (sb + h->p.yc - h->p.oy) / h->p.scale;
-                const double r = R[w];
-                xlo = std::min(xlo, cx - r); xhi = std::max(xhi, cx + r);
-                ylo = std::min(ylo, cy - r); yhi = std::max(yhi, cy + r);
+        const double *T = h->mstep_host.data();
+        const int nw = h->nwing, cols = h->mcols;
+        const double scale = h->p.scale, xc = h->p.xc, yc = h->p.yc, ox = h->p.ox, oy = h->p.oy;
+        auto rows = [&](auto several) {
+            for (int s = 0; s < h->msteps; ++s) {
+                const double *row = T + (size_t)s * cols;
+                if constexpr (several) range.add(row, nw);
+                double xlo = 1e300, xhi = -1e300, ylo = 1e300, yhi = -1e300;
+                for (int w = 0; w < nw; ++w) {
+                    const double sa = row[4 + 9 * w], sb = row[7 + 9 * w];
+                    const double cx = (sa + xc - ox) / scale, cy = (sb + yc - oy) / scale, r = R[w];
+                    xlo = std::min(xlo, cx - r); xhi = std::max(xhi, cx + r);
+                    ylo = std::min(ylo, cy - r); yhi = std::max(yhi, cy + r);
+                }
+                wmax = std::max(wmax, (int)ceil(xhi - xlo) + 2);
+                hmax = std::max(hmax, (int)ceil(yhi - ylo) + 2);
+                gx0 = std::min(gx0, xlo); gx1 = std::max(gx1, xhi);
+                gy0 = std::min(gy0, ylo); gy1 = std::max(gy1, yhi);
             }
-            wmax = std::max(wmax, (int)ceil(xhi - xlo) + 2);
-            hmax = std::max(hmax, (int)ceil(yhi - ylo) + 2);
-            gx0 = std::min(gx0, xlo); gx1 = std::max(gx1, xhi);
-            gy0 = std::min(gy0, ylo); gy1 = std::max(gy1, yhi);
-        }
+        };
+        if (nw > 1) rows(std::true_type());
+        else rows(std::false_type());
         wmax = std::min(wmax, h->nx);
         hmax = std::min(hmax, h->ny);
     }
