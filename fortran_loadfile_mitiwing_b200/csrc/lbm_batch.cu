@@ -242,8 +242,8 @@ int reserve(lbm_batch *b, int ncase, int ntab)
 {
     if (ncase <= b->cap && ntab <= b->table_cap) return LBM_OK;
     sync_streams(b);
-    // half as much again, so that adding cases one by one (lbm_batch_create
-    // does) allocates the some 60 arrays a few times and not once a case
+    // half as much again, so that adding cases one by one allocates the some
+    // 60 arrays a few times and not once a case
     const int nc = ncase <= b->cap ? b->cap : std::max(ncase, b->cap + b->cap / 2 + 8);
     const int nt = ntab <= b->table_cap ? b->table_cap : std::max(ntab, b->table_cap + b->table_cap / 2);
     free_arrays(b);
@@ -317,7 +317,9 @@ int check_case(lbm_batch *b, lbm_handle *h)
     return LBM_OK;
 }
 
-int add_case(lbm_batch *b, lbm_handle *h)
+// (`more` cases with `more_need` table entries are to follow: one allocation
+// of the some 60 arrays for all of them)
+int add_case(lbm_batch *b, lbm_handle *h, int more = 0, int more_need = 0)
 {
     if (b->cases.empty() && (b->prec != h->prec || b->fbatch != h->fbatch || b->nslots != h->nslots)) {
         // an empty batch takes the settings of the case that joins it
@@ -334,7 +336,7 @@ int add_case(lbm_batch *b, lbm_handle *h)
     if (rc) return rc;
     int need = table_need(h);
     for (lbm_handle *o : b->cases) need += table_need(o);
-    if ((rc = reserve(b, (int)b->cases.size() + 1, need))) return rc;
+    if ((rc = reserve(b, (int)b->cases.size() + 1 + more, need + more_need))) return rc;
     b->cases.push_back(h);
     sync_streams(b);
     clear_graphs(b);
@@ -394,8 +396,10 @@ int lbm_batch_create(lbm_t *const *cases, int count, lbm_batch_t **out)
     for (int r = 0; r < kLoopRing; ++r)
         for (cudaEvent_t *ev : {&b->ev_lup[r], &b->ev_luse[r]})
             if ((e = cudaEventCreateWithFlags(ev, cudaEventDisableTiming)) != cudaSuccess) return fail(e, "event");
+    int rest = 0;   // table entries of the cases after the first
+    for (int c = 1; c < count; ++c) rest += table_need(cases[c]);
     for (int c = 0; c < count; ++c) {
-        const int rc = add_case(b, cases[c]);
+        const int rc = add_case(b, cases[c], c == 0 ? count - 1 : 0, c == 0 ? rest : 0);
         if (rc) {
             free_batch(b);
             delete b;
